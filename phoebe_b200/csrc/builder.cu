@@ -20,10 +20,10 @@
 //    same q3 = q1+q2; each evaluated pair therefore feeds the "+" rate of
 //    (q1,q2) and the "-" rates of (q1,-q2).  Energies, velocities and Bose
 //    factors of -q2 are read from the mesh tables at the index of -q2.
-//  * Accumulation is owner-computes per q1 tile: a CTA owns 32 q1 points and a
-//    slice of q2, keeps its partial linewidths in registers and adds them to
-//    its own slot of a partial buffer; a final kernel sums the slots in a
-//    fixed order (deterministic, no atomics), then applies degeneracy
+//  * Accumulation is owner-computes per q1 tile: a CTA owns a tile of q1 points
+//    and a slice of q2, keeps its partial linewidths in registers and adds
+//    them to its own slot of a partial buffer; a final kernel sums the slots in
+//    a fixed order (deterministic, no atomics), then applies degeneracy
 //    averaging and the exclusion of acoustic Gamma modes.
 #include <algorithm>
 #include <cmath>
@@ -41,6 +41,7 @@
 #include "phx_consts.h"
 #include "phx_internal.h"
 
+#include "pair64.cuh"
 #include "pair_common.cuh"
 #include "wide.cuh"
 
@@ -48,7 +49,7 @@ using namespace pairc;
 
 namespace {
 
-constexpr int kTile = 32;    // q1 points per CTA
+constexpr int kTile = 32;    // q1 points per CTA of the isotope kernel
 
 __global__ void bose_kernel(int nq, int nb, int nT, const double* __restrict__ E,
                             const double* __restrict__ temps, double* __restrict__ bose) {
@@ -210,6 +211,12 @@ void fold_tiled_launch(int nb, int nr2, int nr3, const phx_v3* v, const phx_band
                                                                   dmax);
 }
 
+// The operand image of one chunk of q2 for the FP64 pair kernel (nb = 6).
+cudaError_t fold64(const phx_v3* v, const phx_bands* b, int c0, int cnt, void* img, cudaStream_t st) {
+  return pair64::launch_fold(v->nr2, v->nr3, v->d_D3w, v->d_R2, v->d_R3, b->d_q,
+                             reinterpret_cast<const double2*>(b->d_U), c0, cnt, static_cast<double*>(img), st);
+}
+
 struct PairArgs {
   MeshArgs m;
   int nr3;
@@ -217,356 +224,14 @@ struct PairArgs {
   const double2* Dp;
   int q2_first, q2_count, q2_per_slot;
   double* partial;   // (S, nq, nb, nT)
-  // matrix modes (pair_fp64_kernel<NB, true>): column-major blocks of the
-  // scattering matrix, element (row, col) at col * ld + row, row = q1 nb + b1.
-  //   mat_full = 1: matP is the whole matrix (one temperature); the "+" rates
-  //     of (q1 b1, q2 b2) and minus the "-" rates of (q1 b1, -q2 b2) are added
-  //     atomically (each element receives one of each).
-  //   mat_full = 0: slabs of the chunk, column j nb + b2 (j = q2 - q2_first):
-  //     matP the "+" rates of (q1 b1, q2 b2), matM the "-" rates of
-  //     (q1 b1, -q2 b2), each temperature mat_tstride elements further on;
-  //     every element of the slabs is stored.
-  double* matP;
-  double* matM;
-  long long ld;
-  size_t mat_tstride;
-  int mat_full;
 };
-
-template <int NB, bool MAT = false>
-__global__ void __launch_bounds__(kTile * NB, 1) pair_fp64_kernel(PairArgs P) {
-  const MeshArgs& M = P.m;
-  extern __shared__ __align__(16) char sraw[];
-  const int nr3 = P.nr3, nT = M.nT;
-  double2* ph = reinterpret_cast<double2*>(sraw);      // [nr3][32]
-  double2* e1s = ph + (size_t)nr3 * kTile;             // [NB*NB][32]
-  double2* e3s = e1s + NB * NB * kTile;                // [NB*NB][32]
-  double* Wx = reinterpret_cast<double*>(e3s + NB * NB * kTile);  // [NB][NB*NB][32]
-  double* b1s = Wx + NB * NB * NB * kTile;              // [nT][NB][32]
-  const int tid = threadIdx.x, ql = tid & 31, b2 = tid >> 5;
-  const int q1 = blockIdx.x * kTile + ql;
-  const bool valid = q1 < M.nq;
-  const int q1c = valid ? q1 : M.nq - 1;
-  const int n0 = M.n0, n1 = M.n1, n2 = M.n2, nq = M.nq;
-  // --- per-CTA setup: phases e^{-i q1.R3}, e1, Bose(q1)
-  for (int i = tid; i < nr3 * kTile; i += blockDim.x) {
-    const int r = i / kTile, l = i % kTile;
-    const int qq = min(blockIdx.x * kTile + l, nq - 1);
-    const double* q = M.qcart + 3 * qq;
-    double sn, cs;
-    sincos(-(q[0] * P.R3[3 * r] + q[1] * P.R3[3 * r + 1] + q[2] * P.R3[3 * r + 2]), &sn, &cs);
-    ph[i] = cmk(cs, sn);
-  }
-  for (int i = tid; i < NB * NB * kTile; i += blockDim.x) {
-    const int e = i / kTile, l = i % kTile;
-    const int qq = min(blockIdx.x * kTile + l, nq - 1);
-    e1s[i] = M.U[(size_t)qq * NB * NB + e];
-  }
-  for (int i = tid; i < nT * NB * kTile; i += blockDim.x) {
-    const int l = i % kTile, cb = i / kTile, b = cb % NB, c = cb / NB;
-    const int qq = min(blockIdx.x * kTile + l, nq - 1);
-    b1s[i] = M.bose[((size_t)c * nq + qq) * NB + b];
-  }
-  double E1[NB];
-  int g1s[NB], g1n[NB];
-#pragma unroll
-  for (int b = 0; b < NB; ++b) E1[b] = M.E[(size_t)q1c * NB + b];
-  deg_blocks<NB>(E1, g1s, g1n);
-  double acc[NB][kMaxT];
-#pragma unroll
-  for (int b = 0; b < NB; ++b)
-#pragma unroll
-    for (int c = 0; c < kMaxT; ++c) acc[b][c] = 0.0;
-  __syncthreads();
-
-  const int jbeg = blockIdx.y * P.q2_per_slot;
-  const int jend = min(P.q2_count, jbeg + P.q2_per_slot);
-  for (int j = jbeg; j < jend; ++j) {
-    const int iq2 = P.q2_first + j;
-    const int iq2m = mesh_neg(iq2, n0, n1, n2);
-    const int iq3 = mesh_add(q1c, iq2, n0, n1, n2);
-    // stage e3 of the 32 q3 points
-    for (int i = tid; i < NB * NB * kTile; i += blockDim.x) {
-      const int e = i / kTile, l = i % kTile;
-      const int qq = min(blockIdx.x * kTile + l, nq - 1);
-      const int q3 = mesh_add(qq, iq2, n0, n1, n2);
-      e3s[i] = M.U[(size_t)q3 * NB * NB + e];
-    }
-    __syncthreads();
-    // T(a,c) = sum_r3 e^{-i q1.R3} Dp(q2)[r3][a][b2][c]
-    double2 T[NB][NB];
-#pragma unroll
-    for (int a = 0; a < NB; ++a)
-#pragma unroll
-      for (int c = 0; c < NB; ++c) T[a][c] = cmk(0.0, 0.0);
-    const double2* D = P.Dp + (size_t)j * nr3 * NB * NB * NB + b2 * NB;
-    for (int r = 0; r < nr3; ++r) {
-      const double2 p = ph[r * kTile + ql];
-      const double2* Dr = D + (size_t)r * NB * NB * NB;
-#pragma unroll
-      for (int a = 0; a < NB; ++a)
-#pragma unroll
-        for (int c = 0; c < NB; ++c) cfma(T[a][c], p, __ldg(Dr + a * NB * NB + c));
-    }
-    // X(b1,c) = sum_a e1(a,b1) T(a,c), in place column by column
-#pragma unroll
-    for (int c = 0; c < NB; ++c) {
-      double2 col[NB];
-#pragma unroll
-      for (int a = 0; a < NB; ++a) col[a] = T[a][c];
-#pragma unroll
-      for (int b1 = 0; b1 < NB; ++b1) {
-        double2 x = cmk(0.0, 0.0);
-#pragma unroll
-        for (int a = 0; a < NB; ++a) cfma(x, e1s[(a * NB + b1) * kTile + ql], col[a]);
-        T[b1][c] = x;
-      }
-    }
-    // V(b1,b3) = sum_c X(b1,c) conj(e3(c,b3)); W = |V|^2
-    double W[NB][NB];
-#pragma unroll
-    for (int b1 = 0; b1 < NB; ++b1) {
-#pragma unroll
-      for (int b3 = 0; b3 < NB; ++b3) {
-        double2 v = cmk(0.0, 0.0);
-#pragma unroll
-        for (int c = 0; c < NB; ++c) cfmac(v, T[b1][c], e3s[(c * NB + b3) * kTile + ql]);
-        W[b1][b3] = v.x * v.x + v.y * v.y;
-      }
-    }
-    // symmetrise over degenerate blocks of b1 (E1) and b3 (E3)
-    double E3[NB];
-    int g3s[NB], g3n[NB];
-#pragma unroll
-    for (int b = 0; b < NB; ++b) E3[b] = M.E[(size_t)iq3 * NB + b];
-    deg_blocks<NB>(E3, g3s, g3n);
-#pragma unroll
-    for (int b1 = 0; b1 < NB; ++b1) {
-      double row[NB];
-#pragma unroll
-      for (int b3 = 0; b3 < NB; ++b3) {
-        double s = 0.0;
-#pragma unroll
-        for (int k = 0; k < NB; ++k) s += (g3s[k] == g3s[b3]) ? W[b1][k] : 0.0;
-        row[b3] = s / (double)g3n[b3];
-      }
-#pragma unroll
-      for (int b3 = 0; b3 < NB; ++b3) W[b1][b3] = row[b3];
-    }
-#pragma unroll
-    for (int b3 = 0; b3 < NB; ++b3) {
-      double colv[NB];
-#pragma unroll
-      for (int b1 = 0; b1 < NB; ++b1) {
-        double s = 0.0;
-#pragma unroll
-        for (int k = 0; k < NB; ++k) s += (g1s[k] == g1s[b1]) ? W[k][b3] : 0.0;
-        colv[b1] = s / (double)g1n[b1];
-      }
-#pragma unroll
-      for (int b1 = 0; b1 < NB; ++b1) W[b1][b3] = colv[b1];
-    }
-    // exchange across b2 (one warp per b2) and average over E2 blocks
-#pragma unroll
-    for (int b1 = 0; b1 < NB; ++b1)
-#pragma unroll
-      for (int b3 = 0; b3 < NB; ++b3) Wx[((b2 * NB + b1) * NB + b3) * kTile + ql] = W[b1][b3];
-    __syncthreads();
-    double E2v[NB];
-    int g2s[NB], g2n[NB];
-#pragma unroll
-    for (int b = 0; b < NB; ++b) E2v[b] = M.E[(size_t)iq2 * NB + b];
-    deg_blocks<NB>(E2v, g2s, g2n);
-    int mys = 0, myn = 1;
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-      if (b == b2) { mys = g2s[b]; myn = g2n[b]; }
-    if (myn > 1) {
-#pragma unroll
-      for (int b1 = 0; b1 < NB; ++b1)
-#pragma unroll
-        for (int b3 = 0; b3 < NB; ++b3) {
-          double s = 0.0;
-          for (int k = mys; k < mys + myn; ++k) s += Wx[((k * NB + b1) * NB + b3) * kTile + ql];
-          W[b1][b3] = s / (double)myn;
-        }
-    }
-    // epilogue: "+" rates of (q1,q2) and "-" rates of (q1,-q2)
-    const double en2 = M.E[(size_t)iq2 * NB + b2];
-    const double en2m = M.E[(size_t)iq2m * NB + b2];
-    const bool ok2 = en2 >= phxc::phExcludeCutoff && en2 >= phxc::phEnergyCutoff;
-    const bool ok2m = en2m >= phxc::phExcludeCutoff && en2m >= phxc::phEnergyCutoff;
-    double v2[3] = {0, 0, 0}, v2m[3] = {0, 0, 0};
-    if (M.smearing == PHX_SMEAR_ADAPTIVE) {
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        v2[i] = M.vg[((size_t)iq2 * NB + b2) * 3 + i];
-        v2m[i] = M.vg[((size_t)iq2m * NB + b2) * 3 + i];
-      }
-    }
-    if constexpr (MAT) {
-      // one temperature at a time: the sums over b3 of the "+" rates (sp) and
-      // of the two "-" rates (sm) of each b1, which also make the linewidths
-#pragma unroll 1
-      for (int c = 0; c < nT; ++c) {
-        double sp[NB], sm[NB];
-#pragma unroll
-        for (int b1 = 0; b1 < NB; ++b1) sp[b1] = sm[b1] = 0.0;
-        if (valid && (ok2 || ok2m)) {
-          const double n2c = M.bose[((size_t)c * nq + iq2) * NB + b2];
-          const double n2mc = M.bose[((size_t)c * nq + iq2m) * NB + b2];
-#pragma unroll
-          for (int b3 = 0; b3 < NB; ++b3) {
-            const double en3 = E3[b3];
-            if (en3 < phxc::phEnergyCutoff) continue;
-            double sgp = M.sigma, sgm = M.sigma;
-            bool vzp = false, vzm = false;
-            if (M.smearing == PHX_SMEAR_ADAPTIVE) {
-              const double* v3 = M.vg + ((size_t)iq3 * NB + b3) * 3;
-              const double dp0 = v2[0] - v3[0], dp1 = v2[1] - v3[1], dp2 = v2[2] - v3[2];
-              const double dm0 = v2m[0] - v3[0], dm1 = v2m[1] - v3[1], dm2 = v2m[2] - v3[2];
-              vzp = (dp0 * dp0 + dp1 * dp1 + dp2 * dp2) == 0.0;
-              vzm = (dm0 * dm0 + dm1 * dm1 + dm2 * dm2) == 0.0;
-              sgp = floor_sigma(adaptive_sigma(M.qT, dp0, dp1, dp2));
-              sgm = floor_sigma(adaptive_sigma(M.qT, dm0, dm1, dm2));
-            }
-            const double n3c = M.bose[((size_t)c * nq + iq3) * NB + b3];
-#pragma unroll
-            for (int b1 = 0; b1 < NB; ++b1) {
-              const double en1 = E1[b1];
-              if (en1 < phxc::phExcludeCutoff || en1 < phxc::phEnergyCutoff) continue;
-              const double w = W[b1][b3];
-              const double n1 = b1s[(c * NB + b1) * kTile + ql];
-              if (ok2) {
-                const double dlt = delta_fn(M.smearing, sgp, en1 + en2 - en3, vzp);
-                if (dlt > 0.0) sp[b1] += phxc::pi * 0.25 * w * dlt * M.norm / (en1 * en2 * en3) * n1 * n2c * (n3c + 1.0);
-              }
-              if (ok2m) {
-                double d1 = delta_fn(M.smearing, sgm, en1 + en3 - en2m, vzm);
-                double d2 = delta_fn(M.smearing, sgm, en2m + en3 - en1, vzm);
-                if (d1 > 0.0 || d2 > 0.0) {
-                  d1 = fmax(d1, 0.0);
-                  d2 = fmax(d2, 0.0);
-                  const double f = phxc::pi * 0.25 * w * M.norm / (en1 * en2m * en3);
-                  sm[b1] += f * n3c * n1 * (n2mc + 1.0) * d1 + f * n2mc * n3c * (n1 + 1.0) * d2;
-                }
-              }
-            }
-          }
-        }
-#pragma unroll
-        for (int b1 = 0; b1 < NB; ++b1)
-#pragma unroll
-          for (int cc = 0; cc < kMaxT; ++cc)
-            if (cc == c) acc[b1][cc] += 0.5 * (sp[b1] + sm[b1]);
-        if (valid) {
-          const size_t row = (size_t)q1 * NB;
-          if (P.mat_full) {
-            double* colp = P.matP + (size_t)(iq2 * NB + b2) * P.ld + row;
-            double* colm = P.matP + (size_t)(iq2m * NB + b2) * P.ld + row;
-#pragma unroll
-            for (int b1 = 0; b1 < NB; ++b1) {
-              if (sp[b1] != 0.0) atomicAdd(colp + b1, sp[b1]);
-              if (sm[b1] != 0.0) atomicAdd(colm + b1, -sm[b1]);
-            }
-          } else {
-            const size_t o = c * P.mat_tstride + (size_t)(j * NB + b2) * P.ld + row;
-#pragma unroll
-            for (int b1 = 0; b1 < NB; ++b1) {
-              P.matP[o + b1] = sp[b1];
-              P.matM[o + b1] = sm[b1];
-            }
-          }
-        }
-      }
-    } else if (valid && (ok2 || ok2m)) {
-#pragma unroll
-      for (int b3 = 0; b3 < NB; ++b3) {
-        const double en3 = E3[b3];
-        if (en3 < phxc::phEnergyCutoff) continue;
-        double sp = M.sigma, sm = M.sigma;
-        bool vzp = false, vzm = false;
-        if (M.smearing == PHX_SMEAR_ADAPTIVE) {
-          const double* v3 = M.vg + ((size_t)iq3 * NB + b3) * 3;
-          const double dp0 = v2[0] - v3[0], dp1 = v2[1] - v3[1], dp2 = v2[2] - v3[2];
-          const double dm0 = v2m[0] - v3[0], dm1 = v2m[1] - v3[1], dm2 = v2m[2] - v3[2];
-          vzp = (dp0 * dp0 + dp1 * dp1 + dp2 * dp2) == 0.0;
-          vzm = (dm0 * dm0 + dm1 * dm1 + dm2 * dm2) == 0.0;
-          sp = floor_sigma(adaptive_sigma(M.qT, dp0, dp1, dp2));
-          sm = floor_sigma(adaptive_sigma(M.qT, dm0, dm1, dm2));
-        }
-        double n3[kMaxT];
-#pragma unroll
-        for (int c = 0; c < kMaxT; ++c)
-          n3[c] = c < nT ? M.bose[((size_t)c * nq + iq3) * NB + b3] : 0.0;
-        double n2[kMaxT], n2m[kMaxT];
-#pragma unroll
-        for (int c = 0; c < kMaxT; ++c) {
-          n2[c] = c < nT ? M.bose[((size_t)c * nq + iq2) * NB + b2] : 0.0;
-          n2m[c] = c < nT ? M.bose[((size_t)c * nq + iq2m) * NB + b2] : 0.0;
-        }
-#pragma unroll
-        for (int b1 = 0; b1 < NB; ++b1) {
-          const double en1 = E1[b1];
-          if (en1 < phxc::phExcludeCutoff || en1 < phxc::phEnergyCutoff) continue;
-          const double w = W[b1][b3];
-          if (ok2) {
-            const double dlt = delta_fn(M.smearing, sp, en1 + en2 - en3, vzp);
-            if (dlt > 0.0) {
-              const double f = phxc::pi * 0.25 * w * dlt * M.norm / (en1 * en2 * en3);
-#pragma unroll
-              for (int c = 0; c < kMaxT; ++c)
-                if (c < nT) {
-                  const double n1 = b1s[(c * NB + b1) * kTile + ql];
-                  acc[b1][c] += 0.5 * (f * n1 * n2[c] * (n3[c] + 1.0));
-                }
-            }
-          }
-          if (ok2m) {
-            double d1 = delta_fn(M.smearing, sm, en1 + en3 - en2m, vzm);
-            double d2 = delta_fn(M.smearing, sm, en2m + en3 - en1, vzm);
-            if (d1 > 0.0 || d2 > 0.0) {
-              d1 = fmax(d1, 0.0);
-              d2 = fmax(d2, 0.0);
-              const double f = phxc::pi * 0.25 * w * M.norm / (en1 * en2m * en3);
-#pragma unroll
-              for (int c = 0; c < kMaxT; ++c)
-                if (c < nT) {
-                  const double n1 = b1s[(c * NB + b1) * kTile + ql];
-                  const double r1 = f * n3[c] * n1 * (n2m[c] + 1.0) * d1;
-                  const double r2 = f * n2m[c] * n3[c] * (n1 + 1.0) * d2;
-                  acc[b1][c] += 0.5 * (r1 + r2);
-                }
-            }
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-  // reduce over the b2 warps and add to this CTA's partial slot
-#pragma unroll
-  for (int b1 = 0; b1 < NB; ++b1)
-#pragma unroll
-    for (int c = 0; c < kMaxT; ++c) Wx[((b2 * NB + b1) * kMaxT + c) * kTile + ql] = acc[b1][c];
-  __syncthreads();
-  if (b2 == 0 && valid) {
-    double* out = P.partial + ((size_t)blockIdx.y * nq + q1) * NB * nT;
-    for (int b1 = 0; b1 < NB; ++b1)
-      for (int c = 0; c < nT; ++c) {
-        double s = 0.0;
-        for (int k = 0; k < NB; ++k) s += Wx[((k * NB + b1) * kMaxT + c) * kTile + ql];
-        out[b1 * nT + c] += s;
-      }
-  }
-}
 
 // ---------------------------------------------------------------------------
 // Any nb up to kMaxNbGeneric (the 15-branch cells), with an optional per-q1
 // window on q2: one block per (q1, q2 slot), the R3 transform, the e1 and e3
 // contractions, |V|^2, the three symmetrisation passes and the rates of each
 // q2 run through shared memory (two nb^3 complex buffers).  Same algebra,
-// cutoffs and time-reversal pairing as pair_fp64_kernel: the "+" vertex of
+// cutoffs and time-reversal pairing as pair64_kernel: the "+" vertex of
 // (q1, q2) gives the "+" process of (q1, q2) and the "-" process of
 // (q1, -q2); with a window, each of the two is counted only when its q2 is
 // inside the window of q1.
@@ -1361,7 +1026,8 @@ int run_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Aout_d,
   int max_slots = 0;
   for (auto& c : cands) max_slots = std::max(max_slots, c.slots);
   const size_t nb3 = (size_t)NB * NB * NB;
-  const size_t sz_dp = align_up(sizeof(double2) * max_chunk * nr3 * nb3);
+  const size_t sz_dp = align_up(split ? sizeof(double2) * max_chunk * nr3 * nb3
+                                      : pair64::image_bytes(nr3) * max_chunk);
   const size_t sz_part = align_up(sizeof(double) * max_slots * nq * NB * nT);
   const size_t sz_bose = align_up(sizeof(double) * nT * nq * NB);
   const size_t sz_T = align_up(sizeof(double) * 8);
@@ -1405,7 +1071,7 @@ int run_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Aout_d,
     }
   }
   const double emax = split ? b->emax : 0.0;
-  PairArgs P{};
+  pair64::Args P{};
   P.m.nq = nq;
   P.m.nb = NB;
   P.m.nT = nT;
@@ -1424,14 +1090,12 @@ int run_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Aout_d,
   P.m.norm = 1.0 / (double)nq;
   P.nr3 = nr3;
   P.R3 = v->d_R3;
-  P.Dp = Dp;
+  P.img = reinterpret_cast<const double*>(Dp);
   P.partial = partial;
-  const size_t smem_pair = sizeof(double2) * ((size_t)nr3 * kTile + 2 * NB * NB * kTile) +
-                           sizeof(double) * ((size_t)NB * NB * NB * kTile + (size_t)kMaxT * NB * kTile);
+  P.status = ctx->d_status;
   if (!split) {
-    PHX_ARG(ctx, smem_pair <= 227 * 1024, "phx_ph_linewidths: too many R3 vectors for the FP64 path");
-    PHX_CUDA(ctx, cudaFuncSetAttribute(pair_fp64_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem_pair));
+    PHX_ARG(ctx, nr3 <= pair64::kMaxR3, "phx_ph_linewidths: too many R3 vectors for the FP64 path");
+    PHX_CUDA(ctx, pair64::set_attributes(nr3, false, p->smearing));
   }
   const size_t smem_fold = fold_tiled_smem(NB, nr2);
   PHX_ARG(ctx, smem_fold <= 227 * 1024, "phx_ph_linewidths: too many R2 vectors");
@@ -1444,21 +1108,21 @@ int run_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Aout_d,
   auto chunk_work = [&](const BuilderPlan& pl, int c0, int cnt, cudaEvent_t pe0, cudaEvent_t pe1,
                         int* launches, unsigned* overflow = nullptr, int edge_only = 0) -> int {
     if (fp16) PHX_CUDA(ctx, cudaMemsetAsync(dmax, 0, sizeof(unsigned), st));
-    fold_tiled_launch(NB, nr2, nr3, v, b, c0, cnt, Dp, st, fp16 ? dmax : nullptr);
+    if (split) fold_tiled_launch(NB, nr2, nr3, v, b, c0, cnt, Dp, st, fp16 ? dmax : nullptr);
+    else PHX_CUDA(ctx, fold64(v, b, c0, cnt, Dp, st));
     ++*launches;
     if (split)
       return phx_split_pair_chunk(ctx, P.m, v, b, Dp, Bimg, rec, emax, c0, cnt, pl.slots, partial, launches,
                                   pe0, pe1, fp16, dmax, edges, edge_count, edge_cap, edge_peak, overflow,
                                   edge_only);
-    PairArgs Q = P;
+    pair64::Args Q = P;
     Q.q2_first = c0;
     Q.q2_count = cnt;
     Q.q2_per_slot = (cnt + pl.slots - 1) / pl.slots;
     if (pe0) PHX_CUDA(ctx, phx_record_event(pe0, st));
-    pair_fp64_kernel<NB><<<dim3(tiles, pl.slots), kTile * NB, smem_pair, st>>>(Q);
+    PHX_CUDA(ctx, pair64::launch_pair(Q, pl.slots, false, st));
     if (pe1) PHX_CUDA(ctx, phx_record_event(pe1, st));
     ++*launches;
-    PHX_CUDA(ctx, cudaGetLastError());
     return PHX_OK;
   };
   PHX_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), st));
@@ -1857,7 +1521,7 @@ int run_builder_generic(phx_v3* v, phx_bands* b, const phx_lw_params* p, double*
 // ---------------------------------------------------------------------------
 // Matrix modes of the builder (ph_scattering.cpp, switchCase 0 and 1, without
 // symmetries), FP64, nb = 6.  The q2 loop is the linewidth builder's: the R2
-// fold of a chunk, then pair_fp64_kernel<6, true>, whose epilogue also keeps,
+// fold of a chunk, then pair64_kernel<true, .>, whose epilogue also keeps,
 // per (q1 b1, q2 b2), the sums over b3 of the "+" and of the "-" rates.
 //   mode 0 (A_full): they go straight into the stored matrix (ns x ns,
 //     column-major; nT = 1), isotope rates after the last chunk, then the
@@ -1887,7 +1551,7 @@ int run_matrix_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
   }
   const int slots = std::min(split ? (full ? 28 : 7) : 8, chunk);
   const size_t nb3 = (size_t)NB * NB * NB;
-  const size_t sz_dp = align_up(sizeof(double2) * chunk * nr3 * nb3);
+  const size_t sz_dp = align_up(split ? sizeof(double2) * chunk * nr3 * nb3 : pair64::image_bytes(nr3) * chunk);
   const size_t sz_part = align_up(sizeof(double) * slots * nq * NB * nT);
   const size_t sz_bose = align_up(sizeof(double) * nT * nq * NB);
   const size_t sz_T = align_up(sizeof(double) * 8);
@@ -1929,7 +1593,7 @@ int run_matrix_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
     }
     PHX_TRY(phx_split_set_attributes(ctx, nr3, nT));
   }
-  PairArgs P{};
+  pair64::Args P{};
   P.m.nq = nq;
   P.m.nb = NB;
   P.m.nT = nT;
@@ -1948,18 +1612,16 @@ int run_matrix_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
   P.m.norm = 1.0 / (double)nq;
   P.nr3 = nr3;
   P.R3 = v->d_R3;
-  P.Dp = Dp;
+  P.img = reinterpret_cast<const double*>(Dp);
+  P.status = ctx->d_status;
   P.partial = partial;
   P.matP = full ? A_full : slabP;
   P.matM = slabM;
   P.ld = ns;
   P.mat_tstride = slab_elems;
   P.mat_full = full ? 1 : 0;
-  const size_t smem_pair = sizeof(double2) * ((size_t)nr3 * kTile + 2 * NB * NB * kTile) +
-                           sizeof(double) * ((size_t)NB * NB * NB * kTile + (size_t)kMaxT * NB * kTile);
-  PHX_ARG(ctx, smem_pair <= 227 * 1024, "scattering matrix: too many R3 vectors for the FP64 path");
-  PHX_CUDA(ctx, cudaFuncSetAttribute(pair_fp64_kernel<NB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem_pair));
+  PHX_ARG(ctx, nr3 <= pair64::kMaxR3, "scattering matrix: too many R3 vectors for the FP64 path");
+  if (!split) PHX_CUDA(ctx, pair64::set_attributes(nr3, true, p->smearing));
   const size_t smem_fold = fold_tiled_smem(NB, nr2);
   PHX_ARG(ctx, smem_fold <= 227 * 1024, "scattering matrix: too many R2 vectors");
   if (smem_fold > 48 * 1024)
@@ -1999,15 +1661,16 @@ int run_matrix_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
                                      nullptr, nullptr, fp16, dmax, edges, edge_count, phx_split_edge_cap(),
                                      edge_peak, edge_over, 0, &mo));
       } else {
-        fold_tiled_launch(NB, nr2, nr3, v, b, c0, cnt, Dp, st);
+        // the matrix sums go in by atomics, onto zeroed slabs
+        if (!full) PHX_CUDA(ctx, cudaMemsetAsync(slabP, 0, sizeof(double) * 2 * nT * slab_elems, st));
+        PHX_CUDA(ctx, fold64(v, b, c0, cnt, Dp, st));
         ++launches;
-        PairArgs Q = P;
+        pair64::Args Q = P;
         Q.q2_first = c0;
         Q.q2_count = cnt;
         Q.q2_per_slot = (cnt + slots - 1) / slots;
-        pair_fp64_kernel<NB, true><<<dim3(tiles, slots), kTile * NB, smem_pair, st>>>(Q);
+        PHX_CUDA(ctx, pair64::launch_pair(Q, slots, true, st));
         ++launches;
-        PHX_CUDA(ctx, cudaGetLastError());
       }
       if (!full) {
         if (giso) {
@@ -2736,7 +2399,9 @@ namespace {
 
 constexpr size_t kStaticScratchBytes = size_t(16) << 20;  // 16 MiB per GPU
 
-__device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
+constexpr size_t kStaticPadBytes = size_t(16) << 10;
+
+__device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes + kStaticPadBytes];
 
 std::mutex g_static_mutex;
 // device address of g_static_scratch, per device, with the CUDA context it was
@@ -2810,30 +2475,25 @@ int run_builder_static(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
                       std::to_string(kStaticScratchBytes) + " bytes (reduce mesh points or temperatures)");
     return PHX_ERR_ARG;
   }
-  const size_t smem_pair = sizeof(double2) * ((size_t)nr3 * kTile + 2 * NB * NB * kTile) +
-                           sizeof(double) * ((size_t)NB * NB * NB * kTile + (size_t)kMaxT * NB * kTile);
-  PHX_ARG(ctx, smem_pair <= 227 * 1024, "phx_ph_linewidths_static: too many R3 vectors");
+  PHX_ARG(ctx, nr3 <= pair64::kMaxR3, "phx_ph_linewidths_static: too many R3 vectors");
   const size_t smem_fold = sizeof(double2) * ((size_t)nr2 + 2 * NB * NB);
   PHX_ARG(ctx, smem_fold <= 227 * 1024, "phx_ph_linewidths_static: too many R2 vectors");
-  const int chunk = (int)std::min<size_t>({(kStaticScratchBytes - fixed) / per_q2, (size_t)512,
-                                           (size_t)(q2e - q2b)});
-  PHX_CUDA(ctx, cudaFuncSetAttribute(pair_fp64_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem_pair));
-  if (smem_fold > 48 * 1024)
-    PHX_CUDA(ctx, cudaFuncSetAttribute(fold_q2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem_fold));
+  // the operand image pads R3 to a multiple of four; kStaticPadBytes holds the padding of one q2
+  const int chunk = (int)std::min<size_t>({(kStaticScratchBytes + kStaticPadBytes - fixed) / pair64::image_bytes(nr3),
+                                           (size_t)512, (size_t)(q2e - q2b)});
+  PHX_CUDA(ctx, pair64::set_attributes(nr3, false, p->smearing));
   void* base_v = nullptr;
   PHX_TRY(static_scratch_address(ctx, &base_v));
   char* base = static_cast<char*>(base_v);
   double* partial = reinterpret_cast<double*>(base);
   double* bose = reinterpret_cast<double*>(base + sz_part);
   double* temps = reinterpret_cast<double*>(base + sz_part + sz_bose);
-  double2* Dp = reinterpret_cast<double2*>(base + fixed);
+  double* img = reinterpret_cast<double*>(base + fixed);
   // the array keeps the previous call's contents: clear what accumulates
   PHX_CUDA(ctx, cudaMemcpyAsync(temps, p->temperatures, sizeof(double) * nT, cudaMemcpyHostToDevice, st));
   PHX_CUDA(ctx, cudaMemsetAsync(partial, 0, sizeof(double) * (size_t)nq * NB * nT, st));
   bose_kernel<<<std::min(1024, (nq * NB * nT + 255) / 256), 256, 0, st>>>(nq, NB, nT, b->d_E, temps, bose);
-  PairArgs P{};
+  pair64::Args P{};
   P.m.nq = nq;
   P.m.nb = NB;
   P.m.nT = nT;
@@ -2852,25 +2512,28 @@ int run_builder_static(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
   P.m.norm = 1.0 / (double)nq;
   P.nr3 = nr3;
   P.R3 = v->d_R3;
-  P.Dp = Dp;
+  P.img = img;
+  P.status = ctx->d_status;
   P.partial = partial;
-  const int tiles = (nq + kTile - 1) / kTile;
+  PHX_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), st));
   for (int c0 = q2b; c0 < q2e; c0 += chunk) {
     const int cnt = std::min(chunk, q2e - c0);
-    const int per_block = 8;
-    fold_q2_kernel<<<dim3(nr3, (cnt + per_block - 1) / per_block), 128, smem_fold, st>>>(
-        NB, nr2, nr3, v->d_D3w, v->d_R2, v->d_R3, b->d_q, reinterpret_cast<const double2*>(b->d_U), c0,
-        cnt, per_block, Dp);
+    PHX_CUDA(ctx, fold64(v, b, c0, cnt, img, st));
     P.q2_first = c0;
     P.q2_count = cnt;
     P.q2_per_slot = cnt;
-    pair_fp64_kernel<NB><<<dim3(tiles, 1), kTile * NB, smem_pair, st>>>(P);
-    PHX_CUDA(ctx, cudaGetLastError());
+    PHX_CUDA(ctx, pair64::launch_pair(P, 1, false, st));
   }
   finalize_kernel<<<(nq + 127) / 128, 128, 0, st>>>(nq, NB, nT, 1, partial, b->d_E, p->finalize, nullptr, nullptr,
                                                     0.0, Aout_d);
   PHX_CUDA(ctx, cudaGetLastError());
+  int kst = 0;
+  PHX_CUDA(ctx, cudaMemcpyAsync(&kst, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
   PHX_CUDA(ctx, cudaStreamSynchronize(st));
+  if (kst) {
+    phx_set_error(ctx, PHX_ERR_CUDA, "phx_ph_linewidths_static: kernel status " + std::to_string(kst));
+    return PHX_ERR_CUDA;
+  }
   return PHX_OK;
 }
 

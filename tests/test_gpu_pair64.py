@@ -1,0 +1,93 @@
+"""The FP64 pair kernel of the 6-branch cells (tensor-pipe R3 transform) against
+the oracle on identical band structures, at the edges of its tiles: meshes
+smaller than a warp's 8 q1 and than a block's tile, q1 counts that are no
+multiple of either, R3 counts around the K step of 4 and beyond one ring stage,
+and the largest R3 count the path takes (fewer warps per block).  1e-10 is the
+bar of the other FP64 linewidth tests (sums of ~1e5 terms, each with a few
+rounding errors of 1e-16, and the cancellation of the R3 sum)."""
+import numpy as np
+import pytest
+
+import oracle
+from phoebe_b200 import constants as C
+from phoebe_b200 import lattice, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _fc3(cr, nr3):
+    """A random real tensor on one R2 and nr3 R3 vectors (no sum rule: the kernels need none)."""
+    R, _ = synth.lattice_cube(cr, 3)
+    rng = np.random.default_rng(nr3)
+    o = np.argsort(np.linalg.norm(R, axis=1), kind="stable")
+    D3 = rng.normal(size=(6, 6, 6, nr3, 1)) * 0.05
+    nat = cr.num_atoms
+    return synth.FC3(D3, R[o[1:2]], R[o[:nr3]], np.ones((1, nat, nat)), np.ones((nr3, nat, nat)), nr3)
+
+
+def _bands(ctx, cr, mesh):
+    from phoebe_b200.core import PhononH0
+    h0 = PhononH0(ctx, cr, synth.diamond_fc2(cr))
+    bands = h0.populate(mesh, withVelocities=True)
+    h0.close()
+    return bands
+
+
+def _close(a, b, rtol):
+    scale = np.abs(b).max()
+    assert scale > 0
+    big = np.abs(b) > 1e-6 * scale
+    assert (np.abs(a - b)[big] / np.abs(b)[big]).max() < rtol
+    assert np.abs(a - b)[~big].max(initial=0.0) < rtol * 1e-6 * scale
+
+
+@pytest.mark.parametrize("smearing,temps", [("adaptive", (100.0, 300.0, 600.0, 900.0)), ("gaussian", (300.0,))])
+@pytest.mark.parametrize("mesh,nr3", [((2, 2, 1), 1), ((3, 3, 1), 4), ((4, 4, 4), 5), ((5, 3, 5), 48),
+                                      ((3, 3, 3), 49), ((5, 4, 3), 97), ((2, 3, 2), 262)])
+def test_linewidths_at_tile_edges(ctx, mesh, nr3, smearing, temps):
+    from phoebe_b200.core import Interaction3Ph, PhScatteringMatrix
+    cr = synth.diamond_crystal()
+    fc3 = _fc3(cr, nr3)
+    bands = _bands(ctx, cr, mesh)
+    E, U, vg = bands.get()
+    T = np.array([C.kelvin_to_ry(t) for t in temps])
+    v3 = Interaction3Ph(ctx, cr, fc3)
+    sm = PhScatteringMatrix(v3, bands, T, smearing, 0.3 / C.ryToTHz)
+    A = sm.setup()
+    m = lattice.Mesh(cr, mesh)
+    ref = oracle.Interaction3Ph(cr, fc3).linewidths(mesh, E, U, vg, m.cartesian_coords(), cr.reciprocal_cell, T,
+                                                    smearing, 0.3 / C.ryToTHz)
+    _close(A, ref, 1e-10)
+    # a rank's q2 slice of one point
+    part = sm.setup(1, 2, finalize=False)
+    rest = [sm.setup(0, 1, finalize=False), sm.setup(2, bands.nq, finalize=False)]
+    whole = sm.setup(finalize=False)
+    np.testing.assert_allclose(part + rest[0] + rest[1], whole, rtol=1e-12, atol=1e-14 * np.abs(whole).max())
+    v3.close()
+    bands.close()
+
+
+@pytest.mark.parametrize("smearing", ["adaptive", "gaussian"])
+def test_matrix_modes_with_degenerate_points(ctx, diamond, smearing):
+    """Stored matrix and matrix-free product; the diamond's symmetry points have degenerate
+    blocks of b1, b2 and b3, some across the kernel's pairs of b2."""
+    from phoebe_b200.core import Interaction3Ph, PhScatteringMatrix
+    cr, mesh = diamond["crystal"], (3, 4, 3)
+    bands = _bands(ctx, cr, mesh)
+    E, U, vg = bands.get()
+    T = C.kelvin_to_ry(300.0)
+    sigma = 0.5 / C.ryToTHz
+    ref = oracle.Interaction3Ph(cr, diamond["fc3"])
+    q = lattice.Mesh(cr, mesh).cartesian_coords()
+    mat, lw = ref.scattering_matrix(mesh, E, U, vg, q, cr.reciprocal_cell, T, smearing, sigma)
+    v3 = Interaction3Ph(ctx, cr, diamond["fc3"])
+    sm = PhScatteringMatrix(v3, bands, [T], smearing, sigma, in_memory=True)
+    _close(sm.setup(), lw[None], 1e-10)
+    _close(sm.getMatrixRows(0, sm.num_states), mat, 1e-10)
+    x = np.random.default_rng(1).normal(size=(2, 1, 3, sm.num_states))
+    free = PhScatteringMatrix(v3, bands, [T], smearing, sigma)
+    y = free.dot(x)
+    np.testing.assert_allclose(y, sm.dot(x), rtol=0, atol=1e-11 * np.abs(y).max())
+    sm.close()
+    v3.close()
+    bands.close()
