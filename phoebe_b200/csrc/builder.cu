@@ -627,49 +627,49 @@ __global__ void __launch_bounds__(kTile * kMaxNbGeneric) isotope_kernel(IsoArgs 
 // averaging, ph_scattering.cpp:819-860), then zero for excluded states.
 // The matrix modes pass average = 0: their diagonal is not averaged
 // (ph_scattering.cpp:809-817).
-__global__ void finalize_kernel(int nq, int nb, int nT, int nslots, const double* __restrict__ partial,
-                                const double* __restrict__ E, int finalize, const double* __restrict__ vg,
-                                const double* __restrict__ temps, double boundary_length,
-                                double* __restrict__ Aout, int average = 1) {
-  const int iq = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per q: its lanes sum the slots of the (b, T) values, which are
+// consecutive in memory (on a coarse mesh a builder call has many slots).
+constexpr int kFinWarps = 4;
+__global__ void __launch_bounds__(32 * kFinWarps)
+finalize_kernel(int nq, int nb, int nT, int nslots, const double* __restrict__ partial,
+                const double* __restrict__ E, int finalize, const double* __restrict__ vg,
+                const double* __restrict__ temps, double boundary_length, double* __restrict__ Aout,
+                int average = 1) {
+  __shared__ double sums[kFinWarps][64 * kMaxT];
+  const int iq = blockIdx.x * kFinWarps + threadIdx.x / 32, lane = threadIdx.x % 32;
   if (iq >= nq) return;
+  double* lw = sums[threadIdx.x / 32];   // [b][T]
   const size_t ns = (size_t)nq * nb;
-  double lw[64];
-  for (int c = 0; c < nT; ++c) {
-    for (int b = 0; b < nb; ++b) {
-      double s = 0.0;
-      for (int k = 0; k < nslots; ++k) s += partial[(((size_t)k * nq + iq) * nb + b) * nT + c];
-      lw[b] = s;
-    }
+  const double* Eq = E + (size_t)iq * nb;
+  for (int t = lane; t < nb * nT; t += 32) {
+    double s = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < nslots; ++k) s += partial[((size_t)k * nq + iq) * nb * nT + t];
+    lw[t] = s;
+  }
+  __syncwarp();
+  for (int t = lane; t < nb * nT; t += 32) {
+    const int b = t / nT, c = t % nT;
+    const double e = Eq[b];
+    double v = lw[t];
     if (finalize && average && c == 0) {
       // degeneracyAveragingLinewidths (scattering.cpp:1168-1207), row 0 only
-      double tmp[64];
-      for (int b1 = 0; b1 < nb; ++b1) {
-        int n = 0;
-        double t = 0.0;
-        for (int b2 = 0; b2 < nb; ++b2)
-          if (fabs(E[(size_t)iq * nb + b2] - E[(size_t)iq * nb + b1]) < phxc::degThreshold) {
-            ++n;
-            t += lw[b2];
-          }
-        tmp[b1] = t / (double)(float)n;
-      }
-      for (int b = 0; b < nb; ++b) lw[b] = tmp[b];
+      int n = 0;
+      v = 0.0;
+      for (int b2 = 0; b2 < nb; ++b2)
+        if (fabs(Eq[b2] - e) < phxc::degThreshold) {
+          ++n;
+          v += lw[b2 * nT];
+        }
+      v /= (double)(float)n;
     }
-    if (finalize && boundary_length > 0.0 && vg) {
-      for (int b = 0; b < nb; ++b) {
-        const double e = E[(size_t)iq * nb + b];
-        if (e < phxc::phExcludeCutoff) continue;
-        const double* v = vg + ((size_t)iq * nb + b) * 3;
-        const double x = sinh(e / 2.0 / temps[c]);
-        lw[b] += sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]) / boundary_length * (0.25 / x / x);
-      }
+    if (finalize && boundary_length > 0.0 && vg && !(e < phxc::phExcludeCutoff)) {
+      const double* u = vg + ((size_t)iq * nb + b) * 3;
+      const double x = sinh(e / 2.0 / temps[c]);
+      v += sqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]) / boundary_length * (0.25 / x / x);
     }
-    for (int b = 0; b < nb; ++b) {
-      double v = lw[b];
-      if (finalize && E[(size_t)iq * nb + b] < phxc::phExcludeCutoff) v = 0.0;
-      Aout[(size_t)c * ns + (size_t)iq * nb + b] = v;
-    }
+    if (finalize && e < phxc::phExcludeCutoff) v = 0.0;
+    Aout[(size_t)c * ns + (size_t)iq * nb + b] = v;
   }
 }
 
@@ -861,6 +861,26 @@ struct PlanKey {
 std::mutex g_plan_mutex;
 std::map<PlanKey, BuilderPlan> g_plans;
 
+// Slots of a chunk of `cnt` q2 for `tiles` q1 tiles: one block per (tile,
+// slot), one block per SM.  The fixed slot counts of the tuned plans leave most
+// SMs idle when there are few tiles (5^3: one tile), so this one takes the
+// count that minimises waves x (q2 of a slot + one, about what a block's
+// set-up of phases and eigenvectors costs).  Measured: split 5^3 2.02 -> 0.40
+// ms a call (7 -> 125 slots), FP64 8^3 4.3 -> 2.2 ms (8 -> 18 slots).
+// (slot_bytes: one slot's sums; at most 64 MB of them beyond the fixed count).
+int fill_slots(int tiles, int cnt, int fixed, int sms, size_t slot_bytes) {
+  int best = std::min(fixed, cnt);
+  long best_cost = -1;
+  for (int s = 1; s <= cnt && (s <= fixed || s * slot_bytes <= (size_t(64) << 20)); ++s) {
+    const long waves = ((long)tiles * s + sms - 1) / sms, cost = waves * ((cnt + s - 1) / s + 1);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = s;
+    }
+  }
+  return best;
+}
+
 bool find_plan(const PlanKey& k, BuilderPlan* out) {
   std::lock_guard<std::mutex> lock(g_plan_mutex);
   auto it = g_plans.find(k);
@@ -1023,7 +1043,13 @@ int run_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Aout_d,
   int max_chunk = 0;
   for (auto& c : cands) max_chunk = std::max(max_chunk, c.chunk);
   max_chunk = std::min(max_chunk, std::max(1, q2e - q2b));
-  int max_slots = 0;
+  // a range of q2 that is too short to be tuned (coarse meshes, slices)
+  const bool few_q2 = q2e - q2b < 2 * cands[0].chunk;
+  const int tiles_pair = (nq + (split ? 127 : pair64::tile_q1(nr3) - 1)) / (split ? 128 : pair64::tile_q1(nr3));
+  const size_t slot_bytes = sizeof(double) * nq * NB * nT;
+  int max_slots = few_q2 ? fill_slots(tiles_pair, std::min(cands[0].chunk, std::max(1, q2e - q2b)), cands[0].slots,
+                                      ctx->num_sms, slot_bytes)
+                         : 0;
   for (auto& c : cands) max_slots = std::max(max_slots, c.slots);
   const size_t nb3 = (size_t)NB * NB * NB;
   const size_t sz_dp = align_up(split ? sizeof(double2) * max_chunk * nr3 * nb3
@@ -1134,7 +1160,7 @@ int run_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Aout_d,
   cudaGetDevice(&dev);
   const PlanKey pk{split ? 1 + fp16 : 0, NB, nq, nr3, nr2, nT, dev};
   BuilderPlan plan = cands[0];
-  if (!env_off("PHX_TUNE") && q2e - q2b >= 2 * cands[0].chunk && !find_plan(pk, &plan)) {
+  if (!env_off("PHX_TUNE") && !few_q2 && !find_plan(pk, &plan)) {
     int dummy = 0;
     if (split) PHX_TRY(phx_split_pack_records(ctx, P.m, rec, &dummy));
     bose_kernel<<<std::min(1024, (nq * NB * nT + 255) / 256), 256, 0, st>>>(nq, NB, nT, b->d_E, temps, bose);
@@ -1167,6 +1193,7 @@ int run_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Aout_d,
     store_plan(pk, plan);
   }
   plan.chunk = std::min(plan.chunk, std::max(1, q2e - q2b));
+  if (few_q2) plan.slots = fill_slots(tiles_pair, plan.chunk, plan.slots, ctx->num_sms, slot_bytes);
   plan.slots = std::min(plan.slots, plan.chunk);
   const int nslots = plan.slots;
   // the device work of the call
@@ -1194,7 +1221,7 @@ int run_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Aout_d,
       ++launches;
       PHX_CUDA(ctx, cudaGetLastError());
     }
-    finalize_kernel<<<(nq + 127) / 128, 128, 0, st>>>(nq, NB, nT, nslots, partial, b->d_E, p->finalize, b->d_vg,
+    finalize_kernel<<<(nq + kFinWarps - 1) / kFinWarps, 32 * kFinWarps, 0, st>>>(nq, NB, nT, nslots, partial, b->d_E, p->finalize, b->d_vg,
                                                       temps, p->boundary_length, Aout_d);
     ++launches;
     PHX_CUDA(ctx, cudaGetLastError());
@@ -1275,7 +1302,7 @@ int run_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Aout_d,
       }
     }
     if (rc == PHX_OK && overflowed) {
-      finalize_kernel<<<(nq + 127) / 128, 128, 0, st>>>(nq, NB, nT, nslots, partial, b->d_E, p->finalize, b->d_vg,
+      finalize_kernel<<<(nq + kFinWarps - 1) / kFinWarps, 32 * kFinWarps, 0, st>>>(nq, NB, nT, nslots, partial, b->d_E, p->finalize, b->d_vg,
                                                         temps, p->boundary_length, Aout_d);
       cudaError_t ce = cudaGetLastError();
       if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
@@ -1469,7 +1496,7 @@ int run_builder_generic(phx_v3* v, phx_bands* b, const phx_lw_params* p, double*
       ++launches;
       PHX_CUDA(ctx, cudaGetLastError());
     }
-    finalize_kernel<<<(nq + 127) / 128, 128, 0, st>>>(nq, nb, nT, slots, partial, b->d_E, p->finalize, b->d_vg,
+    finalize_kernel<<<(nq + kFinWarps - 1) / kFinWarps, 32 * kFinWarps, 0, st>>>(nq, nb, nT, slots, partial, b->d_E, p->finalize, b->d_vg,
                                                       temps, p->boundary_length, Aout_d);
     ++launches;
     PHX_CUDA(ctx, cudaGetLastError());
@@ -1711,7 +1738,7 @@ int run_matrix_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
       PHX_CUDA(ctx, cudaGetLastError());
     }
     PHX_CUDA(ctx, cudaEventRecord(evv1, st));
-    finalize_kernel<<<(nq + 127) / 128, 128, 0, st>>>(nq, NB, nT, slots, partial, b->d_E, p->finalize, b->d_vg, temps,
+    finalize_kernel<<<(nq + kFinWarps - 1) / kFinWarps, 32 * kFinWarps, 0, st>>>(nq, NB, nT, slots, partial, b->d_E, p->finalize, b->d_vg, temps,
                                                       p->boundary_length, lw_d, 0);
     ++launches;
     PHX_CUDA(ctx, cudaGetLastError());
@@ -2138,7 +2165,7 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
       ++launches;
       PHX_CUDA(ctx, cudaGetLastError());
     }
-    finalize_kernel<<<(nq + 127) / 128, 128, 0, st>>>(nq, nb, nT, 1, lw, b->d_E, p->finalize, b->d_vg, temps,
+    finalize_kernel<<<(nq + kFinWarps - 1) / kFinWarps, 32 * kFinWarps, 0, st>>>(nq, nb, nT, 1, lw, b->d_E, p->finalize, b->d_vg, temps,
                                                       p->boundary_length, Aout_d);
     ++launches;
     PHX_CUDA(ctx, cudaGetLastError());
@@ -2524,7 +2551,7 @@ int run_builder_static(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
     P.q2_per_slot = cnt;
     PHX_CUDA(ctx, pair64::launch_pair(P, 1, false, st));
   }
-  finalize_kernel<<<(nq + 127) / 128, 128, 0, st>>>(nq, NB, nT, 1, partial, b->d_E, p->finalize, nullptr, nullptr,
+  finalize_kernel<<<(nq + kFinWarps - 1) / kFinWarps, 32 * kFinWarps, 0, st>>>(nq, NB, nT, 1, partial, b->d_E, p->finalize, nullptr, nullptr,
                                                     0.0, Aout_d);
   PHX_CUDA(ctx, cudaGetLastError());
   int kst = 0;

@@ -86,7 +86,7 @@ struct TcArgs {
   const double* R3;
   int nr3;
   const int* q1_order;         // q1 points in k-space blocks of 4x4x2 (warp coherence)
-  int q2_first, q2_count, q2_per_slot;
+  int q2_first, q2_count, q2_per_slot, slots;
   float tol;                   // margin of the FP32 liveness windows (Ry)
   double* partial;             // (S, nq, nb, nT)
   int* status;
@@ -104,7 +104,7 @@ struct TcArgs {
 // A queued triplet one of whose adaptive deltas sat within 1e-5 of the
 // |E| > 2 sigma cut-off: the queue entry and where it was evaluated.
 struct EdgeEvent {
-  unsigned where;    // tile << 12 | slot << 7 | row
+  unsigned where;    // (tile * slots + slot) << 7 | row
   int iq2;
   uint2 entry;       // the queue entry (|V|^2 / n1, meta)
 };
@@ -609,7 +609,7 @@ __device__ __noinline__ void rate_entry(uint2 e, int qd, float ginv, float pre, 
   if (near) {
     // a cut-off decision too close for FP32: edge_fix_kernel re-decides the entry in FP64
     const unsigned i = atomicAdd(P.edge_count, 1u);
-    if (i < P.edge_cap) P.edges[i] = EdgeEvent{(blockIdx.x << 12) | (blockIdx.y << 7) | (unsigned)mm, iq2, e};
+    if (i < P.edge_cap) P.edges[i] = EdgeEvent{(blockIdx.x * gridDim.y + blockIdx.y) << 7 | (unsigned)mm, iq2, e};
   }
   constexpr int AR = Pcfg<NT>::kAccRow;
 #pragma unroll
@@ -1226,7 +1226,7 @@ __global__ void edge_fix_kernel(TcArgs P) {
   const unsigned n = cnt;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const EdgeEvent ev = P.edges[i];
-    const int tile = ev.where >> 12, slot = (ev.where >> 7) & 31, mm = ev.where & 127;
+    const int tile = (ev.where >> 7) / P.slots, slot = (ev.where >> 7) % P.slots, mm = ev.where & 127;
     const int q1 = P.q1_order[tile * kM + mm];
     const int b1 = (ev.entry.y >> 5) & 7;
     double corr[NT];
@@ -1314,6 +1314,7 @@ int phx_split_pair_chunk(phx_ctx* ctx, const pairc::MeshArgs& M, const phx_v3* v
   A.q2_first = q2_first;
   A.q2_count = q2_count;
   A.q2_per_slot = (q2_count + slots - 1) / slots;
+  A.slots = slots;
   // FP32 energies carry a relative rounding of 2^-24; a window test sums
   // four of them and a sigma: 32 units of the largest energy bound it.
   A.tol = (float)(32.0 * std::max(emax, 1e-6) * 5.9604644775390625e-8);
@@ -1328,7 +1329,7 @@ int phx_split_pair_chunk(phx_ctx* ctx, const pairc::MeshArgs& M, const phx_v3* v
   A.edge_overflow = edge_overflow;
   A.edge_only = edge_only;
   A.mat = mat ? *mat : phx_split_matrix{nullptr, nullptr, 0, 0, 0};
-  PHX_ARG(ctx, slots < 32 && (M.nq + kM - 1) / kM < (1 << 20), "split path: at most 31 slots");
+  PHX_ARG(ctx, (long long)((M.nq + kM - 1) / kM) * slots <= (1 << 25), "split path: too many q1 tiles x slots");
   PHX_CUDA(ctx, cudaMemsetAsync(edge_count, 0, sizeof(unsigned), ctx->stream));
   const int tiles = (M.nq + kM - 1) / kM;
   int rc = PHX_OK;

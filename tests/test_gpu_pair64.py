@@ -91,3 +91,27 @@ def test_matrix_modes_with_degenerate_points(ctx, diamond, smearing):
     sm.close()
     v3.close()
     bands.close()
+
+
+@pytest.mark.parametrize("mesh", [(2, 1, 1), (3, 3, 3), (7, 5, 4)])
+def test_coarse_meshes_fill_the_chip(ctx, diamond, mesh):
+    """A q2 range too short to be tuned takes as many slots as fill the SMs; the split path's
+    linewidths keep its 1e-5 bar against FP64, whose own slots sum in another order (1e-12)."""
+    from phoebe_b200.core import Interaction3Ph, PhScatteringMatrix
+    cr = diamond["crystal"]
+    bands = _bands(ctx, cr, mesh)
+    T = np.array([C.kelvin_to_ry(t) for t in (100.0, 300.0)])
+    out = {}
+    for precision in ("fp64", "split_fp16"):
+        v3 = Interaction3Ph(ctx, cr, diamond["fc3"], precision=precision)
+        sm = PhScatteringMatrix(v3, bands, T, "adaptive")
+        out[precision] = sm.setup()
+        assert 1 <= sm.stats.plan_slots <= bands.nq
+        half = sm.setup(0, bands.nq // 2, finalize=False) + sm.setup(bands.nq // 2, bands.nq, finalize=False)
+        whole = sm.setup(finalize=False)
+        np.testing.assert_allclose(half, whole, rtol=1e-12 if precision == "fp64" else 1e-6,
+                                   atol=1e-12 * np.abs(whole).max())
+        v3.close()
+    if np.abs(out["fp64"]).max() > 0:
+        _close(out["split_fp16"], out["fp64"], 1e-5)
+    bands.close()
