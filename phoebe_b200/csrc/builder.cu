@@ -1972,9 +1972,14 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
   PHX_ARG(ctx, !p->isotope_coupling || nb <= 32, "phx_ph_linewidths: isotope scattering supports nb <= 32");
   const int Kp = wide::split_kp(nr3);
   int nq1 = wide::kQ1;
+  // the kernel with one warp per q1 (wide_split.cu) wherever it fits: nb <= 36
+  // and an R3 count that leaves room for its T; it has no shape to tune
+  int warp_q1 = 0, warp_rows = 0;
   if (split) {
     PHX_ARG(ctx, wide::split_smem(nb, Kp, 2) > 0,
             "phx_ph_linewidths: too many branches or R3 vectors for the split path");
+    warp_q1 = wide::warp_q1(nb, Kp, &warp_rows);
+    if (warp_q1) nq1 = warp_q1;
   } else {
     nq1 = wide::fp64_q1(nb, nr3);
     PHX_ARG(ctx, nq1 > 0, "phx_ph_linewidths: too many branches or R3 vectors for the FP64 path");
@@ -2013,11 +2018,13 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
   unsigned* dmax = counters + nchunks;
   if (split && !b->d_U32) {
     const size_t n = (size_t)nq * nb * nb;
-    PHX_CUDA(ctx, phx_dev_alloc(ctx, (void**)&b->d_U32, sizeof(float2) * n));
+    // padded: wide_split.cu reads whole tiles
+    PHX_CUDA(ctx, phx_dev_alloc(ctx, (void**)&b->d_U32, sizeof(float2) * (n + 64)));
     PHX_CUDA(ctx, wide::launch_u32(reinterpret_cast<const double2*>(b->d_U), reinterpret_cast<float2*>(b->d_U32), n,
                                    st));
   }
-  PHX_CUDA(ctx, wide::set_attributes(nb, nr3, split));
+  if (warp_q1) PHX_CUDA(ctx, wide::warp_set_attributes(nb, Kp, p->smearing));
+  else PHX_CUDA(ctx, wide::set_attributes(nb, nr3, split));
   // q1 order: by window cut with a window (tiles of similar q2 sets), else the mesh order
   std::vector<int> order_h(nq);
   for (int i = 0; i < nq; ++i) order_h[i] = i;
@@ -2077,7 +2084,7 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
   const PlanKey pk{20 + fp16, nb, nq, nr3, nr2, nT, dev};
   BuilderPlan shape{A.rt, A.qp};   // (chunk, slots) fields hold (rt, qp) here
   const int tune_q2 = std::min(chunk, 64);   // q2 of the timed chunk (every q1)
-  if (split && !skip && !env_off("PHX_TUNE") && q2e - q2b >= 2 * tune_q2 && !find_plan(pk, &shape)) {
+  if (split && !warp_q1 && !skip && !env_off("PHX_TUNE") && q2e - q2b >= 2 * tune_q2 && !find_plan(pk, &shape)) {
     bose_kernel<<<std::min(1024, (nq * nb * nT + 255) / 256), 256, 0, st>>>(nq, nb, nT, b->d_E, temps, bose);
     if (fp16) PHX_CUDA(ctx, cudaMemsetAsync(dmax, 0, sizeof(unsigned), st));
     PHX_CUDA(ctx, wide::launch_fold(nb, nr2, nr3, v->d_D3w, v->d_r2_ofs, v->d_r2_list, v->r2_max_list, v->d_R2,
@@ -2121,8 +2128,8 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
     store_plan(pk, shape);
   }
   if (split) {
-    A.rt = shape.chunk;
-    A.qp = shape.slots;
+    A.rt = warp_q1 ? warp_rows : shape.chunk;
+    A.qp = warp_q1 ? warp_q1 : shape.slots;
   }
   long long pairs = 0;
   for (int c0 = q2b; c0 < q2e; c0 += chunk) pairs += (long long)nq * std::min(chunk, q2e - c0);
@@ -2154,7 +2161,9 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
       PHX_CUDA(ctx, cudaEventCreate(&pe1));
       g.pair_events.push_back(pe1);
       PHX_CUDA(ctx, phx_record_event(pe0, st));
-      PHX_CUDA(ctx, split ? wide::launch_split(Ac, grid, st) : wide::launch_fp64(Ac, grid, st));
+      PHX_CUDA(ctx, warp_q1 ? wide::launch_warp_split(Ac, grid, st)
+                    : split ? wide::launch_split(Ac, grid, st)
+                            : wide::launch_fp64(Ac, grid, st));
       PHX_CUDA(ctx, phx_record_event(pe1, st));
       ++launches;
     }

@@ -51,6 +51,11 @@ cudaError_t launch_fp64(const Args& A, int grid, cudaStream_t st);
 cudaError_t launch_split(const Args& A, int grid, cudaStream_t st);
 cudaError_t set_attributes(int nb, int nr3, bool split);   // for every tile shape
 int blocks_per_sm(int nb, int nr3, bool split);
+// split kernel with one warp per q1 (wide_split.cu): its q1 per item for this
+// nb and Kp (0: use the kernel above), and the rows of its lanes' tiles
+int warp_q1(int nb, int Kp, int* tile_rows);
+cudaError_t warp_set_attributes(int nb, int Kp, int smearing);
+cudaError_t launch_warp_split(const Args& A, int grid, cudaStream_t st);
 // R2 fold of a chunk of q2 (sparse over the non-zero (r3, r2) blocks)
 size_t fold_smem(int nb, int max_list);
 cudaError_t launch_fold(int nb, int nr2, int nr3, const double* D3w, const int* r2_ofs, const int* r2_list,

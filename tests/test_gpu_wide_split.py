@@ -1,0 +1,82 @@
+"""The split-precision kernel with one warp per q1 (cells of up to 36 branches) at the edges of its
+classes of tile and of its lanes' tiles, against the FP64 builder on the same band structure: the
+split paths' bar of 1e-5 on linewidths above 1e-8 of the largest.  Cells of 1 to 12 atoms (the
+twelve-atom cell's first atoms), q1 counts that are no multiple of an item, R3 counts of one K step
+and of several A stages, q2 windows, both smearings, and an R3 count that leaves no room for the
+kernel (the older one takes over)."""
+import numpy as np
+import pytest
+
+from phoebe_b200 import constants as C
+from phoebe_b200 import lattice, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _cell(nat):
+    cr = synth.twelve_atom_crystal(synth.SEED_BASE + 4)
+    return lattice.Crystal(cr.direct_cell, cr.positions[:nat], np.arange(nat), cr.species_masses[:nat])
+
+
+def _fc3(cr, nr3):
+    R, _ = synth.lattice_cube(cr, 2)
+    rng = np.random.default_rng(nr3)
+    o = np.argsort(np.linalg.norm(R, axis=1), kind="stable")
+    nat, nb = cr.num_atoms, cr.num_bands
+    D3 = rng.normal(size=(nb, nb, nb, nr3, 1)) * 0.05
+    return synth.FC3(D3, R[o[1:2]], R[o[:nr3]], np.ones((1, nat, nat)), np.ones((nr3, nat, nat)), nr3)
+
+
+def _bands(ctx, cr, mesh, rng):
+    """Energies with degenerate blocks in every point, random unitary eigenvectors; -q the conjugate of q."""
+    from phoebe_b200.core import BandStructure
+    n0, n1, n2 = mesh
+    nq, nb = n0 * n1 * n2, cr.num_bands
+    i = np.arange(nq)
+    neg = ((n2 - i // (n0 * n1)) % n2) * n0 * n1 + ((n1 - (i // n0) % n1) % n1) * n0 + (n0 - i % n0) % n0
+    E = np.sort(rng.uniform(5e-4, 4e-3, (nq, nb)), axis=1)
+    E[:, 1] = E[:, 0]
+    E[i % 3 == 0, -1] = E[i % 3 == 0, -2]
+    E = np.minimum(E, E[neg])
+    E = np.sort(E, axis=1)
+    U = np.linalg.qr(rng.normal(size=(nq, nb, nb)) + 1j * rng.normal(size=(nq, nb, nb)))[0]
+    V = rng.normal(size=(nq, nb, 3)) * 5e-4
+    half = i < neg
+    U[neg[half]] = U[half].conj()
+    V[neg[half]] = -V[half]
+    own = i == neg
+    U[own] = np.linalg.qr(rng.normal(size=(own.sum(), nb, nb)))[0]
+    V[own] = 0.0
+    return E, BandStructure.from_arrays(ctx, mesh, cr.reciprocal_cell, E, U, V)
+
+
+@pytest.mark.parametrize("smearing", ["adaptive", "gaussian"])
+@pytest.mark.parametrize("nat,mesh,nr3,window", [(1, (3, 2, 2), 1, False), (3, (3, 3, 2), 27, True), (5, (3, 2, 2), 8, False),
+                                                 (5, (5, 4, 1), 125, True), (6, (3, 2, 2), 48, False), (8, (3, 2, 2), 57, True),
+                                                 (9, (3, 2, 1), 27, False), (12, (3, 2, 1), 48, True),
+                                                 (12, (3, 1, 1), 105, False), (13, (3, 1, 1), 9, False)])
+def test_split_matches_fp64(ctx, nat, mesh, nr3, window, smearing):
+    from phoebe_b200.core import Interaction3Ph, PhScatteringMatrix
+    cr = _cell(nat)
+    E, bands = _bands(ctx, cr, mesh, np.random.default_rng(nat))
+    fc3 = _fc3(cr, nr3)
+    T = np.array([C.kelvin_to_ry(t) for t in (100.0, 300.0, 600.0)])
+    win = synth.q2_window(E, mesh) if window else None
+    out = {}
+    for precision in ("fp64", "split_fp16", "split_bf16"):
+        v3 = Interaction3Ph(ctx, cr, fc3, precision=precision)
+        sm = PhScatteringMatrix(v3, bands, T, smearing, 1e-4, window=win)
+        out[precision] = sm.setup()
+        if precision != "fp64":
+            again = sm.setup(0, 1, finalize=False) + sm.setup(1, bands.nq, finalize=False)
+            whole = sm.setup(finalize=False)
+            # FP16 operands are scaled by the largest of a call: slices round differently
+            np.testing.assert_allclose(again, whole, rtol=1e-5, atol=1e-8 * np.abs(whole).max())
+        v3.close()
+    A = out["fp64"]
+    big = np.abs(A) > 1e-8 * np.abs(A).max()
+    assert big.any()
+    for precision in ("split_fp16", "split_bf16"):
+        assert np.isfinite(out[precision]).all()
+        assert (np.abs(out[precision] - A)[big] / np.abs(A)[big]).max() < 1e-5, precision
+    bands.close()
