@@ -127,21 +127,21 @@ class PhononH0:
     def diagonalizeFromCoordinates(self, q_cart, withMassScaling=True):
         q = f64(np.atleast_2d(q_cart))
         nq = q.shape[0]
-        E = np.zeros((nq, self.nb))
-        U = np.zeros((nq, self.nb, self.nb, 2))
+        E = np.empty((nq, self.nb))
+        U = np.empty((nq, self.nb, self.nb), dtype=np.complex128)
         check(_abi.load().phx_ph_diag(self.h, nq, dptr(q), int(withMassScaling), dptr(E),
                                       dptr(U)), self.ctx.h)
-        return E, U[..., 0] + 1j * U[..., 1]
+        return E, U
 
     def diagonalizeWithVelocities(self, q_cart):
         q = f64(np.atleast_2d(q_cart))
         nq = q.shape[0]
-        E = np.zeros((nq, self.nb))
-        U = np.zeros((nq, self.nb, self.nb, 2))
-        vg = np.zeros((nq, self.nb, 3))
+        E = np.empty((nq, self.nb))
+        U = np.empty((nq, self.nb, self.nb), dtype=np.complex128)
+        vg = np.empty((nq, self.nb, 3))
         check(_abi.load().phx_ph_diag_velocities(self.h, nq, dptr(q), dptr(E), dptr(U), dptr(vg)),
               self.ctx.h)
-        return E, U[..., 0] + 1j * U[..., 1], vg
+        return E, U, vg
 
     def populate(self, mesh, withVelocities=True):
         """Band structure on a full Gamma-centred mesh, resident on the GPU."""
@@ -193,12 +193,12 @@ class BandStructure:
         return cls(ctx, h, mesh, nb, reciprocal_cell)
 
     def get(self, velocities=True):
-        E = np.zeros((self.nq, self.nb))
-        U = np.zeros((self.nq, self.nb, self.nb, 2))
-        vg = np.zeros((self.nq, self.nb, 3)) if velocities else None
+        E = np.empty((self.nq, self.nb))
+        U = np.empty((self.nq, self.nb, self.nb), dtype=np.complex128)
+        vg = np.empty((self.nq, self.nb, 3)) if velocities else None
         check(_abi.load().phx_bands_get(self.h, dptr(E), dptr(U),
                                         dptr(vg) if velocities else None), self.ctx.h)
-        return E, U[..., 0] + 1j * U[..., 1], vg
+        return E, U, vg
 
     def close(self):
         if getattr(self, "h", None):
@@ -247,28 +247,39 @@ class Interaction3Ph:
         nb = self.nb
 
         def pad(evs):
+            # full bands at every q1 (one stacked array of them above all) need no loop over q1
+            if isinstance(evs, (np.ndarray, list, tuple)) and len(evs) == nq1 and nq1 and np.shape(evs[0]) == (nb, nb):
+                try:
+                    whole = np.asarray(evs, dtype=np.complex128)
+                except ValueError:
+                    whole = None
+                if whole is not None and whole.shape == (nq1, nb, nb):
+                    return whole, np.full(nq1, nb)
             out = np.zeros((nq1, nb, nb), dtype=np.complex128)
             for i, e in enumerate(evs):
                 e = np.asarray(e)
                 out[i, :, :e.shape[1]] = e
-            return out
+            return out, np.array([np.asarray(e).shape[1] for e in evs])
 
-        e1, e3p, e3m = pad(ev1s), pad(ev3Pluss), pad(ev3Minss)
+        (e1, n1), (e3p, n3p), (e3m, n3m) = pad(ev1s), pad(ev3Pluss), pad(ev3Minss)
         ev2 = np.asarray(ev2)
         e2 = np.zeros((nb, nb), dtype=np.complex128)
         e2[:, :ev2.shape[1]] = ev2
-        nb1s = i32(nb1s if nb1s is not None else [np.asarray(e).shape[1] for e in ev1s])
+        nb1s = i32(nb1s if nb1s is not None else n1)
         nb2 = int(nb2 if nb2 is not None else ev2.shape[1])
-        nb3p = i32(nb3Pluss if nb3Pluss is not None else [np.asarray(e).shape[1] for e in ev3Pluss])
-        nb3m = i32(nb3Minss if nb3Minss is not None else [np.asarray(e).shape[1] for e in ev3Minss])
+        nb3p = i32(nb3Pluss if nb3Pluss is not None else n3p)
+        nb3m = i32(nb3Minss if nb3Minss is not None else n3m)
         sizeP = int(np.sum(nb1s * nb2 * nb3p))
         sizeM = int(np.sum(nb1s * nb2 * nb3m))
-        outP = np.zeros(max(sizeP, 1))
-        outM = np.zeros(max(sizeM, 1))
+        outP = np.empty(max(sizeP, 1))
+        outM = np.empty(max(sizeM, 1))
         E1, E2, E3p, E3m = c128(e1), c128(e2), c128(e3p), c128(e3m)
         check(_abi.load().phx_v3_couplings_sq(self.h, nq1, dptr(q1), dptr(E1), iptr(nb1s), dptr(E2),
                                               nb2, dptr(E3p), iptr(nb3p), dptr(E3m), iptr(nb3m),
                                               dptr(outP), dptr(outM)), self.ctx.h)
+        if nq1 and all(len(x) == nq1 and (x == x[0]).all() for x in (nb1s, nb3p, nb3m)):
+            return (list(outP[:sizeP].reshape(nq1, nb1s[0], nb2, nb3p[0])),
+                    list(outM[:sizeM].reshape(nq1, nb1s[0], nb2, nb3m[0])))
         cp, cm = [], []
         oP = oM = 0
         for i in range(nq1):
@@ -558,12 +569,12 @@ class ElectronH0Wannier:
     def _diag(self, k_cart, velocities):
         k = f64(np.atleast_2d(k_cart))
         nk = k.shape[0]
-        E = np.zeros((nk, self.nw))
-        U = np.zeros((nk, self.nw, self.nw, 2))
-        vg = np.zeros((nk, self.nw, 3)) if velocities else None
+        E = np.empty((nk, self.nw))
+        U = np.empty((nk, self.nw, self.nw), dtype=np.complex128)
+        vg = np.empty((nk, self.nw, 3)) if velocities else None
         check(_abi.load().phx_el_diag(self.h, nk, dptr(k), dptr(E), dptr(U),
                                       dptr(vg) if velocities else None), self.ctx.h)
-        return E, U[..., 0] + 1j * U[..., 1], vg
+        return E, U, vg
 
     def diagonalizeFromCoordinates(self, k_cart):
         E, U, _ = self._diag(k_cart, False)

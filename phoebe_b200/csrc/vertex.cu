@@ -454,9 +454,10 @@ extern "C" int phx_v3_couplings_sq(phx_v3* v, int nq1, const double* q1s, const 
       rc = PHX_ERR_CUDA;
     }
   }
-  cudaFree(dq); cudaFree(de1); cudaFree(de2); cudaFree(de3p); cudaFree(de3m);
-  cudaFree(doP); cudaFree(doM); cudaFree(dn1); cudaFree(dn3p); cudaFree(dn3m);
-  cudaFree(dofP); cudaFree(dofM);
+  // back to the pool on the stream (cudaFree would synchronise the device for each)
+  for (void* d : {(void*)dq, (void*)de1, (void*)de2, (void*)de3p, (void*)de3m, (void*)doP, (void*)doM, (void*)dn1,
+                  (void*)dn3p, (void*)dn3m, (void*)dofP, (void*)dofM})
+    phx_dev_free(ctx, d);
   return rc;
 }
 
