@@ -227,8 +227,8 @@ struct PairArgs {
 };
 
 // ---------------------------------------------------------------------------
-// Any nb up to kMaxNbGeneric (the 15-branch cells), with an optional per-q1
-// window on q2: one block per (q1, q2 slot), the R3 transform, the e1 and e3
+// Any nb up to kMaxNbGeneric, with an optional per-q1 window on q2, where the R3
+// vectors are too many for wide64.cu's phases in shared memory: one block per (q1, q2 slot), the R3 transform, the e1 and e3
 // contractions, |V|^2, the three symmetrisation passes and the rates of each
 // q2 run through shared memory (two nb^3 complex buffers).  Same algebra,
 // cutoffs and time-reversal pairing as pair64_kernel: the "+" vertex of
@@ -1975,6 +1975,7 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
   // the kernel with one warp per q1 (wide_split.cu) wherever it fits: nb <= 36
   // and an R3 count that leaves room for its T; it has no shape to tune
   int warp_q1 = 0, warp_rows = 0;
+  const int mma_q1 = split ? 0 : wide::q1_fp64_mma(nb, nr3);
   if (split) {
     PHX_ARG(ctx, wide::split_smem(nb, Kp, 2) > 0,
             "phx_ph_linewidths: too many branches or R3 vectors for the split path");
@@ -1982,15 +1983,17 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
     if (warp_q1) nq1 = warp_q1;
   } else {
     nq1 = wide::fp64_q1(nb, nr3);
-    PHX_ARG(ctx, nq1 > 0, "phx_ph_linewidths: too many branches or R3 vectors for the FP64 path");
+    PHX_ARG(ctx, nq1 > 0 || mma_q1 > 0, "phx_ph_linewidths: too many branches or R3 vectors for the FP64 path");
+    if (mma_q1) nq1 = mma_q1;
   }
   PHX_TRY(wide_prepare_blocks(v));
   PHX_ARG(ctx, wide::fold_smem(nb, v->r2_max_list) <= 227 * 1024, "phx_ph_linewidths: too many R2 vectors");
   const size_t nb3 = (size_t)nb * nb * nb;
   const size_t per_q2 = sizeof(double2) * nr3 * nb3 + (split ? wide::split_img_bytes(nb, Kp) : 0);
-  // q2 per chunk: at most 2 GiB of folded vertex (and its image), at most 512 q2
+  // q2 per chunk: at most 2 GiB of folded vertex (and its image), at most 512 q2 (512 MiB up to 16 branches in
+  // FP64, the bound of the shared-memory builder)
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>({(size_t)512, (size_t)(q2e - q2b),
-                                                                (size_t(2) << 30) / per_q2}));
+                                                                (mma_q1 ? size_t(512) << 20 : size_t(2) << 30) / per_q2}));
   const int nchunks = (q2e - q2b + chunk - 1) / chunk;
   const size_t sz_dp = align_up(sizeof(double2) * nr3 * nb3 * chunk);
   const size_t sz_img = split ? align_up(wide::split_img_bytes(nb, Kp) * chunk) : 0;
@@ -2024,6 +2027,7 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
                                    st));
   }
   if (warp_q1) PHX_CUDA(ctx, wide::warp_set_attributes(nb, Kp, p->smearing));
+  else if (mma_q1) PHX_CUDA(ctx, wide::set_attributes_fp64_mma(nb, nr3, p->smearing));
   else PHX_CUDA(ctx, wide::set_attributes(nb, nr3, split));
   // q1 order: by window cut with a window (tiles of similar q2 sets), else the mesh order
   std::vector<int> order_h(nq);
@@ -2076,7 +2080,7 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
   A.skip_base = q2b;
   A.rt = nb > 24 ? 4 : 2;
   A.qp = wide::split_default_qp(nb, Kp);
-  const int grid = ctx->num_sms * wide::blocks_per_sm(nb, nr3, split);
+  const int grid = ctx->num_sms * (mma_q1 ? 1 : wide::blocks_per_sm(nb, nr3, split));
   // split path: the tile shape (register tile, q1 planes per contraction pass)
   // tuned once per problem shape on one chunk (PHX_TUNE=0: the defaults)
   int dev = 0;
@@ -2162,8 +2166,9 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
       g.pair_events.push_back(pe1);
       PHX_CUDA(ctx, phx_record_event(pe0, st));
       PHX_CUDA(ctx, warp_q1 ? wide::launch_warp_split(Ac, grid, st)
-                    : split ? wide::launch_split(Ac, grid, st)
-                            : wide::launch_fp64(Ac, grid, st));
+                    : split  ? wide::launch_split(Ac, grid, st)
+                    : mma_q1 ? wide::launch_fp64_mma(Ac, grid, st)
+                             : wide::launch_fp64(Ac, grid, st));
       PHX_CUDA(ctx, phx_record_event(pe1, st));
       ++launches;
     }
@@ -2265,9 +2270,12 @@ extern "C" int phx_ph_linewidths_d(phx_v3* v, phx_bands* b, const phx_lw_params*
   // against the nb = 6 kernels)
   if (env_on("PHX_WIDE")) return run_builder_wide(v, b, p, Aout_d, stats);
   if (v->nb == 6 && !p->window_energy) return run_builder<6>(v, b, p, Aout_d, stats);
-  // the split precisions and cells beyond 16 branches run on the many-branch
-  // builder; FP64 up to 16 branches (or with a window) on the shared-memory one
-  if (v->precision != PHX_PREC_FP64 || v->nb > kMaxNbGeneric) return run_builder_wide(v, b, p, Aout_d, stats);
+  // the split precisions, cells beyond 16 branches and FP64 where the tensor-pipe
+  // kernel fits run on the many-branch builder; FP64 with more R3 vectors (over
+  // 332 at 15 branches) or R2 vectors than that on the shared-memory one
+  if (v->precision != PHX_PREC_FP64 || v->nb > kMaxNbGeneric ||
+      (wide::q1_fp64_mma(v->nb, v->nr3) && wide::fold_smem(v->nb, v->nr2) <= 227 * 1024))
+    return run_builder_wide(v, b, p, Aout_d, stats);
   return run_builder_generic(v, b, p, Aout_d, stats);
 }
 

@@ -56,6 +56,10 @@ int blocks_per_sm(int nb, int nr3, bool split);
 int warp_q1(int nb, int Kp, int* tile_rows);
 cudaError_t warp_set_attributes(int nb, int Kp, int smearing);
 cudaError_t launch_warp_split(const Args& A, int grid, cudaStream_t st);
+// FP64 kernel on the FP64 tensor pipe, nb <= 16 (wide64.cu): its q1 per item (0: too many R3 vectors)
+int q1_fp64_mma(int nb, int nr3);
+cudaError_t set_attributes_fp64_mma(int nb, int nr3, int smearing);
+cudaError_t launch_fp64_mma(const Args& A, int grid, cudaStream_t st);
 // R2 fold of a chunk of q2 (sparse over the non-zero (r3, r2) blocks)
 size_t fold_smem(int nb, int max_list);
 cudaError_t launch_fold(int nb, int nr2, int nr3, const double* D3w, const int* r2_ofs, const int* r2_list,

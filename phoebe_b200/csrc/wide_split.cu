@@ -48,6 +48,7 @@
 #include "pair_common.cuh"
 #include "phx_consts.h"
 #include "tc.cuh"
+#include "warp_rates.cuh"
 #include "wide.cuh"
 
 using namespace pairc;
@@ -78,16 +79,12 @@ __host__ __device__ inline uint32_t tmem_cols(int nb, int nq) {
   return c;
 }
 
-// per-warp tables: E1, E3, their reciprocals, v3, 1/width of (q2 m2, -q2 m2),
-// sums (doubles); E1, E3 and limits of |e| (floats); blocks (bytes)
-__host__ __device__ inline int warp_bytes(int nb) { return (nb * (8 * (4 + 3 + 2 + kMaxT) + 4 * 4 + 6) + 15) / 16 * 16; }
-
 // 0 total: does not fit
 Layout make_layout(int nb, int Kp, int nq, bool es) {
   Layout L{};
   L.ldx = nb | 1;
   L.plane = nb * L.ldx;
-  L.warp_bytes = warp_bytes(nb);
+  L.warp_bytes = warprates::table_bytes(nb);
   // A stages hold several K steps (a handshake of producer and MMA thread costs
   // some 450 cycles, the MMAs of one K step 250): the most that leaves two stages
   const int nkc = Kp / kKC;
@@ -147,42 +144,9 @@ __device__ bool tile_live(const WideArgs& P, int tile, int iq2, int iq2m) {
   return false;
 }
 
-__device__ __forceinline__ bool state_ok(double e) { return e >= phxc::phExcludeCutoff && e >= phxc::phEnergyCutoff; }
-
-// s = sum_i (qT_i . dv)^2 of the adaptive width sqrt(s / 6); 0 for equal velocities
-__device__ __forceinline__ double width_sq(const double* qT, const double* a, const double* b) {
-  const double v0 = a[0] - b[0], v1 = a[1] - b[1], v2 = a[2] - b[2];
-  double s = 0.0;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const double d = qT[3 * i] * v0 + qT[3 * i + 1] * v1 + qT[3 * i + 2] * v2;
-    s += d * d;
-  }
-  return s;
-}
-
-// W averaged over `count` degenerate blocks (first band f, size z) of the index with stride `step`, a lane
-// per value of the other index (stride `line`)
-__device__ __forceinline__ void average_blocks(float* W, int line, int step, const uint8_t* f, const uint8_t* z,
-                                               int count, int nb, int lane) {
-  for (int t = 0; t < count; ++t) {
-    const int b = f[t], n = z[t];
-    for (int u = lane; u < nb; u += 32) {
-      float* w = W + u * line + b * step;
-      float sum = 0.f;
-      for (int k = 0; k < n; ++k) sum += w[k * step];
-      for (int k = 0; k < n; ++k) w[k * step] = sum / (float)n;
-    }
-  }
-}
-
 template <int NQ, int TR, int TC, bool ES, bool ADAPTIVE>
 __global__ void __launch_bounds__((NQ + 2) * 32, 1) wide_warp_kernel(WideArgs P, Layout L) {
   constexpr int kN = 2 * NQ;
-  // bits of a lane's live processes: 3 kinds x TR x TC cells
-  constexpr int kCells = TR * TC;
-  using Mask = typename std::conditional<3 * kCells <= 32, unsigned, unsigned long long>::type;
-  constexpr int kBits = 8 * sizeof(Mask), kWords = (3 * kCells + kBits - 1) / kBits;
   const MeshArgs& M = P.m;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((128 - (tc::smem_u32(smem_raw) & 127)) & 127);
@@ -344,23 +308,9 @@ __global__ void __launch_bounds__((NQ + 2) * 32, 1) wide_warp_kernel(WideArgs P,
     const unsigned kAll = 0xffffffffu;
     const int qd = warp & 3, grp = warp >> 2;
     const int lr = lane >> 2, lc = lane & 3;
-    const int nT = M.nT, nq = M.nq;
-    constexpr bool adaptive = ADAPTIVE;
+    const int nq = M.nq;
     const double sc = P.fp16 ? (double)fp16_scale(P.dmax) : 1.0;
-    const double rate0 = 0.5 * phxc::pi * 0.25 * M.norm / (sc * sc);
-    const double inv_sigma = adaptive ? 0.0 : 1.0 / M.sigma;
-    double* E1 = reinterpret_cast<double*>(smem + L.warp + (size_t)warp * L.warp_bytes);
-    double* E3 = E1 + nb;
-    double* R1 = E3 + nb;                 // 1 / E1
-    double* R3i = R1 + nb;                // 1 / E3
-    double* V3 = R3i + nb;
-    double* sq = V3 + 3 * nb;             // [nb][+, -] squared widths x 6
-    double* acc = sq + 2 * nb;          // [nb][kMaxT]
-    float* F1 = reinterpret_cast<float*>(acc + nb * kMaxT);   // E1, E3 in FP32
-    float* F3 = F1 + nb;
-    float* lim = F3 + nb;                 // [nb][+, -] bounds on |e|
-    uint8_t* blk = reinterpret_cast<uint8_t*>(lim + 2 * nb);   // first band and size: q1, q3, q2
-    uint8_t *f1 = blk, *z1 = blk + nb, *f3 = blk + 2 * nb, *z3 = blk + 3 * nb, *f2 = blk + 4 * nb, *z2 = blk + 5 * nb;
+    warprates::Vertex<float, TR, TC, ADAPTIVE> v(M, smem + L.warp + (size_t)warp * L.warp_bytes, lane, 1.0 / (sc * sc));
     float2* e1s = reinterpret_cast<float2*>(smem + L.ev) + (size_t)warp * 2 * nbb;
     float2* e3s = e1s + nbb;
     auto wait = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
@@ -415,85 +365,22 @@ __global__ void __launch_bounds__((NQ + 2) * 32, 1) wide_warp_kernel(WideArgs P,
       // tables of this q1 and its q3
       const float2* e1 = ES ? e1s : P.U32 + (size_t)q1c * nbb;
       const float2* e3 = ES ? e3s : P.U32 + (size_t)iq3 * nbb;
-      int blocks1 = 0, blocks3 = 0;
-      float tol = 0.f;
-      unsigned take = 0;   // a lane's states 1 (bits 0..) and 3 (bits 16..) that take part
+      v.q1 = q1c;
+      v.iq2 = iq2;
+      v.iq2m = iq2m;
+      v.iq3 = iq3;
+      v.inw = inw;
       if (inw) {
-        float em = 0.f;
-        for (int b = lane; b < nb; b += 32) {
-          const double x1 = M.E[(size_t)q1 * nb + b], x3 = M.E[(size_t)iq3 * nb + b];
-          E1[b] = x1;
-          E3[b] = x3;
-          R1[b] = 1.0 / x1;
-          R3i[b] = 1.0 / x3;
-          F1[b] = (float)x1;
-          F3[b] = (float)x3;
-          em = fmaxf(em, fmaxf(fabsf((float)x1), fabsf((float)x3)));
-          em = fmaxf(em, (float)fmax(fabs(M.E[(size_t)iq2 * nb + b]), fabs(M.E[(size_t)iq2m * nb + b])));
-        }
-        // three FP32 energies and their sum are within 4.2e-7 of the largest energy of the FP64 one
-        tol = 1e-6f * __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(em)));
-        if (adaptive)
-          for (int e = lane; e < 3 * nb; e += 32) V3[e] = M.vg[(size_t)iq3 * 3 * nb + e];
-        for (int e = lane; e < nb * kMaxT; e += 32) acc[e] = 0.0;
         if (ES)
           for (int e = lane; e < nbb; e += 32) {
             e1s[e] = P.U32[(size_t)q1 * nbb + e];
             e3s[e] = P.U32[(size_t)iq3 * nbb + e];
           }
-        __syncwarp();
-        // forward-scan degenerate blocks (scattering.cpp:1223,1257,1291): those of q1 and q3
-        // as lists of the blocks of two and more, those of q2 for every band
-        int count = 0;
-        if (lane < 3) {
-          const double* e = lane == 0 ? E1 : lane == 1 ? E3 : M.E + (size_t)iq2 * nb;
-          uint8_t *f = blk + 2 * lane * nb, *z = f + nb;
-          for (int b = 0; b < nb;) {
-            const double e0 = e[b];
-            int end = b + 1;
-            while (end < nb && fabs(e0 - e[end]) < phxc::degThreshold) ++end;
-            if (lane < 2) {
-              if (end - b > 1) {
-                f[count] = (uint8_t)b;
-                z[count++] = (uint8_t)(end - b);
-              }
-            } else {
-              for (int k = b; k < end; ++k) {
-                f[k] = (uint8_t)b;
-                z[k] = (uint8_t)(end - b);
-              }
-            }
-            b = end;
-          }
-        }
-        blocks1 = __shfl_sync(kAll, count, 0);
-        blocks3 = __shfl_sync(kAll, count, 1);
-        __syncwarp();
-        for (int i = 0; i < TR; ++i)
-          if (lr + 8 * i < nb && state_ok(E1[lr + 8 * i])) take |= 1u << i;
-        for (int k = 0; k < TC; ++k)
-          if (lc + 4 * k < nb && !(E3[lc + 4 * k] < phxc::phEnergyCutoff)) take |= 0x10000u << k;
+        v.load();
       }
-      // squared widths of (q2 m2, q3 b3) and (-q2 m2, q3 b3) and the bounds on |e|
-      // (FP32 square root, widened beyond its error: the evaluation tests exactly)
-      auto width_table = [&](int m2) {
-        __syncwarp();   // the previous table has been read
-        for (int e = lane; e < 2 * nb; e += 32) {
-          if (adaptive) {
-            const double s2 = width_sq(M.qT, M.vg + ((size_t)(e & 1 ? iq2m : iq2) * nb + m2) * 3, V3 + 3 * (e >> 1));
-            sq[e] = s2;
-            lim[e] = s2 == 0.0 ? tol
-                               : fmaxf(__fsqrt_rn((float)s2) * (float)(2.0 * 0.4082482904638631 * 1.00001),
-                                       (float)(2.0 * phxc::adaptiveCutoff * 1.00001)) + tol;
-          } else {
-            lim[e] = (float)(6.00001 * M.sigma) + tol;
-          }
-        }
-        __syncwarp();
-      };
       bool ok = true;
       for (int b2 = 0; b2 < nb; ++b2, ++s) {
-        if (inw) width_table(f2[b2]);
+        if (inw) v.width_table(v.f2[b2]);   // ahead of the waits
         const int buf = s & 1, tbuf = L.tb == 2 ? buf : 0;
         float2* Tb = reinterpret_cast<float2*>(smem + L.T) + (size_t)tbuf * NQ * L.plane;
         if (L.tb == 1 && s > 0 && !wait(consumed, (s - 1) & 1, 1 << 17)) { ok = false; break; }
@@ -502,15 +389,15 @@ __global__ void __launch_bounds__((NQ + 2) * 32, 1) wide_warp_kernel(WideArgs P,
         // drain: TMEM lane = row (a, c) of an M tile, columns 2q, 2q + 1 = re, im
         for (int t = grp; t < mt_n * (NQ / 8); t += NQ / 4) {
           const int mt = t / (NQ / 8), cg = t % (NQ / 8);
-          float v[16];
+          float d[16];
           const uint32_t ta = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)buf * bufcols + (uint32_t)(mt * kN + cg * 16);
-          tc::tmem_ld8(ta, v);
-          tc::tmem_ld8(ta + 8, v + 8);
-          tc::tmem_wait_ld<16>(v);
+          tc::tmem_ld8(ta, d);
+          tc::tmem_ld8(ta + 8, d + 8);
+          tc::tmem_wait_ld<16>(d);
           const int row = mt * 128 + qd * 32 + lane;
           if (row < nbb) {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) Tb[(size_t)(cg * 8 + q) * L.plane + row] = make_float2(v[2 * q], v[2 * q + 1]);
+            for (int q = 0; q < 8; ++q) Tb[(size_t)(cg * 8 + q) * L.plane + row] = make_float2(d[2 * q], d[2 * q + 1]);
           }
         }
         tc::tc_fence_before();
@@ -589,121 +476,14 @@ __global__ void __launch_bounds__((NQ + 2) * 32, 1) wide_warp_kernel(WideArgs P,
               if (lr + 8 * i < nb && lc + 4 * k < nb)
                 W[(lr + 8 * i) * ldx + lc + 4 * k] = w[i][k].x * w[i][k].x + w[i][k].y * w[i][k].y;
           __syncwarp();
-          // symmetrizeCoupling (scattering.cpp:1209-1318): the blocks of b3, then of b1
-          if (blocks3) {
-            average_blocks(W, ldx, 1, f3, z3, blocks3, nb, lane);
-            __syncwarp();
-          }
-          if (blocks1) {
-            average_blocks(W, 1, ldx, f1, z1, blocks1, nb, lane);
-            __syncwarp();
-          }
-
-          // rates; the block of b2 enters as its members' average
-          const int n2 = z2[b2];
-#pragma unroll 1
-          for (int d2 = 0; d2 < n2; ++d2) {
-            const int m2 = f2[b2] + d2;
-            const double en2 = M.E[(size_t)iq2 * nb + m2], en2m = M.E[(size_t)iq2m * nb + m2];
-            const bool okp = (inw & 1) && state_ok(en2), okm = (inw & 2) && state_ok(en2m);
-            if (!okp && !okm) continue;
-            if (d2 > 0) width_table(m2);   // member 0's was made before the waits
-            const float f2p = (float)en2, f2m = (float)en2m;
-            // lower end of e: a Gaussian below x = -27.4 is under the smallest FP64 number
-            const float low = (float)(27.4 * M.sigma) + tol;
-            const double i2p = rate0 / (en2 * (double)n2), i2m = rate0 / (en2m * (double)n2);
-            // live cells, bit kCells kind + TC i + k: processes delta(E_A + E_B - E_C) with C = 3 ("+"), 2, 1 ("-")
-            Mask live[kWords];
-#pragma unroll
-            for (int u = 0; u < kWords; ++u) live[u] = 0;
-            auto mark = [&](int bit) { live[bit / kBits] |= (Mask)1 << (bit % kBits); };
-            float x1[TR], dif[TR];
-#pragma unroll
-            for (int i = 0; i < TR; ++i) {
-              const float f = F1[lr + 8 * i];
-              x1[i] = f + f2p;
-              dif[i] = f - f2m;
-            }
-#pragma unroll
-            for (int k = 0; k < TC; ++k) {
-              const float x3 = F3[lc + 4 * k];
-              const float2 lm = *reinterpret_cast<const float2*>(lim + 2 * (lc + 4 * k));
-#pragma unroll
-              for (int i = 0; i < TR; ++i) {
-                const float a = x1[i] - x3, b = dif[i] + x3, c = x3 - dif[i];
-                if (ADAPTIVE ? fabsf(a) <= lm.x : (a <= lm.x && a >= -low)) mark(TC * i + k);
-                if (ADAPTIVE ? fabsf(b) <= lm.y : (b <= lm.y && b >= -low)) mark(kCells + TC * i + k);
-                if (ADAPTIVE ? fabsf(c) <= lm.y : (c <= lm.y && c >= -low)) mark(2 * kCells + TC * i + k);
-              }
-            }
-            Mask keep[kWords];
-#pragma unroll
-            for (int u = 0; u < kWords; ++u) keep[u] = 0;
-#pragma unroll
-            for (int kd = 0; kd < 3; ++kd)
-#pragma unroll
-              for (int i = 0; i < TR; ++i) {
-                const Mask bits = (take >> i & 1) && (kd ? okm : okp) ? (Mask)(take >> 16) : (Mask)0;
-                const int at = kd * kCells + TC * i;
-                keep[at / kBits] |= bits << (at % kBits);
-                if (at % kBits + TC > kBits) keep[at / kBits + 1] |= bits >> (kBits - at % kBits);
-              }
-#pragma unroll
-            for (int u = 0; u < kWords; ++u) live[u] &= keep[u];
-#pragma unroll 1
-            for (;;) {
-              int t = -1;
-#pragma unroll
-              for (int u = kWords - 1; u >= 0; --u)
-                if (live[u]) t = kBits * u + (sizeof(Mask) == 8 ? __ffsll(live[u]) : __ffs((int)live[u])) - 1;
-              if (t < 0) break;
-#pragma unroll
-              for (int u = 0; u < kWords; ++u)
-                if (t / kBits == u) live[u] &= live[u] - 1;
-              const int kind = t / kCells, cell = t - kCells * kind, i = cell / TC, k = cell - TC * i;
-              const int b1 = lr + 8 * i, b3 = lc + 4 * k;
-              const double y1 = E1[b1], y2 = kind ? en2m : en2, y3 = E3[b3];
-              const double e = kind == 0 ? y1 + y2 - y3 : kind == 1 ? y1 + y3 - y2 : y2 + y3 - y1;
-              double d = (double)W[b1 * ldx + b3] * (kind ? i2m : i2p) * (R1[b1] * R3i[b3]);
-              if (adaptive) {
-                const double s6 = sq[2 * b3 + (kind ? 1 : 0)] * (1.0 / 6.0);
-                double inv = rsqrt(s6), sg = s6 * inv;
-                if (sg < phxc::adaptiveCutoff) {
-                  sg = phxc::adaptiveCutoff;
-                  inv = 1.0 / phxc::adaptiveCutoff;
-                }
-                const double x = e * inv;
-                // the Gaussian in FP32 (1e-7): |V|^2 carries 1e-6
-                double g = (double)expf((float)(-x * x)) * (inv * (1.0 / (phxc::sqrtPi * phxc::erf2)));
-                if (fabs(e) > 2.0 * sg) g = 0.0;
-                if (s6 == 0.0) g = e == 0.0 ? 1.0 : 0.0;   // equal velocities
-                d *= g;
-              } else {
-                const double x = e * inv_sigma;
-                d *= x > 6.0 ? 0.0 : exp(-x * x) * (inv_sigma * (1.0 / phxc::sqrtPi));
-              }
-              if (d != 0.0)
-                for (int c = 0; c < nT; ++c) {
-                  const double* B = M.bose + (size_t)c * nq * nb;
-                  const double n1 = B[(size_t)q1 * nb + b1], nn2 = B[(size_t)(kind ? iq2m : iq2) * nb + m2],
-                               n3 = B[(size_t)iq3 * nb + b3];
-                  const double a = kind == 2 ? n3 : n1, b = kind == 1 ? n3 : nn2,
-                               z = kind == 0 ? n3 : kind == 1 ? nn2 : n1;
-                  atomicAdd(&acc[b1 * kMaxT + c], d * a * b * (z + 1.0));
-                }
-            }
-          }
+          v.symmetrize(W, ldx);
+          v.rates(b2, W, ldx);
         }
         __syncwarp();
         if (L.tb == 1 && lane == 0) tc::mbar_arrive(consumed);
       }
       if (!ok) { *abort_flag = 1; break; }
-      if (inw)
-        for (int e = lane; e < nb * nT; e += 32) {
-          const int b1 = e / nT, c = e % nT;
-          const double v = acc[b1 * kMaxT + c];
-          if (v != 0.0) atomicAdd(&P.lw[((size_t)q1 * nb + b1) * nT + c], v);
-        }
+      if (inw) v.flush(P.lw);
       __syncwarp();
     }
   }

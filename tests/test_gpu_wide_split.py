@@ -3,10 +3,12 @@ classes of tile and of its lanes' tiles, against the FP64 builder on the same ba
 split paths' bar of 1e-5 on linewidths above 1e-8 of the largest.  Cells of 1 to 12 atoms (the
 twelve-atom cell's first atoms), q1 counts that are no multiple of an item, R3 counts of one K step
 and of several A stages, q2 windows, both smearings, and an R3 count that leaves no room for the
-kernel (the older one takes over)."""
+kernel (the older one takes over).  The FP64 builder itself, whose kernel for up to 16 branches runs
+on the FP64 tensor pipe, against the oracle at the 1e-10 of the other FP64 linewidth tests."""
 import numpy as np
 import pytest
 
+import oracle
 from phoebe_b200 import constants as C
 from phoebe_b200 import lattice, synth
 
@@ -19,7 +21,7 @@ def _cell(nat):
 
 
 def _fc3(cr, nr3):
-    R, _ = synth.lattice_cube(cr, 2)
+    R, _ = synth.lattice_cube(cr, 3)
     rng = np.random.default_rng(nr3)
     o = np.argsort(np.linalg.norm(R, axis=1), kind="stable")
     nat, nb = cr.num_atoms, cr.num_bands
@@ -47,7 +49,7 @@ def _bands(ctx, cr, mesh, rng):
     own = i == neg
     U[own] = np.linalg.qr(rng.normal(size=(own.sum(), nb, nb)))[0]
     V[own] = 0.0
-    return E, BandStructure.from_arrays(ctx, mesh, cr.reciprocal_cell, E, U, V)
+    return E, U, V, BandStructure.from_arrays(ctx, mesh, cr.reciprocal_cell, E, U, V)
 
 
 @pytest.mark.parametrize("smearing", ["adaptive", "gaussian"])
@@ -58,7 +60,7 @@ def _bands(ctx, cr, mesh, rng):
 def test_split_matches_fp64(ctx, nat, mesh, nr3, window, smearing):
     from phoebe_b200.core import Interaction3Ph, PhScatteringMatrix
     cr = _cell(nat)
-    E, bands = _bands(ctx, cr, mesh, np.random.default_rng(nat))
+    E, _, _, bands = _bands(ctx, cr, mesh, np.random.default_rng(nat))
     fc3 = _fc3(cr, nr3)
     T = np.array([C.kelvin_to_ry(t) for t in (100.0, 300.0, 600.0)])
     win = synth.q2_window(E, mesh) if window else None
@@ -79,4 +81,26 @@ def test_split_matches_fp64(ctx, nat, mesh, nr3, window, smearing):
     for precision in ("split_fp16", "split_bf16"):
         assert np.isfinite(out[precision]).all()
         assert (np.abs(out[precision] - A)[big] / np.abs(A)[big]).max() < 1e-5, precision
+    bands.close()
+
+
+@pytest.mark.parametrize("smearing", ["adaptive", "gaussian"])
+@pytest.mark.parametrize("nat,mesh,nr3,window", [(1, (3, 2, 2), 1, False), (2, (5, 4, 1), 4, True), (3, (3, 3, 2), 27, False),
+                                                 (5, (3, 2, 2), 67, True), (5, (3, 2, 1), 130, False),
+                                                 (5, (3, 1, 1), 343, True)])
+def test_fp64_matches_oracle(ctx, nat, mesh, nr3, window, smearing):
+    from phoebe_b200.core import Interaction3Ph, PhScatteringMatrix
+    cr = _cell(nat)
+    E, U, V, bands = _bands(ctx, cr, mesh, np.random.default_rng(nat))
+    fc3 = _fc3(cr, nr3)
+    T = np.array([C.kelvin_to_ry(t) for t in (100.0, 300.0)])
+    win = synth.q2_window(E, mesh) if window else None
+    v3 = Interaction3Ph(ctx, cr, fc3)
+    A = PhScatteringMatrix(v3, bands, T, smearing, 1e-4, window=win).setup()
+    v3.close()
+    q = lattice.Mesh(cr, mesh).cartesian_coords()
+    ref = oracle.Interaction3Ph(cr, fc3).linewidths(mesh, E, U, V, q, cr.reciprocal_cell, T, smearing, 1e-4, window=win)
+    big = np.abs(ref) > 1e-8 * np.abs(ref).max()
+    assert big.any()
+    assert (np.abs(A - ref)[big] / np.abs(ref)[big]).max() < 1e-10
     bands.close()
