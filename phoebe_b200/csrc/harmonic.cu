@@ -113,6 +113,28 @@ __global__ void ph_bands_kernel(H0Dev h, int nq, const double* __restrict__ qs,
         double qq[3] = {q[0], q[1], q[2]};
         qq[dir] += sgn == 0 ? delta : -delta;
         build_dyn(h, qq, s);
+        // in the eigenbasis of q, H = U0^H D U0, hermitised: diagonal up to the
+        // step, so the sweeps are few, and the velocity operator is in the
+        // basis where it is wanted
+        for (int e = tid; e < nb * nb; e += NT) {
+          const int i = e / nb, j = e % nb;
+          double2 acc = cmk(0.0, 0.0);
+          for (int l = 0; l < nb; ++l) cfma(acc, s.H[i * nb + l], s.U0[l * nb + j]);
+          s.T[e] = acc;
+        }
+        __syncthreads();
+        for (int e = tid; e < nb * nb; e += NT) {
+          const int i = e / nb, j = e % nb;
+          double2 acc = cmk(0.0, 0.0);
+          for (int l = 0; l < nb; ++l) cfma(acc, cconj(s.U0[l * nb + i]), s.T[l * nb + j]);
+          s.V[e] = acc;
+        }
+        __syncthreads();
+        for (int e = tid; e < nb * nb; e += NT) {
+          const int i = e / nb, j = e % nb;
+          s.H[e] = cscale(cadd(s.V[e], cconj(s.V[j * nb + i])), 0.5);
+        }
+        __syncthreads();
         if (team_jacobi(nb, nb, s) < 0 && tid == 0) atomicOr(status, 1);
         for (int b = tid; b < nb; b += NT) {
           const double w2 = s.E1[b];
@@ -129,7 +151,7 @@ __global__ void ph_bands_kernel(H0Dev h, int nq, const double* __restrict__ qs,
         }
         __syncthreads();
       }
-      // hermitise (der/2d), then T = DERh U0 and H = U0^H T
+      // velocity operator of this direction: der / 2d, hermitised
       for (int e = tid; e < nb * nb; e += NT) {
         const int i = e / nb, j = e % nb;
         const double2 a = cscale(s.DER[i * nb + j], 1.0 / (2.0 * delta));
@@ -137,19 +159,7 @@ __global__ void ph_bands_kernel(H0Dev h, int nq, const double* __restrict__ qs,
         s.H[e] = cscale(cadd(a, cconj(b)), 0.5);
       }
       __syncthreads();
-      for (int e = tid; e < nb * nb; e += NT) {
-        const int i = e / nb, j = e % nb;
-        double2 acc = cmk(0.0, 0.0);
-        for (int l = 0; l < nb; ++l) cfma(acc, s.H[i * nb + l], s.U0[l * nb + j]);
-        s.T[e] = acc;
-      }
-      __syncthreads();
-      for (int e = tid; e < nb * nb; e += NT) {
-        const int i = e / nb, j = e % nb;
-        double2 acc = cmk(0.0, 0.0);
-        for (int l = 0; l < nb; ++l) cfma(acc, cconj(s.U0[l * nb + i]), s.T[l * nb + j]);
-        s.DER[e] = acc;  // velocity operator for this direction
-      }
+      for (int e = tid; e < nb * nb; e += NT) s.DER[e] = s.H[e];
       __syncthreads();
       for (int b = tid; b < nb; b += NT) s.VG[b] = s.DER[b * nb + b].x;
       __syncthreads();

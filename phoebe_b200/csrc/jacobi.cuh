@@ -93,8 +93,9 @@ __device__ inline int team_jacobi(int n, int ld, const Smem& s) {
   bool done = (n < 2);
   while (!done) {
     if (sweep >= kMaxSweeps) return -1;
-    double rotated = 0.0;
+    bool rotated = false;
     for (int r = 0; r < np - 1; ++r) {
+      int active = 0;
       for (int k = tid; k < npair; k += NT) {
         int p, q;
         if (k == 0) {
@@ -123,12 +124,14 @@ __device__ inline int team_jacobi(int n, int ld, const Smem& s) {
             ro.ph = cmk(b.x / mb, b.y / mb);
             ro.ap = a - t * mb;
             ro.dq = d + t * mb;
-            ro.active = 1;
+            ro.active = active = 1;
           }
         }
         s.rot[k] = ro;
       }
-      __syncthreads();
+      // a step without a rotation (most of the last sweeps) ends here
+      if (!__syncthreads_or(active)) continue;
+      rotated = true;
       // rows: p' = c p - s e^{i phi} q ; q' = s e^{-i phi} p + c q
       for (int idx = tid; idx < npair * n; idx += NT) {
         const Rot ro = s.rot[idx / n];
@@ -169,12 +172,11 @@ __device__ inline int team_jacobi(int n, int ld, const Smem& s) {
         H[ro.q * ld + ro.q] = cmk(ro.dq, 0.0);
         H[ro.p * ld + ro.q] = cmk(0.0, 0.0);
         H[ro.q * ld + ro.p] = cmk(0.0, 0.0);
-        rotated = 1.0;
       }
       __syncthreads();
     }
     ++sweep;
-    done = team_reduce_max(rotated, s.red) == 0.0;
+    done = !rotated;
   }
   // ascending order (stable rank sort)
   for (int i = tid; i < n; i += NT) {
