@@ -339,6 +339,9 @@ struct ElArgs {
   double* out;             // (nT, nk1, nw)
   const float2* g3in;      // precomputed g3 of this k1, g3in[x * g3ld + q], or null
   int g3ld;
+  // the batch's final states with active bands: (row of the batch, q, k2, nb2), *count of them
+  int4* list;
+  int* count;
 };
 
 // adaptive width of a (k1 b1, k2 b2) pair from v = v1 - v2 (delta_function.cpp:65-88);
@@ -380,6 +383,31 @@ __device__ __forceinline__ double el_delta_tab(double ginv, double e, double2 w)
   return exp(-x * x) * w.y * (1.0 / (phxc::sqrtPi * phxc::erf2));
 }
 
+// Final states k2 = k1 + q of the batch's k1 (blockIdx.y) that have active
+// bands, in no fixed order.  With a window around the Fermi level most have none
+// (84% of them with +-0.3 eV on 8 bands of 2 eV hoppings), and a block of the
+// pair kernel for each of those cost more than the pairs: 255 -> 61 us per 16 k1.
+__global__ void __launch_bounds__(256) el_list_kernel(ElArgs A) {
+  const int iq = blockIdx.x * blockDim.x + threadIdx.x, jb = blockIdx.y;
+  const int ik1 = A.ik1s[jb];
+  int nb2 = 0, ik2 = 0;
+  if (iq < A.qmesh[0] * A.qmesh[1] * A.qmesh[2]) {
+    const int x1 = ik1 % A.kmesh[0], y1 = (ik1 / A.kmesh[0]) % A.kmesh[1], z1 = ik1 / (A.kmesh[0] * A.kmesh[1]);
+    const int f0 = A.kmesh[0] / A.qmesh[0], f1 = A.kmesh[1] / A.qmesh[1], f2 = A.kmesh[2] / A.qmesh[2];
+    const int qx = iq % A.qmesh[0], qy = (iq / A.qmesh[0]) % A.qmesh[1], qz = iq / (A.qmesh[0] * A.qmesh[1]);
+    ik2 = (x1 + f0 * qx) % A.kmesh[0] +
+          A.kmesh[0] * ((y1 + f1 * qy) % A.kmesh[1] + A.kmesh[1] * ((z1 + f2 * qz) % A.kmesh[2]));
+    nb2 = A.hi[ik2] - A.lo[ik2];
+  }
+  const unsigned have = __ballot_sync(0xffffffffu, nb2 > 0);
+  if (!have) return;
+  const int lane = threadIdx.x & 31;
+  int first = 0;
+  if (lane == 0) first = atomicAdd(A.count, __popc(have));
+  first = __shfl_sync(0xffffffffu, first, 0);
+  if (nb2 > 0) A.list[first + __popc(have & ((1u << lane) - 1u))] = make_int4(jb, iq, ik2, nb2);
+}
+
 // G3IN: g3 from the tensor-core GEMM (split path); SM: the smearing.  Each
 // combination is its own instantiation, which keeps the kernel's code small.
 template <bool G3IN, int SM>
@@ -389,167 +417,156 @@ __global__ void __launch_bounds__(kPairThreads) el_pair_kernel(ElArgs A) {
   // no phase buffer when g3 comes from the tensor-core GEMM
   const PairSmem s = pair_carve(sraw, G3IN ? 0 : nRp, nph, nw);
   const int tid = threadIdx.x, NT = blockDim.x;
-  const int nq = A.qmesh[0] * A.qmesh[1] * A.qmesh[2];
-  const int jb = blockIdx.y;
-  const int ik1 = A.ik1s[jb], i1 = A.i1s[jb], lo1 = A.lo[ik1], nb1 = A.hi[ik1] - lo1;
-  const double2* cached = A.cached + (size_t)jb * A.cper;
-  const float2* g3in = G3IN ? A.g3in + A.g3offs[jb] : nullptr;
-  const int x1 = ik1 % A.kmesh[0], y1 = (ik1 / A.kmesh[0]) % A.kmesh[1], z1 = ik1 / (A.kmesh[0] * A.kmesh[1]);
-  const int f0 = A.kmesh[0] / A.qmesh[0], f1 = A.kmesh[1] / A.qmesh[1], f2 = A.kmesh[2] / A.qmesh[2];
-  const double* E1 = A.Ek + (size_t)ik1 * nw + lo1;
-  for (int i = tid; i < kMaxW * pairc::kMaxT; i += NT) s.acc[i] = 0.0;
-  // final states of this block
-  if (tid < kQT) {
-    const int iq = blockIdx.x * kQT + tid;
-    int valid = 0, nb2 = 0, ik2 = 0;
-    if (iq < nq) {
-      const int qx = iq % A.qmesh[0], qy = (iq / A.qmesh[0]) % A.qmesh[1], qz = iq / (A.qmesh[0] * A.qmesh[1]);
-      ik2 = (x1 + f0 * qx) % A.kmesh[0] +
-            A.kmesh[0] * ((y1 + f1 * qy) % A.kmesh[1] + A.kmesh[1] * ((z1 + f2 * qz) % A.kmesh[2]));
-      nb2 = A.hi[ik2] - A.lo[ik2];
-      valid = nb2 > 0;
+  static_assert(kQT == 1, "one final state of the list per block and pass");
+  const int count = *A.count;
+  for (int item = blockIdx.x; item < count; item += gridDim.x) {
+    const int4 fs = A.list[item];
+    const int jb = fs.x;
+    const int ik1 = A.ik1s[jb], i1 = A.i1s[jb], lo1 = A.lo[ik1], nb1 = A.hi[ik1] - lo1;
+    const double2* cached = A.cached + (size_t)jb * A.cper;
+    const float2* g3in = G3IN ? A.g3in + A.g3offs[jb] : nullptr;
+    const double* E1 = A.Ek + (size_t)ik1 * nw + lo1;
+    __syncthreads();   // the previous final state's sums have been read
+    for (int i = tid; i < kMaxW * pairc::kMaxT; i += NT) s.acc[i] = 0.0;
+    if (tid == 0) {
+      s.info[0] = 1;
+      s.info[1] = fs.w;
+      s.info[2] = fs.z;
+      s.info[3] = fs.y;
     }
-    s.info[4 * tid] = valid;
-    s.info[4 * tid + 1] = valid ? nb2 : 0;
-    s.info[4 * tid + 2] = ik2;
-    s.info[4 * tid + 3] = iq;
-  }
-  __syncthreads();
-  int any_valid = 0;
-#pragma unroll
-  for (int q = 0; q < kQT; ++q) any_valid |= s.info[4 * q];
-  if (!any_valid) return;
-  // phases e^{+i q3.Rp}/deg with q3 = k2 - k1 (helper_el_scattering.cpp:233-234),
-  // not needed when g3 comes from the tensor-core GEMM
-  for (int i = tid; i < (G3IN ? 0 : kQT * nRp); i += NT) {
-    const int q = i / nRp, r = i % nRp;
-    double2 v = cmk(0.0, 0.0);
-    if (s.info[4 * q]) {
-      const int ik2 = s.info[4 * q + 2];
-      double q3[3];
-      for (int c = 0; c < 3; ++c) q3[c] = A.kcart[3 * ik2 + c] - A.kcart[3 * ik1 + c];
-      double sn, cs;
-      sincos(q3[0] * A.Rp[3 * r] + q3[1] * A.Rp[3 * r + 1] + q3[2] * A.Rp[3 * r + 2], &sn, &cs);
-      v = cmk(cs / A.degP[r], sn / A.degP[r]);
-    }
-    s.ph[i] = v;
-  }
-  for (int i = tid; i < kQT * nw * kMaxW; i += NT) {
-    const int q = i / (nw * kMaxW), w = (i / kMaxW) % nw, b2 = i % kMaxW;
-    double2 v = cmk(0.0, 0.0);
-    if (s.info[4 * q] && b2 < s.info[4 * q + 1]) {
-      const int ik2 = s.info[4 * q + 2];
-      v = A.Uk[((size_t)ik2 * nw + w) * nw + A.lo[ik2] + b2];
-    }
-    s.U2[i] = v;
-  }
-  for (int i = tid; i < kQT * nph * nph; i += NT) {
-    const int q = i / (nph * nph);
-    s.ev3[i] = s.info[4 * q] ? A.evq[(size_t)s.info[4 * q + 3] * nph * nph + i % (nph * nph)] : cmk(0.0, 0.0);
-  }
-  for (int i = tid; i < kQT * kMaxW; i += NT) {
-    const int q = i / kMaxW, b2 = i % kMaxW;
-    s.E2[i] = (s.info[4 * q] && b2 < s.info[4 * q + 1]) ? A.Ek[(size_t)s.info[4 * q + 2] * nw + A.lo[s.info[4 * q + 2]] + b2] : 0.0;
-  }
-  for (int i = tid; i < kQT * nph; i += NT) {
-    const int q = i / nph;
-    s.E3[i] = s.info[4 * q] ? A.Eq[(size_t)s.info[4 * q + 3] * nph + i % nph] : 0.0;
-  }
-  // populations of the final states (el_scattering.cpp:287-300)
-  for (int i = tid; i < kQT * kMaxW * A.nT; i += NT) {
-    const int t = i % A.nT, b2 = (i / A.nT) % kMaxW, q = i / (A.nT * kMaxW);
-    double f = 0.0;
-    if (s.info[4 * q] && b2 < s.info[4 * q + 1]) {
-      const double T = A.temps[t];
-      const int ik2 = s.info[4 * q + 2];
-      const double en2 = A.Ek[(size_t)ik2 * nw + A.lo[ik2] + b2];
-      if (T <= 0.0) {
-        f = en2 <= A.mu ? 1.0 : 0.0;
-      } else {
-        f = 1.0 / (exp((en2 - A.mu) / T) + 1.0);
-        f = fmin(1.0, fmax(0.0, f));
+    __syncthreads();
+    // phases e^{+i q3.Rp}/deg with q3 = k2 - k1 (helper_el_scattering.cpp:233-234),
+    // not needed when g3 comes from the tensor-core GEMM
+    for (int i = tid; i < (G3IN ? 0 : kQT * nRp); i += NT) {
+      const int q = i / nRp, r = i % nRp;
+      double2 v = cmk(0.0, 0.0);
+      if (s.info[4 * q]) {
+        const int ik2 = s.info[4 * q + 2];
+        double q3[3];
+        for (int c = 0; c < 3; ++c) q3[c] = A.kcart[3 * ik2 + c] - A.kcart[3 * ik1 + c];
+        double sn, cs;
+        sincos(q3[0] * A.Rp[3 * r] + q3[1] * A.Rp[3 * r + 1] + q3[2] * A.Rp[3 * r + 2], &sn, &cs);
+        v = cmk(cs / A.degP[r], sn / A.degP[r]);
       }
+      s.ph[i] = v;
     }
-    s.f2[(q * kMaxW + b2) * pairc::kMaxT + t] = f;
-  }
-  for (int i = tid; i < kQT * nph * A.nT; i += NT) {
-    const int t = i % A.nT, nu = (i / A.nT) % nph, q = i / (A.nT * nph);
-    double n = 0.0;
-    const double T = A.temps[t];
-    if (s.info[4 * q] && T > 0.0) {
-      n = 1.0 / (exp(A.Eq[(size_t)s.info[4 * q + 3] * nph + nu] / T) - 1.0);
-      if (n < 0.0) n = 0.0;
+    for (int i = tid; i < kQT * nw * kMaxW; i += NT) {
+      const int q = i / (nw * kMaxW), w = (i / kMaxW) % nw, b2 = i % kMaxW;
+      double2 v = cmk(0.0, 0.0);
+      if (s.info[4 * q] && b2 < s.info[4 * q + 1]) {
+        const int ik2 = s.info[4 * q + 2];
+        v = A.Uk[((size_t)ik2 * nw + w) * nw + A.lo[ik2] + b2];
+      }
+      s.U2[i] = v;
     }
-    s.n3[(q * kMaxPh + nu) * pairc::kMaxT + t] = n;
-  }
-  // adaptive widths of the (b1, b2) pairs (delta_function.cpp:65-88), floored,
-  // as (sigma, 1/sigma) with the zero-velocity flag in the sign bit of sigma
-  for (int x = tid; x < (SM == PHX_SMEAR_ADAPTIVE ? kQT * kMaxW * kMaxW : 0); x += NT) {
-    const int b2 = x % kMaxW, b1 = (x / kMaxW) % kMaxW, q = x / (kMaxW * kMaxW);
-    double2 wv = make_double2(0.0, 0.0);
-    if (s.info[4 * q] && b1 < nb1 && b2 < s.info[4 * q + 1]) {
-      const int ik2 = s.info[4 * q + 2];
-      double v[3];
-      for (int c = 0; c < 3; ++c)
-        v[c] = A.vk[((size_t)ik1 * nw + lo1 + b1) * 3 + c] - A.vk[((size_t)ik2 * nw + A.lo[ik2] + b2) * 3 + c];
-      const ElWidth w = el_width(A, v);
-      double sg = w.sg;
-      if (sg != 0.0 && sg < phxc::adaptiveCutoff) sg = phxc::adaptiveCutoff;
-      wv = make_double2(w.vzero ? -0.0 : sg, sg > 0.0 ? 1.0 / sg : 0.0);
+    for (int i = tid; i < kQT * nph * nph; i += NT) {
+      const int q = i / (nph * nph);
+      s.ev3[i] = s.info[4 * q] ? A.evq[(size_t)s.info[4 * q + 3] * nph * nph + i % (nph * nph)] : cmk(0.0, 0.0);
     }
-    s.wd[x] = wv;
-  }
-  __syncthreads();
-  pair_couplings<G3IN>(cached, nRp, nph, nw, nb1, s, g3in, A.g3ld);
-  pair_symmetrize(E1, nb1, nph, s);
-  // rates (el_scattering.cpp:268-327), one thread per (b1, q, b2, nu) with b1
-  // slowest: when the kQT * kMaxW * nph entries of one b1 fill whole warps
-  // (nph even), a warp reduces its rates and adds them once; otherwise every
-  // thread adds its own
-  const int per_b1 = kQT * kMaxW * nph;
-  const bool warp_sums = per_b1 % 32 == 0;
-  const double ginv = SM == PHX_SMEAR_GAUSSIAN ? 1.0 / A.sigma : 0.0;
-  for (int x = tid; x < nb1 * per_b1; x += NT) {
-    const int nu = x % nph, b2 = (x / nph) % kMaxW, q = (x / (nph * kMaxW)) % kQT, b1 = x / per_b1;
-    double r[pairc::kMaxT];
+    for (int i = tid; i < kQT * kMaxW; i += NT) {
+      const int q = i / kMaxW, b2 = i % kMaxW;
+      s.E2[i] = (s.info[4 * q] && b2 < s.info[4 * q + 1]) ? A.Ek[(size_t)s.info[4 * q + 2] * nw + A.lo[s.info[4 * q + 2]] + b2] : 0.0;
+    }
+    for (int i = tid; i < kQT * nph; i += NT) {
+      const int q = i / nph;
+      s.E3[i] = s.info[4 * q] ? A.Eq[(size_t)s.info[4 * q + 3] * nph + i % nph] : 0.0;
+    }
+    // populations of the final states (el_scattering.cpp:287-300)
+    for (int i = tid; i < kQT * kMaxW * A.nT; i += NT) {
+      const int t = i % A.nT, b2 = (i / A.nT) % kMaxW, q = i / (A.nT * kMaxW);
+      double f = 0.0;
+      if (s.info[4 * q] && b2 < s.info[4 * q + 1]) {
+        const double T = A.temps[t];
+        const int ik2 = s.info[4 * q + 2];
+        const double en2 = A.Ek[(size_t)ik2 * nw + A.lo[ik2] + b2];
+        if (T <= 0.0) {
+          f = en2 <= A.mu ? 1.0 : 0.0;
+        } else {
+          f = 1.0 / (exp((en2 - A.mu) / T) + 1.0);
+          f = fmin(1.0, fmax(0.0, f));
+        }
+      }
+      s.f2[(q * kMaxW + b2) * pairc::kMaxT + t] = f;
+    }
+    for (int i = tid; i < kQT * nph * A.nT; i += NT) {
+      const int t = i % A.nT, nu = (i / A.nT) % nph, q = i / (A.nT * nph);
+      double n = 0.0;
+      const double T = A.temps[t];
+      if (s.info[4 * q] && T > 0.0) {
+        n = 1.0 / (exp(A.Eq[(size_t)s.info[4 * q + 3] * nph + nu] / T) - 1.0);
+        if (n < 0.0) n = 0.0;
+      }
+      s.n3[(q * kMaxPh + nu) * pairc::kMaxT + t] = n;
+    }
+    // adaptive widths of the (b1, b2) pairs (delta_function.cpp:65-88), floored,
+    // as (sigma, 1/sigma) with the zero-velocity flag in the sign bit of sigma
+    for (int x = tid; x < (SM == PHX_SMEAR_ADAPTIVE ? kQT * kMaxW * kMaxW : 0); x += NT) {
+      const int b2 = x % kMaxW, b1 = (x / kMaxW) % kMaxW, q = x / (kMaxW * kMaxW);
+      double2 wv = make_double2(0.0, 0.0);
+      if (s.info[4 * q] && b1 < nb1 && b2 < s.info[4 * q + 1]) {
+        const int ik2 = s.info[4 * q + 2];
+        double v[3];
+        for (int c = 0; c < 3; ++c)
+          v[c] = A.vk[((size_t)ik1 * nw + lo1 + b1) * 3 + c] - A.vk[((size_t)ik2 * nw + A.lo[ik2] + b2) * 3 + c];
+        const ElWidth w = el_width(A, v);
+        double sg = w.sg;
+        if (sg != 0.0 && sg < phxc::adaptiveCutoff) sg = phxc::adaptiveCutoff;
+        wv = make_double2(w.vzero ? -0.0 : sg, sg > 0.0 ? 1.0 / sg : 0.0);
+      }
+      s.wd[x] = wv;
+    }
+    __syncthreads();
+    pair_couplings<G3IN>(cached, nRp, nph, nw, nb1, s, g3in, A.g3ld);
+    pair_symmetrize(E1, nb1, nph, s);
+    // rates (el_scattering.cpp:268-327), one thread per (b1, q, b2, nu) with b1
+    // slowest: when the kQT * kMaxW * nph entries of one b1 fill whole warps
+    // (nph even), a warp reduces its rates and adds them once; otherwise every
+    // thread adds its own
+    const int per_b1 = kQT * kMaxW * nph;
+    const bool warp_sums = per_b1 % 32 == 0;
+    const double ginv = SM == PHX_SMEAR_GAUSSIAN ? 1.0 / A.sigma : 0.0;
+    for (int x = tid; x < nb1 * per_b1; x += NT) {
+      const int nu = x % nph, b2 = (x / nph) % kMaxW, q = (x / (nph * kMaxW)) % kQT, b1 = x / per_b1;
+      double r[pairc::kMaxT];
 #pragma unroll
-    for (int t = 0; t < pairc::kMaxT; ++t) r[t] = 0.0;
-    const double en3 = s.E3[q * nph + nu];
-    if (s.info[4 * q] && b2 < s.info[4 * q + 1] && en3 >= phxc::elPhononCutoff) {
-      const double en1 = E1[b1], en2 = s.E2[q * kMaxW + b2];
-      const double2 wv = SM == PHX_SMEAR_ADAPTIVE ? s.wd[(q * kMaxW + b1) * kMaxW + b2] : make_double2(0.0, 0.0);
-      const double d1 = el_delta_tab<SM>(ginv, en1 - en2 + en3, wv);
-      const double d2 = el_delta_tab<SM>(ginv, en1 - en2 - en3, wv);
-      if (d1 > 0.0 || d2 > 0.0) {
-        const double c = s.cs[((q * kMaxW + b1) * kMaxW + b2) * nph + nu] * A.norm * phxc::pi / en3;
+      for (int t = 0; t < pairc::kMaxT; ++t) r[t] = 0.0;
+      const double en3 = s.E3[q * nph + nu];
+      if (s.info[4 * q] && b2 < s.info[4 * q + 1] && en3 >= phxc::elPhononCutoff) {
+        const double en1 = E1[b1], en2 = s.E2[q * kMaxW + b2];
+        const double2 wv = SM == PHX_SMEAR_ADAPTIVE ? s.wd[(q * kMaxW + b1) * kMaxW + b2] : make_double2(0.0, 0.0);
+        const double d1 = el_delta_tab<SM>(ginv, en1 - en2 + en3, wv);
+        const double d2 = el_delta_tab<SM>(ginv, en1 - en2 - en3, wv);
+        if (d1 > 0.0 || d2 > 0.0) {
+          const double c = s.cs[((q * kMaxW + b1) * kMaxW + b2) * nph + nu] * A.norm * phxc::pi / en3;
 #pragma unroll
-        for (int t = 0; t < pairc::kMaxT; ++t) {
-          if (t < A.nT) {
-            const double fermi2 = s.f2[(q * kMaxW + b2) * pairc::kMaxT + t];
-            const double bose3 = s.n3[(q * kMaxPh + nu) * pairc::kMaxT + t];
-            r[t] = c * ((fermi2 + bose3) * d1 + (1.0 - fermi2 + bose3) * d2);
+          for (int t = 0; t < pairc::kMaxT; ++t) {
+            if (t < A.nT) {
+              const double fermi2 = s.f2[(q * kMaxW + b2) * pairc::kMaxT + t];
+              const double bose3 = s.n3[(q * kMaxPh + nu) * pairc::kMaxT + t];
+              r[t] = c * ((fermi2 + bose3) * d1 + (1.0 - fermi2 + bose3) * d2);
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < pairc::kMaxT; ++t) {
+        if (t < A.nT) {
+          double v = r[t];
+          if (warp_sums) {
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if ((tid & 31) == 0 && v != 0.0) atomicAdd(&s.acc[b1 * pairc::kMaxT + t], v);
+          } else if (v != 0.0) {
+            atomicAdd(&s.acc[b1 * pairc::kMaxT + t], v);
           }
         }
       }
     }
-#pragma unroll
-    for (int t = 0; t < pairc::kMaxT; ++t) {
-      if (t < A.nT) {
-        double v = r[t];
-        if (warp_sums) {
-          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          if ((tid & 31) == 0 && v != 0.0) atomicAdd(&s.acc[b1 * pairc::kMaxT + t], v);
-        } else if (v != 0.0) {
-          atomicAdd(&s.acc[b1 * pairc::kMaxT + t], v);
-        }
-      }
+    __syncthreads();
+    for (int i = tid; i < nb1 * A.nT; i += NT) {
+      const int b1 = i / A.nT, t = i % A.nT;
+      const double v = s.acc[b1 * pairc::kMaxT + t];
+      if (v != 0.0) atomicAdd(&A.out[((size_t)t * A.nk1 + i1) * nw + lo1 + b1], v);
     }
-  }
-  __syncthreads();
-  for (int i = tid; i < nb1 * A.nT; i += NT) {
-    const int b1 = i / A.nT, t = i % A.nT;
-    const double v = s.acc[b1 * pairc::kMaxT + t];
-    if (v != 0.0) atomicAdd(&A.out[((size_t)t * A.nk1 + i1) * nw + lo1 + b1], v);
   }
 }
 
@@ -628,7 +645,8 @@ __global__ void el_k1_bands_kernel(const int* __restrict__ k1s, int nk1, const i
 __global__ void el_batch_gather_kernel(const int* __restrict__ ik, int nb, const int* __restrict__ lo,
                                        const int* __restrict__ hi, const double* __restrict__ kcart,
                                        const double2* __restrict__ Uk, int nw, double* __restrict__ kb,
-                                       double2* __restrict__ ub, int* __restrict__ nbb) {
+                                       double2* __restrict__ ub, int* __restrict__ nbb, int* __restrict__ count) {
+  if (threadIdx.x == 0) *count = 0;   // of the batch's final states
   for (int i = threadIdx.x; i < kB1 * nw * nw; i += blockDim.x) {
     const int j = i / (nw * nw), w = (i / nw) % nw, b = i % nw;
     double2 v = cmk(0.0, 0.0);
@@ -871,7 +889,8 @@ extern "C" int phx_el_linewidths(phx_elph* e, phx_bands* el, phx_bands* ph, cons
                b_out = align256(sizeof(double) * (size_t)nT * std::max(1, nk1) * nw),
                b_kb = align256(sizeof(double) * 3 * kB1), b_ub = align256(sizeof(double2) * kB1 * nw * nw),
                b_nb = align256(sizeof(int) * kB1), b_g1 = align256(sizeof(double2) * kB1 * N);
-  PHX_TRY(elph_reserve(e, 2 * b_lo + 3 * b_k1 + b_out + b_kb + b_ub + b_nb + 2 * b_g1 + b_g3));
+  const size_t b_list = align256(sizeof(int4) * (size_t)kB1 * ph->nq) + 256;
+  PHX_TRY(elph_reserve(e, 2 * b_lo + 3 * b_k1 + b_out + b_kb + b_ub + b_nb + 2 * b_g1 + b_g3 + b_list));
   char* base = static_cast<char*>(e->d_scratch);
   int* dlo = reinterpret_cast<int*>(base);
   int* dhi = reinterpret_cast<int*>(base + b_lo);
@@ -888,6 +907,8 @@ extern "C" int phx_el_linewidths(phx_elph* e, phx_bands* el, phx_bands* ph, cons
   float2* dg3 = split ? reinterpret_cast<float2*>(dBimg + b_B) : nullptr;
   int* dnball = reinterpret_cast<int*>(bb + b_kb + b_ub + b_nb + 2 * b_g1 + b_g3);   // (nk1) active bands
   int* dactik = dnball + b_k1 / sizeof(int);                                        // mesh index of active k1
+  int4* dlist = reinterpret_cast<int4*>(dactik + b_k1 / sizeof(int));               // final states of a batch
+  int* dcount = reinterpret_cast<int*>(reinterpret_cast<char*>(dlist) + b_list - 256);
   cudaStream_t st = ctx->stream;
   cudaEvent_t ev0, ev1;
   PHX_CUDA(ctx, cudaEventCreate(&ev0));
@@ -946,6 +967,8 @@ extern "C" int phx_el_linewidths(phx_elph* e, phx_bands* el, phx_bands* ph, cons
     for (int j = 0; j < 3; ++j) A.qT[i * 3 + j] = el->recip[i * 3 + j] / el->mesh[i];
   A.norm = p->norm;
   A.out = dout;
+  A.list = dlist;
+  A.count = dcount;
   A.g3in = nullptr;
   A.g3ld = 0;
   if (split) {
@@ -957,13 +980,13 @@ extern "C" int phx_el_linewidths(phx_elph* e, phx_bands* el, phx_bands* ph, cons
   const size_t smem = pair_smem_layout(split ? 0 : e->nRp, nph, nw, soff);
   PHX_ARG(ctx, smem <= 227 * 1024, "phx_el_linewidths: too many phonon Bravais vectors");
   constexpr int ad = PHX_SMEAR_ADAPTIVE, ga = PHX_SMEAR_GAUSSIAN;
-  const cudaFuncAttribute fa = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  PHX_CUDA(ctx, cudaFuncSetAttribute(el_pair_kernel<false, ad>, fa, (int)smem));
-  PHX_CUDA(ctx, cudaFuncSetAttribute(el_pair_kernel<false, ga>, fa, (int)smem));
-  PHX_CUDA(ctx, cudaFuncSetAttribute(el_pair_kernel<true, ad>, fa, (int)smem));
-  PHX_CUDA(ctx, cudaFuncSetAttribute(el_pair_kernel<true, ga>, fa, (int)smem));
+  const auto pair_fn = split ? (p->smearing == ad ? el_pair_kernel<true, ad> : el_pair_kernel<true, ga>)
+                             : (p->smearing == ad ? el_pair_kernel<false, ad> : el_pair_kernel<false, ga>);
+  PHX_CUDA(ctx, cudaFuncSetAttribute(pair_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int resident = 1;   // pair blocks per SM
+  PHX_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, pair_fn, kPairThreads, smem));
+  resident = std::max(1, resident);
   const int nq = ph->nq;
-  const int qblocks = (nq + kQT - 1) / kQT;
   const size_t per = N;
   long long pairs = 0;
   for (int b0 = 0; b0 < nact; b0 += kB1) {
@@ -973,7 +996,7 @@ extern "C" int phx_el_linewidths(phx_elph* e, phx_bands* el, phx_bands* ph, cons
     for (int j = 0; j < nb; ++j) nbb[j] = nb1all[rows[j]];
     // k1 coordinates, band counts and U1 of the batch, gathered on the device
     el_batch_gather_kernel<<<1, 256, 0, st>>>(dactik + b0, nb, dlo, dhi, el->d_q,
-                                              reinterpret_cast<const double2*>(el->d_U), nw, dkb, dub, dnb);
+                                              reinterpret_cast<const double2*>(el->d_U), nw, dkb, dub, dnb, dcount);
     ++launches;
     PHX_CUDA(ctx, cudaGetLastError());
     PHX_TRY(elph_cache_batch(e, nb, dkb, dub, dnb, dg1, dcached, split));
@@ -998,15 +1021,10 @@ extern "C" int phx_el_linewidths(phx_elph* e, phx_bands* el, phx_bands* ph, cons
       A.g3in = dg3;
       A.g3ld = g3ld;
     }
-    const dim3 grid(qblocks, nb);
-    const bool adaptive = A.smearing == PHX_SMEAR_ADAPTIVE;
-    if (A.g3in) {
-      if (adaptive) el_pair_kernel<true, ad><<<grid, kPairThreads, smem, st>>>(A);
-      else el_pair_kernel<true, ga><<<grid, kPairThreads, smem, st>>>(A);
-    } else {
-      if (adaptive) el_pair_kernel<false, ad><<<grid, kPairThreads, smem, st>>>(A);
-      else el_pair_kernel<false, ga><<<grid, kPairThreads, smem, st>>>(A);
-    }
+    el_list_kernel<<<dim3((nq + 255) / 256, nb), 256, 0, st>>>(A);
+    const int grid = (int)std::min<long long>((long long)nq * nb, (long long)resident * ctx->num_sms);
+    pair_fn<<<grid, kPairThreads, smem, st>>>(A);
+    ++launches;
     ++launches;
     pairs += (long long)nq * nb;
     PHX_CUDA(ctx, cudaGetLastError());
