@@ -37,23 +37,41 @@ int phx_el_split_g1(phx_ctx* ctx, const uint8_t* gimg, int nRe, long long N, con
 namespace {
 
 constexpr int kB1 = 16;       // k1 points per pass over the coupling tensor
-constexpr int kQT = 1;        // final states per pair block
 constexpr int kMaxW = 8;      // Wannier orbitals
 constexpr int kMaxPh = 12;    // phonon branches
-constexpr int kPairThreads = 64;
+constexpr int kPairThreads = 64;    // of a block that takes one final state at a time
+constexpr int kTileQ = 8;           // final states per FP64 tile (one row each of m8n8k4)
+constexpr int kTileThreads = 192;
 
-// g1[b][e] = sum_Re ph[b][Re] g[Re][e] for the kB1 k1 of the batch (e over nRp*nph*nw*nw)
-__global__ void __launch_bounds__(256) elph_g1_kernel(const float2* __restrict__ g, int nRe, size_t N,
-                                                      const double* __restrict__ Re,
-                                                      const double* __restrict__ degE,
-                                                      const double* __restrict__ k1s, int nb,
-                                                      double2* __restrict__ g1) {
+// D += A B on the FP64 tensor pipe: m8n8k4, lane l holds A(l/4, l%4), B(l%4, l/4)
+// and D(l/4, 2(l%4) + {0,1})
+__device__ __forceinline__ void dmma(double* d, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
+// g1[b][e] = sum_Re ph[b][Re] g[Re][e] for the nb k1 of the batch (e over
+// nRp*nph*nw*nw): a product of the 8 MT phases of each Re with g, read once per
+// batch.  One warp takes 8 kG1Cols columns at a time and all k1; the phases lie in
+// shared memory in the order in which the lanes read them (four Re of a k1 side by
+// side), so that one conflict-free 16-byte load gives a lane both parts of its A.
+// Bound by the FP64 tensor pipe: 16 k1 x 343 Re x 131712 columns take 237 us (24
+// TFLOP/s; 604 us with one thread per column and DFMA, which waited for its loads).
+constexpr int kG1Cols = 4;
+template <int MT>
+__global__ void __launch_bounds__(256, 2) elph_g1_kernel(const float2* __restrict__ g, int nRe, size_t N,
+                                                         const double* __restrict__ Re,
+                                                         const double* __restrict__ degE,
+                                                         const double* __restrict__ k1s, int nb,
+                                                         double2* __restrict__ g1) {
   extern __shared__ __align__(16) char sraw[];
-  double2* ph = reinterpret_cast<double2*>(sraw);  // [kB1][nRe]
-  for (int i = threadIdx.x; i < kB1 * nRe; i += blockDim.x) {
-    const int b = i / nRe, r = i % nRe;
+  double2* ph = reinterpret_cast<double2*>(sraw);  // [Re / 4][8 MT][4]
+  const int nks = (nRe + 3) / 4;
+  for (int i = threadIdx.x; i < nks * 32 * MT; i += blockDim.x) {
+    const int b = (i >> 2) % (8 * MT), r = i / (32 * MT) * 4 + (i & 3);
     double2 v = cmk(0.0, 0.0);
-    if (b < nb) {
+    if (b < nb && r < nRe) {
       const double* k = k1s + 3 * b;
       double sn, cs;
       sincos(k[0] * Re[3 * r] + k[1] * Re[3 * r + 1] + k[2] * Re[3 * r + 2], &sn, &cs);
@@ -62,19 +80,65 @@ __global__ void __launch_bounds__(256) elph_g1_kernel(const float2* __restrict__
     ph[i] = v;
   }
   __syncthreads();
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < N; e += (size_t)gridDim.x * blockDim.x) {
-    double2 acc[kB1];
+  const int lane = threadIdx.x & 31, lr = lane & 3, lc = lane >> 2;
+  const size_t tiles = (N + 8 * kG1Cols - 1) / (8 * kG1Cols);
+  for (size_t t = blockIdx.x * (size_t)(blockDim.x / 32) + threadIdx.x / 32; t < tiles;
+       t += (size_t)gridDim.x * (blockDim.x / 32)) {
+    const size_t e0 = t * 8 * kG1Cols;
+    double re[MT][kG1Cols][2], im[MT][kG1Cols][2];
 #pragma unroll
-    for (int b = 0; b < kB1; ++b) acc[b] = cmk(0.0, 0.0);
-    for (int r = 0; r < nRe; ++r) {
-      const float2 x = __ldg(g + (size_t)r * N + e);
-      const double2 xd = cmk((double)x.x, (double)x.y);
+    for (int m = 0; m < MT; ++m)
 #pragma unroll
-      for (int b = 0; b < kB1; ++b) acc[b] = cadd(acc[b], cmul(xd, ph[b * nRe + r]));
+      for (int j = 0; j < kG1Cols; ++j) re[m][j][0] = re[m][j][1] = im[m][j][0] = im[m][j][1] = 0.0;
+    float2 nx[kG1Cols];
+    auto load = [&](int ks) {
+      const int r = 4 * ks + lr;
+#pragma unroll
+      for (int j = 0; j < kG1Cols; ++j) {
+        const size_t e = e0 + 8 * j + lc;
+        nx[j] = r < nRe && e < N ? __ldg(g + (size_t)r * N + e) : make_float2(0.f, 0.f);
+      }
+    };
+    load(0);
+#pragma unroll 2
+    for (int ks = 0; ks < nks; ++ks) {
+      double xr[kG1Cols], xi[kG1Cols];
+#pragma unroll
+      for (int j = 0; j < kG1Cols; ++j) {
+        xr[j] = (double)nx[j].x;
+        xi[j] = (double)nx[j].y;
+      }
+      if (ks + 1 < nks) load(ks + 1);
+      double2 f[MT];
+#pragma unroll
+      for (int m = 0; m < MT; ++m) f[m] = ph[ks * 32 * MT + m * 32 + lane];
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int j = 0; j < kG1Cols; ++j) {
+          dmma(re[m][j], f[m].x, xr[j]);
+          dmma(im[m][j], f[m].x, xi[j]);
+        }
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int j = 0; j < kG1Cols; ++j) {
+          dmma(re[m][j], -f[m].y, xi[j]);
+          dmma(im[m][j], f[m].y, xr[j]);
+        }
     }
 #pragma unroll
-    for (int b = 0; b < kB1; ++b)
-      if (b < nb) g1[(size_t)b * N + e] = acc[b];
+    for (int m = 0; m < MT; ++m) {
+      const int b = 8 * m + lc;
+      if (b >= nb) continue;
+#pragma unroll
+      for (int j = 0; j < kG1Cols; ++j)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const size_t e = e0 + 8 * j + 2 * lr + c;
+          if (e < N) g1[(size_t)b * N + e] = cmk(re[m][j][c], im[m][j][c]);
+        }
+    }
   }
 }
 
@@ -100,53 +164,62 @@ __global__ void elph_rot_kernel(const double2* __restrict__ g1, int nRpPh, int n
 }
 
 // ---------------------------------------------------------------------------
-// pair block: couplings of kQT final states of one k1
+// pair block: couplings of QT final states of one k1.  w1 is the number of
+// initial bands that the buffers hold: kMaxW for QT = 1, the batch's largest for
+// a tile of several states.
 // ---------------------------------------------------------------------------
 struct PairSmem {
-  double2* ph;    // [kQT][nRp]
-  double2* g3;    // [kQT][nph][kMaxW(b1)][nw]
+  int w1;
+  double2* ph;    // [QT][nRp]; of a tile [nRp / 4][QT][4], in the space of g4
+  double2* g3;    // [QT][nph][w1][nw]
   double2* g4;    // same
-  double2* U2;    // [kQT][nw][kMaxW(b2)]
-  double2* ev3;   // [kQT][nph][nph]
-  double* cs;     // [kQT][kMaxW][kMaxW][nph] |g|^2
-  double* E2;     // [kQT][kMaxW]
-  double* E3;     // [kQT][nph]
+  double2* U2;    // [QT][nw][kMaxW(b2)]
+  double2* ev3;   // [QT][nph][nph]
+  double* cs;     // [QT][w1][kMaxW][nph] |g|^2
+  double* E2;     // [QT][kMaxW]
+  double* E3;     // [QT][nph]
   double* acc;    // [kMaxW][kMaxT] block sums of the rates
-  int* info;      // [kQT][4]: valid, nb2, k2 index, q index
-  double* f2;     // [kQT][kMaxW][kMaxT] Fermi occupation of the final electron states
-  double* n3;     // [kQT][kMaxPh][kMaxT] Bose occupation of the phonons
-  double2* wd;    // [kQT][kMaxW(b1)][kMaxW(b2)] adaptive width: (sigma, |v1 - v2| == 0)
+  int* info;      // [QT][4]: valid, nb2, k2 index, q index
+  double* f2;     // [QT][kMaxW][kMaxT] Fermi occupation of the final electron states
+  double* n3;     // [QT][kMaxPh][kMaxT] Bose occupation of the phonons
+  double2* wd;    // [QT][w1][kMaxW(b2)] adaptive width: (sigma, |v1 - v2| == 0)
 };
 
-__host__ __device__ inline size_t pair_smem_layout(int nRp, int nph, int nw, size_t* off) {
+template <int QT>
+__host__ __device__ inline size_t pair_smem_layout(int nRp, int nph, int nw, int w1, size_t* off) {
   size_t o = 0;
   auto take = [&](size_t bytes) {
     const size_t r = o;
     o += (bytes + 15) & ~size_t(15);
     return r;
   };
-  off[0] = take(sizeof(double2) * kQT * nRp);
+  // the phases of a tile are dead when g4 is written: they share its space
+  const size_t phb = sizeof(double2) * QT * (QT > 1 ? (nRp + 3) / 4 * 4 : nRp);
+  off[0] = QT > 1 ? 0 : take(phb);
   // |g|^2 (cs) is written after g4 is complete, when g3 is dead: it shares g3's space
-  const size_t g3b = sizeof(double2) * kQT * nph * kMaxW * nw, csb = sizeof(double) * kQT * kMaxW * kMaxW * nph;
+  const size_t g3b = sizeof(double2) * QT * nph * w1 * nw, csb = sizeof(double) * QT * w1 * kMaxW * nph;
   off[1] = take(g3b > csb ? g3b : csb);
-  off[2] = take(sizeof(double2) * kQT * nph * kMaxW * nw);
-  off[3] = take(sizeof(double2) * kQT * nw * kMaxW);
-  off[4] = take(sizeof(double2) * kQT * nph * nph);
+  off[2] = take(QT > 1 && phb > g3b ? phb : g3b);
+  if (QT > 1) off[0] = off[2];
+  off[3] = take(sizeof(double2) * QT * nw * kMaxW);
+  off[4] = take(sizeof(double2) * QT * nph * nph);
   off[5] = off[1];
-  off[6] = take(sizeof(double) * kQT * kMaxW);
-  off[7] = take(sizeof(double) * kQT * nph);
+  off[6] = take(sizeof(double) * QT * kMaxW);
+  off[7] = take(sizeof(double) * QT * nph);
   off[8] = take(sizeof(double) * kMaxW * pairc::kMaxT);
-  off[9] = take(sizeof(int) * kQT * 4);
-  off[10] = take(sizeof(double) * kQT * kMaxW * pairc::kMaxT);
-  off[11] = take(sizeof(double) * kQT * kMaxPh * pairc::kMaxT);
-  off[12] = take(sizeof(double2) * kQT * kMaxW * kMaxW);
+  off[9] = take(sizeof(int) * QT * 4);
+  off[10] = take(sizeof(double) * QT * kMaxW * pairc::kMaxT);
+  off[11] = take(sizeof(double) * QT * kMaxPh * pairc::kMaxT);
+  off[12] = take(sizeof(double2) * QT * w1 * kMaxW);
   return o;
 }
 
-__device__ inline PairSmem pair_carve(char* base, int nRp, int nph, int nw) {
+template <int QT>
+__device__ inline PairSmem pair_carve(char* base, int nRp, int nph, int nw, int w1) {
   size_t off[13];
-  pair_smem_layout(nRp, nph, nw, off);
+  pair_smem_layout<QT>(nRp, nph, nw, w1, off);
   PairSmem s;
+  s.w1 = w1;
   s.ph = reinterpret_cast<double2*>(base + off[0]);
   s.g3 = reinterpret_cast<double2*>(base + off[1]);
   s.g4 = reinterpret_cast<double2*>(base + off[2]);
@@ -163,93 +236,137 @@ __device__ inline PairSmem pair_carve(char* base, int nRp, int nph, int nw) {
   return s;
 }
 
-// |g|^2 of the kQT final states whose phases, U2 (nb2 columns) and ev3 are staged;
+// g3[q][nu][b1][w2] = sum_Rp ph[q][Rp] cached[Rp][nu][b1][w2] of a tile on the FP64
+// tensor pipe.  A warp takes 8 columns x = (nu, b1, w2) at a time, all Rp and all
+// states: cached is read once per tile, as two B fragments (its real and imaginary
+// parts) per 16-byte load.
+__device__ void pair_g3_tile(const double2* __restrict__ cached, int nRp, int nph, int nw, int nb1,
+                             const PairSmem& s) {
+  const int lane = threadIdx.x & 31, lr = lane & 3, lc = lane >> 2;
+  const int nx = nph * nb1 * nw, nks = (nRp + 3) / 4;
+  const size_t rs = (size_t)nph * nw * nw;
+  for (int x0 = (threadIdx.x / 32) * 8; x0 < nx; x0 += blockDim.x / 32 * 8) {
+    const int x = x0 + lc;
+    const double2* src = cached + ((size_t)(x / (nw * nb1)) * nw + (x / nw) % nb1) * nw + x % nw;
+    double re[2][2] = {}, im[2][2] = {};   // two chains each
+    auto load = [&](int ks) {
+      const int r = 4 * ks + lr;
+      return x < nx && r < nRp ? __ldg(src + r * rs) : cmk(0.0, 0.0);
+    };
+    constexpr int D = 4;   // loads in flight
+    double2 c[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) c[d] = load(d);
+    for (int k0 = 0; k0 < nks; k0 += D) {
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        const double2 v = c[d];
+        c[d] = load(k0 + d + D);
+        if (k0 + d < nks) {
+          const double2 f = s.ph[(k0 + d) * 4 * kTileQ + lane];
+          dmma(re[0], f.x, v.x);
+          dmma(im[0], f.x, v.y);
+          dmma(re[1], -f.y, v.y);
+          dmma(im[1], f.y, v.x);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int xo = x0 + 2 * lr + i;   // column of this lane's sums, state lc
+      if (xo < nx) {
+        const int w2 = xo % nw, b1 = (xo / nw) % nb1, nu = xo / (nw * nb1);
+        s.g3[((lc * nph + nu) * s.w1 + b1) * nw + w2] = cmk(re[0][i] + re[1][i], im[0][i] + im[1][i]);
+      }
+    }
+  }
+}
+
+// |g|^2 of the QT final states whose phases, U2 (nb2 columns) and ev3 are staged;
 // cached is (nRp, nph, nw(b1), nw) of one k1 with nb1 active bands.  G3IN:
 // g3 comes from the tensor-core GEMM (split path) instead of the FP64 Rp
 // transform; each path is its own instantiation, so that each kernel holds
 // only its code (the pair kernel is bound by instruction fetch otherwise).
-template <bool G3IN>
+template <int QT, bool G3IN>
 __device__ void pair_couplings(const double2* __restrict__ cached, int nRp, int nph, int nw, int nb1,
                                const PairSmem& s, const float2* __restrict__ g3in = nullptr, int g3ld = 0) {
-  const int tid = threadIdx.x, NT = blockDim.x;
+  const int tid = threadIdx.x, NT = blockDim.x, W1 = QT == 1 ? kMaxW : s.w1;
   const int nx = nph * nb1 * nw;
   if constexpr (G3IN) {
     // g3 from the tensor-core GEMM, stored g3in[x * g3ld + q] (q = phonon mesh index)
-    for (int i = tid; i < kQT * nx; i += NT) {
-      const int q = i % kQT, x = i / kQT;
+    for (int i = tid; i < QT * nx; i += NT) {
+      const int q = i % QT, x = i / QT;
       const int w2 = x % nw, b1 = (x / nw) % nb1, nu = x / (nw * nb1);
       double2 v = cmk(0.0, 0.0);
       if (s.info[4 * q]) {
         const float2 f = g3in[(size_t)x * g3ld + s.info[4 * q + 3]];
         v = cmk((double)f.x, (double)f.y);
       }
-      s.g3[((q * nph + nu) * kMaxW + b1) * nw + w2] = v;
+      s.g3[((q * nph + nu) * W1 + b1) * nw + w2] = v;
     }
-  }
-  // g3[q][nu][b1][w2] = sum_Rp ph[q][Rp] cached[Rp][nu][b1][w2]
-  for (int x = tid; x < (G3IN ? 0 : nx); x += NT) {
-    const int w2 = x % nw, b1 = (x / nw) % nb1, nu = x / (nw * nb1);
-    const size_t cx = ((size_t)nu * nw + b1) * nw + w2;
-    double2 acc[kQT];
-#pragma unroll
-    for (int q = 0; q < kQT; ++q) acc[q] = cmk(0.0, 0.0);
-    for (int r = 0; r < nRp; ++r) {
-      const double2 c = cached[(size_t)r * nph * nw * nw + cx];
-#pragma unroll
-      for (int q = 0; q < kQT; ++q) acc[q] = cadd(acc[q], cmul(s.ph[q * nRp + r], c));
+  } else if constexpr (QT == kTileQ) {
+    pair_g3_tile(cached, nRp, nph, nw, nb1, s);
+  } else {
+    // g3[nu][b1][w2] = sum_Rp ph[Rp] cached[Rp][nu][b1][w2] of one state
+    static_assert(QT == 1, "a state at a time");
+    for (int x = tid; x < nx; x += NT) {
+      const int w2 = x % nw, b1 = (x / nw) % nb1, nu = x / (nw * nb1);
+      const size_t cx = ((size_t)nu * nw + b1) * nw + w2;
+      double2 acc = cmk(0.0, 0.0);
+      for (int r = 0; r < nRp; ++r) acc = cadd(acc, cmul(s.ph[r], cached[(size_t)r * nph * nw * nw + cx]));
+      s.g3[(nu * W1 + b1) * nw + w2] = acc;
     }
-#pragma unroll
-    for (int q = 0; q < kQT; ++q) s.g3[((q * nph + nu) * kMaxW + b1) * nw + w2] = acc[q];
   }
   __syncthreads();
   // g4[q][nu2][b1][w2] = sum_nu g3[q][nu][b1][w2] ev3[q][nu][nu2]
-  for (int x = tid; x < kQT * nx; x += NT) {
+  for (int x = tid; x < QT * nx; x += NT) {
     const int q = x / nx, r = x % nx;
     const int w2 = r % nw, b1 = (r / nw) % nb1, nu2 = r / (nw * nb1);
     double2 acc = cmk(0.0, 0.0);
     for (int nu = 0; nu < nph; ++nu)
-      acc = cadd(acc, cmul(s.g3[((q * nph + nu) * kMaxW + b1) * nw + w2], s.ev3[(q * nph + nu) * nph + nu2]));
-    s.g4[((q * nph + nu2) * kMaxW + b1) * nw + w2] = acc;
+      acc = cadd(acc, cmul(s.g3[((q * nph + nu) * W1 + b1) * nw + w2], s.ev3[(q * nph + nu) * nph + nu2]));
+    s.g4[((q * nph + nu2) * W1 + b1) * nw + w2] = acc;
   }
   __syncthreads();
   // |g[q][b1][b2][nu]|^2 with g = sum_w2 conj(U2[q][w2][b2]) g4[q][nu][b1][w2]
-  for (int x = tid; x < kQT * nb1 * kMaxW * nph; x += NT) {
+  for (int x = tid; x < QT * nb1 * kMaxW * nph; x += NT) {
     const int nu = x % nph, b2 = (x / nph) % kMaxW, b1 = (x / (nph * kMaxW)) % nb1, q = x / (nph * kMaxW * nb1);
     double v = 0.0;
     if (b2 < s.info[4 * q + 1]) {
       double2 acc = cmk(0.0, 0.0);
       for (int w2 = 0; w2 < nw; ++w2)
-        acc = cadd(acc, cmul(cconj(s.U2[(q * nw + w2) * kMaxW + b2]), s.g4[((q * nph + nu) * kMaxW + b1) * nw + w2]));
+        acc = cadd(acc, cmul(cconj(s.U2[(q * nw + w2) * kMaxW + b2]), s.g4[((q * nph + nu) * W1 + b1) * nw + w2]));
       v = acc.x * acc.x + acc.y * acc.y;
     }
-    s.cs[((q * kMaxW + b1) * kMaxW + b2) * nph + nu] = v;
+    s.cs[((q * W1 + b1) * kMaxW + b2) * nph + nu] = v;
   }
   __syncthreads();
 }
 
-// symmetrizeCoupling (scattering.cpp:1209-1318) of the kQT couplings:
+// symmetrizeCoupling (scattering.cpp:1209-1318) of the QT couplings:
 // forward-scan degenerate blocks of b1 (E1), then b2 (E2[q]), then nu (E3[q])
+template <int QT>
 __device__ void pair_symmetrize(const double* E1, int nb1, int nph, const PairSmem& s) {
-  const int tid = threadIdx.x, NT = blockDim.x;
+  const int tid = threadIdx.x, NT = blockDim.x, W1 = QT == 1 ? kMaxW : s.w1;
   auto C = [&](int q, int b1, int b2, int nu) -> double& {
-    return s.cs[((q * kMaxW + b1) * kMaxW + b2) * nph + nu];
+    return s.cs[((q * W1 + b1) * kMaxW + b2) * nph + nu];
   };
   // A forward-scan block of two or more states exists exactly when two
   // neighbouring energies are within the threshold; a pass without one is
   // the identity and is skipped (block-wide votes, which are also barriers).
   const bool n1 = tid + 1 < nb1 && fabs(E1[tid] - E1[tid + 1]) < 1.0e-6;
   bool n2 = false, n3 = false;
-  if (tid < kQT * kMaxW) {
+  if (tid < QT * kMaxW) {
     const int q = tid / kMaxW, b = tid % kMaxW;
     n2 = s.info[4 * q] && b + 1 < s.info[4 * q + 1] && fabs(s.E2[q * kMaxW + b] - s.E2[q * kMaxW + b + 1]) < 1.0e-6;
   }
-  if (tid < kQT * nph) {
+  if (tid < QT * nph) {
     const int q = tid / nph, nu = tid % nph;
     n3 = s.info[4 * q] && nu + 1 < nph && fabs(s.E3[q * nph + nu] - s.E3[q * nph + nu + 1]) < 1.0e-6;
   }
   if (!__syncthreads_or(n1 || n2 || n3)) return;
   if (__syncthreads_or(n1)) {
-    for (int x = tid; x < kQT * kMaxW * nph; x += NT) {
+    for (int x = tid; x < QT * kMaxW * nph; x += NT) {
       const int q = x / (kMaxW * nph), b2 = (x / nph) % kMaxW, nu = x % nph;
       if (!s.info[4 * q] || b2 >= s.info[4 * q + 1]) continue;
       for (int ib = 0; ib < nb1;) {
@@ -268,7 +385,7 @@ __device__ void pair_symmetrize(const double* E1, int nb1, int nph, const PairSm
     }
   }
   if (__syncthreads_or(n2)) {
-    for (int x = tid; x < kQT * kMaxW * nph; x += NT) {
+    for (int x = tid; x < QT * kMaxW * nph; x += NT) {
       const int q = x / (kMaxW * nph), b1 = (x / nph) % kMaxW, nu = x % nph;
       const int nb2 = s.info[4 * q + 1];
       if (!s.info[4 * q] || b1 >= nb1) continue;
@@ -289,7 +406,7 @@ __device__ void pair_symmetrize(const double* E1, int nb1, int nph, const PairSm
     }
   }
   if (__syncthreads_or(n3)) {
-    for (int x = tid; x < kQT * kMaxW * kMaxW; x += NT) {
+    for (int x = tid; x < QT * kMaxW * kMaxW; x += NT) {
       const int q = x / (kMaxW * kMaxW), b1 = (x / kMaxW) % kMaxW, b2 = x % kMaxW;
       if (!s.info[4 * q] || b1 >= nb1 || b2 >= s.info[4 * q + 1]) continue;
       const double* E3 = s.E3 + q * nph;
@@ -339,9 +456,11 @@ struct ElArgs {
   double* out;             // (nT, nk1, nw)
   const float2* g3in;      // precomputed g3 of this k1, g3in[x * g3ld + q], or null
   int g3ld;
-  // the batch's final states with active bands: (row of the batch, q, k2, nb2), *count of them
+  // the final states with active bands of row j of the batch: (q, k2, nb2) at
+  // list[j * nq ..], count[j] of them; w1: the largest nb1 of the batch's k1
   int4* list;
   int* count;
+  int nb, w1;
 };
 
 // adaptive width of a (k1 b1, k2 b2) pair from v = v1 - v2 (delta_function.cpp:65-88);
@@ -386,7 +505,7 @@ __device__ __forceinline__ double el_delta_tab(double ginv, double e, double2 w)
 // Final states k2 = k1 + q of the batch's k1 (blockIdx.y) that have active
 // bands, in no fixed order.  With a window around the Fermi level most have none
 // (84% of them with +-0.3 eV on 8 bands of 2 eV hoppings), and a block of the
-// pair kernel for each of those cost more than the pairs: 255 -> 61 us per 16 k1.
+// pair kernel for each of those cost as much as the pairs: 255 -> 128 us per 16 k1.
 __global__ void __launch_bounds__(256) el_list_kernel(ElArgs A) {
   const int iq = blockIdx.x * blockDim.x + threadIdx.x, jb = blockIdx.y;
   const int ik1 = A.ik1s[jb];
@@ -403,44 +522,65 @@ __global__ void __launch_bounds__(256) el_list_kernel(ElArgs A) {
   if (!have) return;
   const int lane = threadIdx.x & 31;
   int first = 0;
-  if (lane == 0) first = atomicAdd(A.count, __popc(have));
+  if (lane == 0) first = atomicAdd(A.count + jb, __popc(have));
   first = __shfl_sync(0xffffffffu, first, 0);
-  if (nb2 > 0) A.list[first + __popc(have & ((1u << lane) - 1u))] = make_int4(jb, iq, ik2, nb2);
+  if (nb2 > 0)
+    A.list[(size_t)jb * (A.qmesh[0] * A.qmesh[1] * A.qmesh[2]) + first + __popc(have & ((1u << lane) - 1u))] =
+        make_int4(iq, ik2, nb2, 0);
 }
 
 // G3IN: g3 from the tensor-core GEMM (split path); SM: the smearing.  Each
 // combination is its own instantiation, which keeps the kernel's code small.
-template <bool G3IN, int SM>
-__global__ void __launch_bounds__(kPairThreads) el_pair_kernel(ElArgs A) {
+// QT: final states of one k1 per pass of a block.  Tiles of 8 give the FP64 Rp
+// transform the rows of m8n8k4 (pair_g3_tile) and share the barriers of the short
+// stages: per 16 k1 of a 20^3 q mesh 962 -> 260 us in FP64, where one state at a time
+// read all of cached (263 KB with 343 Rp) from L2 for every state, and 128 -> 92 us in
+// the split path.  Bound by the latency of the stages between the barriers, so the
+// registers are held to 6 blocks per SM in the split path (4 blocks: 101 us), and
+// to 3 in FP64, whose phases fill shared memory.
+template <int QT, bool G3IN, int SM>
+__global__ void __launch_bounds__(QT == 1 ? kPairThreads : kTileThreads, QT == 1 ? 1 : G3IN ? 6 : 3)
+    el_pair_kernel(ElArgs A) {
   extern __shared__ __align__(16) char sraw[];
   const int nw = A.nw, nph = A.nph, nRp = A.nRp;
   // no phase buffer when g3 comes from the tensor-core GEMM
-  const PairSmem s = pair_carve(sraw, G3IN ? 0 : nRp, nph, nw);
-  const int tid = threadIdx.x, NT = blockDim.x;
-  static_assert(kQT == 1, "one final state of the list per block and pass");
-  const int count = *A.count;
-  for (int item = blockIdx.x; item < count; item += gridDim.x) {
-    const int4 fs = A.list[item];
-    const int jb = fs.x;
+  const PairSmem s = pair_carve<QT>(sraw, G3IN ? 0 : nRp, nph, nw, QT == 1 ? kMaxW : A.w1);
+  const int tid = threadIdx.x, NT = blockDim.x, W1 = QT == 1 ? kMaxW : A.w1;
+  // lane j: tiles of the rows up to and with j of the batch
+  static_assert(kB1 <= 31, "a lane for each k1 of a batch");
+  const int lane = tid & 31, own = lane < A.nb ? (A.count[lane] + QT - 1) / QT : 0;
+  int incl = own;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  for (int item = blockIdx.x; item < total; item += gridDim.x) {
+    const int jb = __popc(__ballot_sync(0xffffffffu, incl <= item));
+    const int first = (item - __shfl_sync(0xffffffffu, incl - own, jb)) * QT;
+    const int left = A.count[jb] - first;   // states of the row from here on
+    const int4* states = A.list + (size_t)jb * (A.qmesh[0] * A.qmesh[1] * A.qmesh[2]) + first;
     const int ik1 = A.ik1s[jb], i1 = A.i1s[jb], lo1 = A.lo[ik1], nb1 = A.hi[ik1] - lo1;
     const double2* cached = A.cached + (size_t)jb * A.cper;
     const float2* g3in = G3IN ? A.g3in + A.g3offs[jb] : nullptr;
     const double* E1 = A.Ek + (size_t)ik1 * nw + lo1;
     __syncthreads();   // the previous final state's sums have been read
     for (int i = tid; i < kMaxW * pairc::kMaxT; i += NT) s.acc[i] = 0.0;
-    if (tid == 0) {
-      s.info[0] = 1;
-      s.info[1] = fs.w;
-      s.info[2] = fs.z;
-      s.info[3] = fs.y;
+    if (tid < QT) {
+      const int4 fs = tid < left ? states[tid] : make_int4(0, 0, 0, 0);
+      s.info[4 * tid] = tid < left;
+      s.info[4 * tid + 1] = fs.z;
+      s.info[4 * tid + 2] = fs.y;
+      s.info[4 * tid + 3] = fs.x;
     }
     __syncthreads();
     // phases e^{+i q3.Rp}/deg with q3 = k2 - k1 (helper_el_scattering.cpp:233-234),
     // not needed when g3 comes from the tensor-core GEMM
-    for (int i = tid; i < (G3IN ? 0 : kQT * nRp); i += NT) {
-      const int q = i / nRp, r = i % nRp;
+    const int rows = QT == 1 ? nRp : (nRp + 3) / 4 * 4;
+    for (int i = tid; i < (G3IN ? 0 : QT * rows); i += NT) {
+      const int q = QT == 1 ? 0 : (i >> 2) % QT, r = QT == 1 ? i : i / (4 * QT) * 4 + (i & 3);
       double2 v = cmk(0.0, 0.0);
-      if (s.info[4 * q]) {
+      if (r < nRp && s.info[4 * q]) {
         const int ik2 = s.info[4 * q + 2];
         double q3[3];
         for (int c = 0; c < 3; ++c) q3[c] = A.kcart[3 * ik2 + c] - A.kcart[3 * ik1 + c];
@@ -450,7 +590,7 @@ __global__ void __launch_bounds__(kPairThreads) el_pair_kernel(ElArgs A) {
       }
       s.ph[i] = v;
     }
-    for (int i = tid; i < kQT * nw * kMaxW; i += NT) {
+    for (int i = tid; i < QT * nw * kMaxW; i += NT) {
       const int q = i / (nw * kMaxW), w = (i / kMaxW) % nw, b2 = i % kMaxW;
       double2 v = cmk(0.0, 0.0);
       if (s.info[4 * q] && b2 < s.info[4 * q + 1]) {
@@ -459,20 +599,20 @@ __global__ void __launch_bounds__(kPairThreads) el_pair_kernel(ElArgs A) {
       }
       s.U2[i] = v;
     }
-    for (int i = tid; i < kQT * nph * nph; i += NT) {
+    for (int i = tid; i < QT * nph * nph; i += NT) {
       const int q = i / (nph * nph);
       s.ev3[i] = s.info[4 * q] ? A.evq[(size_t)s.info[4 * q + 3] * nph * nph + i % (nph * nph)] : cmk(0.0, 0.0);
     }
-    for (int i = tid; i < kQT * kMaxW; i += NT) {
+    for (int i = tid; i < QT * kMaxW; i += NT) {
       const int q = i / kMaxW, b2 = i % kMaxW;
       s.E2[i] = (s.info[4 * q] && b2 < s.info[4 * q + 1]) ? A.Ek[(size_t)s.info[4 * q + 2] * nw + A.lo[s.info[4 * q + 2]] + b2] : 0.0;
     }
-    for (int i = tid; i < kQT * nph; i += NT) {
+    for (int i = tid; i < QT * nph; i += NT) {
       const int q = i / nph;
       s.E3[i] = s.info[4 * q] ? A.Eq[(size_t)s.info[4 * q + 3] * nph + i % nph] : 0.0;
     }
     // populations of the final states (el_scattering.cpp:287-300)
-    for (int i = tid; i < kQT * kMaxW * A.nT; i += NT) {
+    for (int i = tid; i < QT * kMaxW * A.nT; i += NT) {
       const int t = i % A.nT, b2 = (i / A.nT) % kMaxW, q = i / (A.nT * kMaxW);
       double f = 0.0;
       if (s.info[4 * q] && b2 < s.info[4 * q + 1]) {
@@ -488,7 +628,7 @@ __global__ void __launch_bounds__(kPairThreads) el_pair_kernel(ElArgs A) {
       }
       s.f2[(q * kMaxW + b2) * pairc::kMaxT + t] = f;
     }
-    for (int i = tid; i < kQT * nph * A.nT; i += NT) {
+    for (int i = tid; i < QT * nph * A.nT; i += NT) {
       const int t = i % A.nT, nu = (i / A.nT) % nph, q = i / (A.nT * nph);
       double n = 0.0;
       const double T = A.temps[t];
@@ -500,8 +640,8 @@ __global__ void __launch_bounds__(kPairThreads) el_pair_kernel(ElArgs A) {
     }
     // adaptive widths of the (b1, b2) pairs (delta_function.cpp:65-88), floored,
     // as (sigma, 1/sigma) with the zero-velocity flag in the sign bit of sigma
-    for (int x = tid; x < (SM == PHX_SMEAR_ADAPTIVE ? kQT * kMaxW * kMaxW : 0); x += NT) {
-      const int b2 = x % kMaxW, b1 = (x / kMaxW) % kMaxW, q = x / (kMaxW * kMaxW);
+    for (int x = tid; x < (SM == PHX_SMEAR_ADAPTIVE ? QT * W1 * kMaxW : 0); x += NT) {
+      const int b2 = x % kMaxW, b1 = (x / kMaxW) % W1, q = x / (kMaxW * W1);
       double2 wv = make_double2(0.0, 0.0);
       if (s.info[4 * q] && b1 < nb1 && b2 < s.info[4 * q + 1]) {
         const int ik2 = s.info[4 * q + 2];
@@ -516,28 +656,28 @@ __global__ void __launch_bounds__(kPairThreads) el_pair_kernel(ElArgs A) {
       s.wd[x] = wv;
     }
     __syncthreads();
-    pair_couplings<G3IN>(cached, nRp, nph, nw, nb1, s, g3in, A.g3ld);
-    pair_symmetrize(E1, nb1, nph, s);
+    pair_couplings<QT, G3IN>(cached, nRp, nph, nw, nb1, s, g3in, A.g3ld);
+    pair_symmetrize<QT>(E1, nb1, nph, s);
     // rates (el_scattering.cpp:268-327), one thread per (b1, q, b2, nu) with b1
-    // slowest: when the kQT * kMaxW * nph entries of one b1 fill whole warps
+    // slowest: when the QT * kMaxW * nph entries of one b1 fill whole warps
     // (nph even), a warp reduces its rates and adds them once; otherwise every
     // thread adds its own
-    const int per_b1 = kQT * kMaxW * nph;
+    const int per_b1 = QT * kMaxW * nph;
     const bool warp_sums = per_b1 % 32 == 0;
     const double ginv = SM == PHX_SMEAR_GAUSSIAN ? 1.0 / A.sigma : 0.0;
     for (int x = tid; x < nb1 * per_b1; x += NT) {
-      const int nu = x % nph, b2 = (x / nph) % kMaxW, q = (x / (nph * kMaxW)) % kQT, b1 = x / per_b1;
+      const int nu = x % nph, b2 = (x / nph) % kMaxW, q = (x / (nph * kMaxW)) % QT, b1 = x / per_b1;
       double r[pairc::kMaxT];
 #pragma unroll
       for (int t = 0; t < pairc::kMaxT; ++t) r[t] = 0.0;
       const double en3 = s.E3[q * nph + nu];
       if (s.info[4 * q] && b2 < s.info[4 * q + 1] && en3 >= phxc::elPhononCutoff) {
         const double en1 = E1[b1], en2 = s.E2[q * kMaxW + b2];
-        const double2 wv = SM == PHX_SMEAR_ADAPTIVE ? s.wd[(q * kMaxW + b1) * kMaxW + b2] : make_double2(0.0, 0.0);
+        const double2 wv = SM == PHX_SMEAR_ADAPTIVE ? s.wd[(q * W1 + b1) * kMaxW + b2] : make_double2(0.0, 0.0);
         const double d1 = el_delta_tab<SM>(ginv, en1 - en2 + en3, wv);
         const double d2 = el_delta_tab<SM>(ginv, en1 - en2 - en3, wv);
         if (d1 > 0.0 || d2 > 0.0) {
-          const double c = s.cs[((q * kMaxW + b1) * kMaxW + b2) * nph + nu] * A.norm * phxc::pi / en3;
+          const double c = s.cs[((q * W1 + b1) * kMaxW + b2) * nph + nu] * A.norm * phxc::pi / en3;
 #pragma unroll
           for (int t = 0; t < pairc::kMaxT; ++t) {
             if (t < A.nT) {
@@ -573,46 +713,35 @@ __global__ void __launch_bounds__(kPairThreads) el_pair_kernel(ElArgs A) {
 // API variant: explicit final states (q3, U2, ev3), |g|^2 written out
 __global__ void __launch_bounds__(kPairThreads) elph_api_pair_kernel(
     const double2* __restrict__ cached, int nRp, int nph, int nw, int nb1, const double* __restrict__ Rp,
-    const double* __restrict__ degP, int nk2, const double* __restrict__ q3s, const double2* __restrict__ U2s,
+    const double* __restrict__ degP, const double* __restrict__ q3s, const double2* __restrict__ U2s,
     const int* __restrict__ nb2s, int nb2max, const double2* __restrict__ ev3s, double* __restrict__ out) {
   extern __shared__ __align__(16) char sraw[];
-  const PairSmem s = pair_carve(sraw, nRp, nph, nw);
+  const PairSmem s = pair_carve<1>(sraw, nRp, nph, nw, kMaxW);
   const int tid = threadIdx.x, NT = blockDim.x;
-  if (tid < kQT) {
-    const int j = blockIdx.x * kQT + tid;
-    s.info[4 * tid] = j < nk2;
-    s.info[4 * tid + 1] = j < nk2 ? nb2s[j] : 0;
-    s.info[4 * tid + 2] = j;
-    s.info[4 * tid + 3] = j;
+  const int j = blockIdx.x;   // one final state per block
+  if (tid == 0) {
+    s.info[0] = 1;
+    s.info[1] = nb2s[j];
+    s.info[2] = j;
+    s.info[3] = j;
   }
+  const double* q3 = q3s + 3 * (size_t)j;
+  for (int r = tid; r < nRp; r += NT) {
+    double sn, cs;
+    sincos(q3[0] * Rp[3 * r] + q3[1] * Rp[3 * r + 1] + q3[2] * Rp[3 * r + 2], &sn, &cs);
+    s.ph[r] = cmk(cs / degP[r], sn / degP[r]);
+  }
+  for (int i = tid; i < nw * kMaxW; i += NT) {
+    const int w = i / kMaxW, b2 = i % kMaxW;
+    s.U2[i] = b2 < nb2s[j] ? U2s[((size_t)j * nw + w) * nb2max + b2] : cmk(0.0, 0.0);
+  }
+  for (int i = tid; i < nph * nph; i += NT) s.ev3[i] = ev3s[(size_t)j * nph * nph + i];
   __syncthreads();
-  for (int i = tid; i < kQT * nRp; i += NT) {
-    const int q = i / nRp, r = i % nRp, j = blockIdx.x * kQT + q;
-    double2 v = cmk(0.0, 0.0);
-    if (j < nk2) {
-      const double* q3 = q3s + 3 * j;
-      double sn, cs;
-      sincos(q3[0] * Rp[3 * r] + q3[1] * Rp[3 * r + 1] + q3[2] * Rp[3 * r + 2], &sn, &cs);
-      v = cmk(cs / degP[r], sn / degP[r]);
-    }
-    s.ph[i] = v;
-  }
-  for (int i = tid; i < kQT * nw * kMaxW; i += NT) {
-    const int q = i / (nw * kMaxW), w = (i / kMaxW) % nw, b2 = i % kMaxW, j = blockIdx.x * kQT + q;
-    s.U2[i] = (j < nk2 && b2 < nb2s[j]) ? U2s[((size_t)j * nw + w) * nb2max + b2] : cmk(0.0, 0.0);
-  }
-  for (int i = tid; i < kQT * nph * nph; i += NT) {
-    const int q = i / (nph * nph), j = blockIdx.x * kQT + q;
-    s.ev3[i] = j < nk2 ? ev3s[(size_t)j * nph * nph + i % (nph * nph)] : cmk(0.0, 0.0);
-  }
-  __syncthreads();
-  pair_couplings<false>(cached, nRp, nph, nw, nb1, s);
-  for (int x = tid; x < kQT * nb1 * nb2max * nph; x += NT) {
-    const int nu = x % nph, b2 = (x / nph) % nb2max, b1 = (x / (nph * nb2max)) % nb1, q = x / (nph * nb2max * nb1);
-    const int j = blockIdx.x * kQT + q;
-    if (j >= nk2) continue;
+  pair_couplings<1, false>(cached, nRp, nph, nw, nb1, s);
+  for (int x = tid; x < nb1 * nb2max * nph; x += NT) {
+    const int nu = x % nph, b2 = (x / nph) % nb2max, b1 = x / (nph * nb2max);
     out[(((size_t)j * nb1 + b1) * nb2max + b2) * nph + nu] =
-        b2 < kMaxW ? s.cs[((q * kMaxW + b1) * kMaxW + b2) * nph + nu] : 0.0;
+        b2 < kMaxW ? s.cs[(b1 * kMaxW + b2) * nph + nu] : 0.0;
   }
 }
 
@@ -646,7 +775,7 @@ __global__ void el_batch_gather_kernel(const int* __restrict__ ik, int nb, const
                                        const int* __restrict__ hi, const double* __restrict__ kcart,
                                        const double2* __restrict__ Uk, int nw, double* __restrict__ kb,
                                        double2* __restrict__ ub, int* __restrict__ nbb, int* __restrict__ count) {
-  if (threadIdx.x == 0) *count = 0;   // of the batch's final states
+  if (threadIdx.x < kB1) count[threadIdx.x] = 0;   // of the batch's final states
   for (int i = threadIdx.x; i < kB1 * nw * nw; i += blockDim.x) {
     const int j = i / (nw * nw), w = (i / nw) % nw, b = i % nw;
     double2 v = cmk(0.0, 0.0);
@@ -717,11 +846,14 @@ int elph_cache_batch(phx_elph* e, int nb, const double* d_k1s, const double2* d_
     PHX_CUDA(ctx, cudaGetLastError());
     return PHX_OK;
   }
-  const size_t smem = sizeof(double2) * kB1 * e->nRe;
-  if (smem > 48 * 1024)
-    PHX_CUDA(ctx, cudaFuncSetAttribute(elph_g1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int grid = (int)std::min<size_t>((N + 255) / 256, (size_t)ctx->num_sms * 8);
-  elph_g1_kernel<<<grid, 256, smem, ctx->stream>>>(reinterpret_cast<const float2*>(e->d_g), e->nRe, N, e->d_Re,
+  const int mt = nb > 8 ? 2 : 1;
+  const auto g1_fn = mt == 2 ? elph_g1_kernel<2> : elph_g1_kernel<1>;
+  const size_t smem = sizeof(double2) * 32 * mt * ((e->nRe + 3) / 4);
+  // one limit on nRe for every batch size: the phases of kB1 k1
+  PHX_CUDA(ctx, cudaFuncSetAttribute(g1_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem * 2 / mt)));
+  const size_t tiles = (N + 8 * kG1Cols - 1) / (8 * kG1Cols);
+  const int grid = (int)std::min<size_t>((tiles + 7) / 8, (size_t)ctx->num_sms * 2);
+  g1_fn<<<grid, 256, smem, ctx->stream>>>(reinterpret_cast<const float2*>(e->d_g), e->nRe, N, e->d_Re,
                                                    e->d_degE, d_k1s, nb, d_g1);
   PHX_CUDA(ctx, cudaGetLastError());
   elph_rot_kernel<<<std::min<size_t>((N * nb + 255) / 256, (size_t)ctx->num_sms * 16), 256, 0, ctx->stream>>>(
@@ -732,7 +864,7 @@ int elph_cache_batch(phx_elph* e, int nb, const double* d_k1s, const double2* d_
 
 size_t pair_smem(const phx_elph* e) {
   size_t off[13];
-  return pair_smem_layout(e->nRp, e->nph, e->nw, off);
+  return pair_smem_layout<1>(e->nRp, e->nph, e->nw, kMaxW, off);
 }
 
 }  // namespace
@@ -848,8 +980,8 @@ extern "C" int phx_elph_couplings_sq(phx_elph* e, int nk2, const double* q3, con
   const size_t smem = pair_smem(e);
   PHX_ARG(ctx, smem <= 227 * 1024, "phx_elph_couplings_sq: too many phonon Bravais vectors");
   PHX_CUDA(ctx, cudaFuncSetAttribute(elph_api_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  elph_api_pair_kernel<<<(nk2 + kQT - 1) / kQT, kPairThreads, smem, ctx->stream>>>(
-      reinterpret_cast<const double2*>(e->d_cached), e->nRp, nph, nw, nb1, e->d_Rp, e->d_degP, nk2, dq, dU, dn,
+  elph_api_pair_kernel<<<nk2, kPairThreads, smem, ctx->stream>>>(
+      reinterpret_cast<const double2*>(e->d_cached), e->nRp, nph, nw, nb1, e->d_Rp, e->d_degP, dq, dU, dn,
       nb2max, dev, dout);
   PHX_CUDA(ctx, cudaGetLastError());
   PHX_CUDA(ctx, cudaMemcpyAsync(coupling, dout, sizeof(double) * (size_t)nk2 * nb1 * nb2max * nph,
@@ -977,14 +1109,25 @@ extern "C" int phx_el_linewidths(phx_elph* e, phx_bands* el, phx_bands* ph, cons
     ++launches;
   }
   size_t soff[13];
-  const size_t smem = pair_smem_layout(split ? 0 : e->nRp, nph, nw, soff);
+  size_t smem = pair_smem_layout<1>(split ? 0 : e->nRp, nph, nw, kMaxW, soff);
   PHX_ARG(ctx, smem <= 227 * 1024, "phx_el_linewidths: too many phonon Bravais vectors");
+  A.w1 = std::max(1, *std::max_element(nb1all.begin(), nb1all.end()));
+  // tiles of 8 final states where the buffers of a tile fit (343 Rp, 6 branches, 8
+  // orbitals and all 8 bands active: 122 KB); past that, as with 12 branches and 8
+  // active bands, one state at a time
+  const size_t tile_smem = pair_smem_layout<kTileQ>(split ? 0 : e->nRp, nph, nw, A.w1, soff);
+  const bool tiled = tile_smem <= 227 * 1024;
+  if (tiled) smem = tile_smem;
   constexpr int ad = PHX_SMEAR_ADAPTIVE, ga = PHX_SMEAR_GAUSSIAN;
-  const auto pair_fn = split ? (p->smearing == ad ? el_pair_kernel<true, ad> : el_pair_kernel<true, ga>)
-                             : (p->smearing == ad ? el_pair_kernel<false, ad> : el_pair_kernel<false, ga>);
+  const bool adaptive = p->smearing == ad;
+  const auto pair_fn = split && tiled ? (adaptive ? el_pair_kernel<kTileQ, true, ad> : el_pair_kernel<kTileQ, true, ga>)
+                       : split ? (adaptive ? el_pair_kernel<1, true, ad> : el_pair_kernel<1, true, ga>)
+                       : tiled ? (adaptive ? el_pair_kernel<kTileQ, false, ad> : el_pair_kernel<kTileQ, false, ga>)
+                               : (adaptive ? el_pair_kernel<1, false, ad> : el_pair_kernel<1, false, ga>);
+  const int pair_threads = tiled ? kTileThreads : kPairThreads;
   PHX_CUDA(ctx, cudaFuncSetAttribute(pair_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int resident = 1;   // pair blocks per SM
-  PHX_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, pair_fn, kPairThreads, smem));
+  PHX_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, pair_fn, pair_threads, smem));
   resident = std::max(1, resident);
   const int nq = ph->nq;
   const size_t per = N;
@@ -1012,6 +1155,7 @@ extern "C" int phx_el_linewidths(phx_elph* e, phx_bands* el, phx_bands* ph, cons
     // one launch for the batch: blockIdx.y = k1 of the batch
     A.cached = dcached;
     A.cper = per;
+    A.nb = nb;
     for (int j = 0; j < nb; ++j) {
       A.ik1s[j] = p->k1_list[rows[j]];
       A.i1s[j] = rows[j];
@@ -1023,7 +1167,7 @@ extern "C" int phx_el_linewidths(phx_elph* e, phx_bands* el, phx_bands* ph, cons
     }
     el_list_kernel<<<dim3((nq + 255) / 256, nb), 256, 0, st>>>(A);
     const int grid = (int)std::min<long long>((long long)nq * nb, (long long)resident * ctx->num_sms);
-    pair_fn<<<grid, kPairThreads, smem, st>>>(A);
+    pair_fn<<<grid, pair_threads, smem, st>>>(A);
     ++launches;
     ++launches;
     pairs += (long long)nq * nb;
