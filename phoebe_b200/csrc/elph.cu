@@ -142,24 +142,28 @@ __global__ void __launch_bounds__(256, 2) elph_g1_kernel(const float2* __restric
   }
 }
 
-// cached[b](Rp, nu, b1, w2) = sum_w1 g1[b](Rp, nu, w1, w2) U1[b][w1][b1]   (b1 < nb1[b], else 0)
+// cached[b](Rp, nu, b1, w2) = sum_w1 g1[b](Rp, nu, w1, w2) U1[b][w1][b1] for b1 < nb1[b];
+// the other bands are read by nothing and not written.  A thread keeps the nw
+// values of one (Rp, nu, w2) for all b1: g1 is read once.  Bound by reading g1:
+// 16 k1 of 2058 x 8 x 8 take 15 us (48 with one thread per (b1, w2), most of which
+// wrote zeros).
 __global__ void elph_rot_kernel(const double2* __restrict__ g1, int nRpPh, int nw, int nb,
                                 const double2* __restrict__ U1s, const int* __restrict__ nb1s,
                                 double2* __restrict__ cached) {
-  const size_t per = (size_t)nRpPh * nw * nw;
-  const size_t total = per * nb;
+  const size_t per = (size_t)nRpPh * nw, total = per * nb;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const int b = (int)(i / per);
-    const size_t rest = i % per;
-    const int w2 = (int)(rest % nw), b1 = (int)((rest / nw) % nw);
-    const size_t rp = rest / (nw * nw);
-    double2 acc = cmk(0.0, 0.0);
-    if (b1 < nb1s[b]) {
-      const double2* G = g1 + (size_t)b * per + rp * nw * nw;
-      const double2* U = U1s + (size_t)b * nw * nw;
-      for (int w1 = 0; w1 < nw; ++w1) acc = cadd(acc, cmul(G[w1 * nw + w2], U[w1 * nw + b1]));
+    const int b = (int)(i / per), w2 = (int)(i % nw), nb1 = nb1s[b];
+    const size_t at = (i / nw) * nw * nw + w2;   // (b, rp) row of nw x nw
+    double2 G[kMaxW];
+#pragma unroll
+    for (int w1 = 0; w1 < kMaxW; ++w1) G[w1] = w1 < nw ? g1[at + (size_t)w1 * nw] : cmk(0.0, 0.0);
+    for (int b1 = 0; b1 < nb1; ++b1) {
+      double2 acc = cmk(0.0, 0.0);
+#pragma unroll
+      for (int w1 = 0; w1 < kMaxW; ++w1)
+        if (w1 < nw) acc = cadd(acc, cmul(G[w1], __ldg(U1s + ((size_t)b * nw + w1) * nw + b1)));
+      cached[at + (size_t)b1 * nw] = acc;
     }
-    cached[i] = acc;
   }
 }
 
@@ -841,7 +845,7 @@ int elph_cache_batch(phx_elph* e, int nb, const double* d_k1s, const double2* d_
       PHX_TRY(phx_el_split_g_image(ctx, e->d_g, e->nRe, (long long)N, e->d_gimg));
     }
     PHX_TRY(phx_el_split_g1(ctx, e->d_gimg, e->nRe, (long long)N, e->d_Re, e->d_degE, nb, d_k1s, e->d_kimg, d_g1));
-    elph_rot_kernel<<<std::min<size_t>((N * nb + 255) / 256, (size_t)ctx->num_sms * 16), 256, 0, ctx->stream>>>(
+    elph_rot_kernel<<<std::min<size_t>((N / e->nw * nb + 255) / 256, (size_t)ctx->num_sms * 16), 256, 0, ctx->stream>>>(
         d_g1, e->nRp * e->nph, e->nw, nb, d_U1s, d_nb1s, d_cached);
     PHX_CUDA(ctx, cudaGetLastError());
     return PHX_OK;
@@ -856,7 +860,7 @@ int elph_cache_batch(phx_elph* e, int nb, const double* d_k1s, const double2* d_
   g1_fn<<<grid, 256, smem, ctx->stream>>>(reinterpret_cast<const float2*>(e->d_g), e->nRe, N, e->d_Re,
                                                    e->d_degE, d_k1s, nb, d_g1);
   PHX_CUDA(ctx, cudaGetLastError());
-  elph_rot_kernel<<<std::min<size_t>((N * nb + 255) / 256, (size_t)ctx->num_sms * 16), 256, 0, ctx->stream>>>(
+  elph_rot_kernel<<<std::min<size_t>((N / e->nw * nb + 255) / 256, (size_t)ctx->num_sms * 16), 256, 0, ctx->stream>>>(
       d_g1, e->nRp * e->nph, e->nw, nb, d_U1s, d_nb1s, d_cached);
   PHX_CUDA(ctx, cudaGetLastError());
   return PHX_OK;
@@ -1138,7 +1142,7 @@ extern "C" int phx_el_linewidths(phx_elph* e, phx_bands* el, phx_bands* ph, cons
     std::vector<int> nbb(kB1, 0);
     for (int j = 0; j < nb; ++j) nbb[j] = nb1all[rows[j]];
     // k1 coordinates, band counts and U1 of the batch, gathered on the device
-    el_batch_gather_kernel<<<1, 256, 0, st>>>(dactik + b0, nb, dlo, dhi, el->d_q,
+    el_batch_gather_kernel<<<1, 1024, 0, st>>>(dactik + b0, nb, dlo, dhi, el->d_q,
                                               reinterpret_cast<const double2*>(el->d_U), nw, dkb, dub, dnb, dcount);
     ++launches;
     PHX_CUDA(ctx, cudaGetLastError());
