@@ -10,14 +10,14 @@
 // TMEM regions, so the MMA of one part overlaps the CUDA-core epilogue of the
 // others.
 //
-// Epilogue (12 warps; TMEM lane quarter = warp & 3 = 32 q1 rows, k = warp >> 2):
-//  * the three warps of a quarter stage the records of q3 = q1 + q2 for their
+// Epilogue (16 warps; TMEM lane quarter = warp & 3 = 32 q1 rows, k = warp >> 2):
+//  * the four warps of a quarter stage the records of q3 = q1 + q2 for their
 //    rows (one 592-byte record per mesh point: FP32 eigenvectors, energies,
 //    velocity projections, Bose factors, degenerate blocks);
-//  * warp k decides, for b2 = 2k, 2k+1 and every (b1, b3), whether any of the
-//    three delta functions of the triplet can be non-zero (FP32 windows with a
-//    rounding margin); the masks are shared in shared memory;
-//  * warp k handles the rows (b1, b2) with (b1 + b2) % 3 == k: it contracts
+//  * warp k decides, for three of the twelve (b2, half of b3) and every b1,
+//    whether any of the three delta functions of the triplet can be non-zero
+//    (FP32 windows with a rounding margin); the masks are shared in shared memory;
+//  * warp k handles three of the twelve rows (b1, b2) of a part: it contracts
 //    the rows of X it needs with e1 and e3 in FP32 and queues the live
 //    triplets (|V|^2 and indices) in shared memory; 32 queued triplets at a
 //    time get their delta functions and Bose factors with every lane busy,
@@ -50,8 +50,9 @@ constexpr int kNH = 144;           // N columns per part: 2 b2 x 36 (a,c) x {re,
 constexpr int kStages = 2;
 constexpr int kRegion = 160;       // TMEM columns per accumulator region (>= kNH)
 constexpr int kTmemCols = 512;
-constexpr int kEpiWarps = 12;
-constexpr int kThreads = (kEpiWarps + 2) * 32;
+constexpr int kQW = 4;             // epilogue warps per quarter of the tile
+constexpr int kEpiWarps = 4 * kQW;
+constexpr int kThreads = (kEpiWarps + 4) * 32;   // + producer, MMA issuer, two idle warps
 constexpr uint32_t kPartBytes = kNH * kKC * 2;    // one of hi / lo: 4608 B
 constexpr uint32_t kStageBytes = 2 * kPartBytes;  // hi + lo: 9216 B
 constexpr uint32_t kBSbo = (kKC / 8) * 128;       // 256 B between 8-row groups
@@ -71,11 +72,12 @@ constexpr int kU2Chunks = kRecChunks - kChBand;   // band blocks + blocks word
 //    q1, padded to an odd stride so that the rows of a warp fall in distinct
 //    banks;
 //  * kQueue: live-triplet queue entries per warp (a push round adds at most
-//    32 to fewer than 32 queued).
+//    32 to fewer than 32 queued: 63 entries, which keep the arrays of 16 warps
+//    within the limit on R3 that 12 warps had).
 template <int NT>
 struct Pcfg {
   static constexpr int kAccRow = 6 * NT + 1;
-  static constexpr int kQueue = 64;
+  static constexpr int kQueue = 63;
 };
 
 struct TcArgs {
@@ -458,7 +460,7 @@ __device__ __noinline__ unsigned expand_b3(unsigned c, unsigned gp3) {
   return o;
 }
 
-// Liveness of (b1, b2, b3) for all b1 at one (b2, b3): bit b1 is set when
+// Liveness of (b1, b2, b3) for all b1 at one (b2, b3): bit 3 b1 is set when
 // one of the three deltas may be non-zero (FP32 windows widened by tol).
 __device__ __forceinline__ unsigned live6(int smearing, float sg, float tol, const float* E1f,
                                           float E2f, float E2mf, const Band& x2, const Band& x2m,
@@ -483,7 +485,7 @@ __device__ __forceinline__ unsigned live6(int smearing, float sg, float tol, con
 #pragma unroll
   for (int b1 = 0; b1 < 6; ++b1) {
     const bool live = fabsf(E1f[b1] - cp) <= hp || fabsf(E1f[b1] - c1) <= hm || fabsf(E1f[b1] - c2) <= hm;
-    msk |= live ? (1u << b1) : 0u;
+    msk |= live ? (1u << (3 * b1)) : 0u;
   }
   return msk;
 }
@@ -492,8 +494,13 @@ __device__ __forceinline__ unsigned live6(int smearing, float sg, float tol, con
 // the fused pair kernel
 // ---------------------------------------------------------------------------
 
-// Warp roles (448 threads): warps 0-11 epilogue, warp 12 producer (bulk
-// copies of B stages), warp 13 MMA issuer.
+// Warp roles (640 threads): warps 0-15 epilogue, warp 16 producer (bulk
+// copies of B stages), warp 17 MMA issuer, two idle (they cost nothing, and the
+// code compiled for 576 threads spilled more: 96.0 instead of 92.9 ms at 20^3).  The epilogue issues on half of the
+// cycles (FMA pipe 19%, ALU 31%, tensor pipe 6%; the rest waits for TMEM, shared
+// memory and branches), so its warps count more than their registers: 16 at 96
+// against 12 at 128 registers, with a few spills outside the loops: 20^3
+// adaptive, 3 temperatures, 94.7 -> 92.9 ms, 12^3 8.70 -> 8.35 ms.
 struct Smem {
   uint32_t aPart;
   uint8_t* A;          // [hi | lo] 128 x Kp BF16
@@ -504,8 +511,8 @@ struct Smem {
   float* N1;           // [NT*6][128]
   uint4* rec;          // staged q3 records [kRecChunks][128]
   uint4* u2;           // [4 quarters][2: q2, -q2][kU2Chunks]
-  unsigned long long* need;  // [6 b2][128] bit b1*6+b3
-  uint2* queue;        // [12 warps][kQueue] live triplets awaiting their rates
+  unsigned* need;      // [6 b2][2: b3 < 3, b3 >= 3][128] bit b1*3 + b3%3
+  uint2* queue;        // [kEpiWarps][kQueue] live triplets awaiting their rates
   float* acc;          // [4 quarters][32 rows][kAccRow: 6 b1 x NT + pad] rates of the current q2
   uint64_t* bars;
 };
@@ -524,7 +531,7 @@ __host__ __device__ inline size_t smem_layout(int Kp, size_t* off) {
   off[5] = o; o += align16(NT * 6 * kM * sizeof(float));       // N1
   off[6] = o; o += align16((size_t)kRecChunks * kM * 16);      // staged records
   off[7] = o; o += align16(4 * 2 * kU2Chunks * 16);            // q2 bands
-  off[8] = o; o += align16(6 * kM * sizeof(unsigned long long));  // masks
+  off[8] = o; o += align16(12 * kM * sizeof(unsigned));        // masks
   off[9] = o; o += align16(kEpiWarps * Pcfg<NT>::kQueue * sizeof(uint2));   // queues
   off[10] = o; o += align16(4 * 32 * Pcfg<NT>::kAccRow * sizeof(float));  // q2 accumulators
   off[11] = o; o += align16(32 * sizeof(uint64_t));            // barriers, tmem slot, flag
@@ -545,7 +552,7 @@ __device__ __forceinline__ Smem carve(uint8_t* base, int Kp) {
   s.N1 = reinterpret_cast<float*>(base + off[5]);
   s.rec = reinterpret_cast<uint4*>(base + off[6]);
   s.u2 = reinterpret_cast<uint4*>(base + off[7]);
-  s.need = reinterpret_cast<unsigned long long*>(base + off[8]);
+  s.need = reinterpret_cast<unsigned*>(base + off[8]);
   s.queue = reinterpret_cast<uint2*>(base + off[9]);
   s.acc = reinterpret_cast<float*>(base + off[10]);
   s.bars = reinterpret_cast<uint64_t*>(base + off[11]);
@@ -625,7 +632,7 @@ __global__ void __launch_bounds__(kThreads, 1) pair_tc_kernel(TcArgs P) {
   uint64_t* full = S.bars;                // [kStages]
   uint64_t* empty = full + kStages;       // [kStages]
   uint64_t* accf = empty + kStages;       // [kParts] MMA of a part done
-  uint64_t* acce = accf + kParts;         // [kParts] part released by the 12 epilogue warps
+  uint64_t* acce = accf + kParts;         // [kParts] part released by the epilogue warps
   uint64_t* done = acce + kParts;         // MMA drain
   uint64_t* stg = done + 1;               // [4] q3 records of a quarter staged
   uint64_t* lvb = stg + 4;                // [4] liveness masks of a quarter written
@@ -648,9 +655,9 @@ __global__ void __launch_bounds__(kThreads, 1) pair_tc_kernel(TcArgs P) {
     }
     tc::mbar_init(done, 1);
     for (int q = 0; q < 4; ++q) {
-      tc::mbar_init(&stg[q], 96);
-      tc::mbar_init(&lvb[q], 96);
-      tc::mbar_init(&rel[q], 96);
+      tc::mbar_init(&stg[q], 32 * kQW);
+      tc::mbar_init(&lvb[q], 32 * kQW);
+      tc::mbar_init(&rel[q], 32 * kQW);
     }
     *abort_flag = 0;
     tc::fence_mbar_init();
@@ -755,12 +762,12 @@ __global__ void __launch_bounds__(kThreads, 1) pair_tc_kernel(TcArgs P) {
       tc::mma_commit(done);
       tc::mbar_wait_sleep(done, 0, P.status, 8);
     }
-  } else {
+  } else if (warp < kEpiWarps) {
     // ---------------- epilogue ----------------
-    // Warp k of quarter qd handles the rows (b1, b2) with (b1 + b2) % 3 == k,
-    // so the three warps of a quarter share every b2 and every b1 evenly; the
-    // rates go to FP32 accumulators of the quarter (one q2 at a time), which
-    // warp k folds into FP64 registers for b1 = k and k + 3.
+    // Of the twelve rows (b1, b2) of a part, in the order of b2 and then b1,
+    // warp k of quarter qd handles k, k + 4 and k + 8, so the four warps share
+    // every part evenly; the rates go to FP32 accumulators of the quarter (one
+    // q2 at a time), which warp k folds into FP64 registers for b1 = k and k + 4.
     const int qd = warp & 3, k = warp >> 2;
     const int m = qd * 32 + lane;
     const bool valid = tile0 + m < nq;
@@ -778,7 +785,7 @@ __global__ void __launch_bounds__(kThreads, 1) pair_tc_kernel(TcArgs P) {
     const bool deg1 = gp1 != kIdentityBlocks;
     unsigned ok1 = 0;
 #pragma unroll
-    for (int b = 0; b < 6; ++b) ok1 |= (valid && S.En1[b * kM + m] >= phxc::phExcludeCutoff) ? (1u << b) : 0u;
+    for (int b = 0; b < 6; ++b) ok1 |= (valid && S.En1[b * kM + m] >= phxc::phExcludeCutoff) ? (1u << (3 * b)) : 0u;
     double acc0[NT], acc1[NT];
 #pragma unroll
     for (int t = 0; t < NT; ++t) acc0[t] = acc1[t] = 0.0;
@@ -790,7 +797,7 @@ __global__ void __launch_bounds__(kThreads, 1) pair_tc_kernel(TcArgs P) {
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
       qacc[lane * AR + k * NT + t] = 0.f;
-      qacc[lane * AR + (k + 3) * NT + t] = 0.f;
+      if (k + kQW < 6) qacc[lane * AR + (k + kQW) * NT + t] = 0.f;
     }
     int qn = 0;  // queued live triplets (warp-uniform)
     const unsigned lanemask_lt = (1u << lane) - 1u;
@@ -800,9 +807,11 @@ __global__ void __launch_bounds__(kThreads, 1) pair_tc_kernel(TcArgs P) {
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
         acc0[t] += (double)qacc[lane * AR + k * NT + t];
-        acc1[t] += (double)qacc[lane * AR + (k + 3) * NT + t];
         qacc[lane * AR + k * NT + t] = 0.f;
-        qacc[lane * AR + (k + 3) * NT + t] = 0.f;
+        if (k + kQW < 6) {
+          acc1[t] += (double)qacc[lane * AR + (k + kQW) * NT + t];
+          qacc[lane * AR + (k + kQW) * NT + t] = 0.f;
+        }
       }
     };
     bool failed = false;
@@ -818,8 +827,8 @@ __global__ void __launch_bounds__(kThreads, 1) pair_tc_kernel(TcArgs P) {
       {
         const uint4* src = P.rec + (size_t)iq3 * kRecChunks;
 #pragma unroll 1
-        for (int c = k; c < kRecChunks; c += 3) cp_async16(&S.rec[c * kM + m], src + c);
-        if (k == 2 && lane < kU2Chunks) {
+        for (int c = k; c < kRecChunks; c += kQW) cp_async16(&S.rec[c * kM + m], src + c);
+        if (k == kQW - 1 && lane < kU2Chunks) {
           cp_async16(&u2[lane], P.rec + (size_t)iq2 * kRecChunks + kChBand + lane);
           cp_async16(&u2[kU2Chunks + lane], P.rec + (size_t)iq2m * kRecChunks + kChBand + lane);
         }
@@ -830,33 +839,28 @@ __global__ void __launch_bounds__(kThreads, 1) pair_tc_kernel(TcArgs P) {
       const unsigned gp2 = u2[kU2Chunks - 1].x;
       const unsigned gp3 = srow[kChGp * kM].x;
       const bool deg2 = gp2 != kIdentityBlocks, deg3 = gp3 != kIdentityBlocks;
-      // ---- liveness of b2 = 2k, 2k+1 for all (b1, b3)
+      // ---- liveness of three of the twelve (b2, half of b3) for all b1
       {
         float E1f[6];
 #pragma unroll
         for (int b = 0; b < 6; ++b) E1f[b] = (float)S.En1[b * kM + m];
 #pragma unroll 1
-        for (int bl = 0; bl < 2; ++bl) {
-          const int b2 = 2 * k + bl;
+        for (int u = 3 * k; u < 3 * k + 3; ++u) {
+          const int b2 = u >> 1, b30 = 3 * (u & 1);
           const Band x2 = load_band<1>(u2 + 3 * b2, 1);
           const Band x2m = load_band<1>(u2 + kU2Chunks + 3 * b2, 1);
           const float E2f = (float)x2.E, E2mf = (float)x2m.E;
           const bool ok2 = x2.E >= phxc::phExcludeCutoff, ok2m = x2m.E >= phxc::phExcludeCutoff;
-          unsigned long long nd = 0;
+          unsigned nd = 0;
           if (ok2 || ok2m) {
 #pragma unroll 1
-            for (int b3 = 0; b3 < 6; ++b3) {
-              const Band x3 = load_band<1>(srow + (kChBand + 3 * b3) * kM, kM);
+            for (int b3 = 0; b3 < 3; ++b3) {
+              const Band x3 = load_band<1>(srow + (kChBand + 3 * (b30 + b3)) * kM, kM);
               if (!(x3.E >= phxc::phEnergyCutoff)) continue;
-              const unsigned c = live6(smearing, sg, P.tol, E1f, E2f, E2mf, x2, x2m, ok2, ok2m,
-                                       (float)x3.E, x3) & ok1;
-              unsigned long long sp = 0;
-#pragma unroll
-              for (int b1 = 0; b1 < 6; ++b1) sp |= (unsigned long long)((c >> b1) & 1u) << (6 * b1);
-              nd |= sp << b3;
+              nd |= (live6(smearing, sg, P.tol, E1f, E2f, E2mf, x2, x2m, ok2, ok2m, (float)x3.E, x3) & ok1) << b3;
             }
           }
-          S.need[b2 * kM + m] = nd;
+          S.need[u * kM + m] = nd;
         }
       }
       tc::mbar_arrive(&lvb[qd]);
@@ -869,18 +873,23 @@ __global__ void __launch_bounds__(kThreads, 1) pair_tc_kernel(TcArgs P) {
 #pragma unroll 1
         for (int bl = 0; bl < 2; ++bl) {
           const int b2 = 2 * h + bl;
-          const int r0 = (k + 6 - b2 % 3) % 3;       // owned b1 = r0, r0 + 3
+          const int r0 = (k + 2 * bl) & (kQW - 1);   // owned b1 = r0 and, if below 6, r0 + 4
+          const bool two = r0 + kQW < 6;
           const unsigned bmO0 = deg1 ? blk_mask(gp1, r0) : (1u << r0);
-          const unsigned bmO1 = deg1 ? blk_mask(gp1, r0 + 3) : (1u << (r0 + 3));
+          const unsigned bmO1 = !two ? 0u : deg1 ? blk_mask(gp1, r0 + kQW) : (1u << (r0 + kQW));
           // b3 masks of the owned b1 (expanded over the blocks of b2 and b3)
-          unsigned long long nsrc = S.need[b2 * kM + m];
+          unsigned nlo = S.need[2 * b2 * kM + m], nhi = S.need[(2 * b2 + 1) * kM + m];
           const unsigned bm2 = deg2 ? blk_mask(gp2, b2) : (1u << b2);
           if (bm2 != (1u << b2)) {
             for (int b = 0; b < 6; ++b)
-              if (b != b2 && ((bm2 >> b) & 1u)) nsrc |= S.need[b * kM + m];
+              if (b != b2 && ((bm2 >> b) & 1u)) {
+                nlo |= S.need[2 * b * kM + m];
+                nhi |= S.need[(2 * b + 1) * kM + m];
+              }
           }
-          unsigned nO0 = (unsigned)(nsrc >> (6 * r0)) & 63u;
-          unsigned nO1 = (unsigned)(nsrc >> (6 * (r0 + 3))) & 63u;
+          auto live_b3 = [&](int b1) { return ((nlo >> (3 * b1)) & 7u) | (((nhi >> (3 * b1)) & 7u) << 3); };
+          unsigned nO0 = live_b3(r0);
+          unsigned nO1 = two ? live_b3(r0 + kQW) : 0u;
           if (deg3) {
             if (nO0) nO0 = expand_b3(nO0, gp3);
             if (nO1) nO1 = expand_b3(nO1, gp3);
@@ -966,7 +975,7 @@ __global__ void __launch_bounds__(kThreads, 1) pair_tc_kernel(TcArgs P) {
                   const int nd = __popc(o ? bmO1 : bmO0) * n23;
                   const float ws = nd == 1 ? w : w / (float)nd;
                   queue[qn + __popc(bal & lanemask_lt)] =
-                      make_uint2(__float_as_uint(ws), (unsigned)lane | ((unsigned)(r0 + 3 * o) << 5) |
+                      make_uint2(__float_as_uint(ws), (unsigned)lane | ((unsigned)(r0 + kQW * o) << 5) |
                                                           ((unsigned)(__ffs(m2) - 1) << 8) |
                                                           ((unsigned)(__ffs(m3) - 1) << 11));
                   m3 &= m3 - 1;
@@ -1016,7 +1025,7 @@ __global__ void __launch_bounds__(kThreads, 1) pair_tc_kernel(TcArgs P) {
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
         out[k * NT + t] += acc0[t];
-        out[(k + 3) * NT + t] += acc1[t];
+        if (k + kQW < 6) out[(k + kQW) * NT + t] += acc1[t];
       }
     }
   }

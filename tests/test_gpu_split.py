@@ -98,3 +98,18 @@ def test_near_cutoff_events_beyond_the_list_capacity(ctx, diamond):
     A64, _, _, _ = _builder(ctx, diamond, mesh, "adaptive", temps, "fp64")
     rel64 = np.abs(A1 - A64)[big] / np.abs(A64)[big]
     assert rel64.max() < 1e-5, rel64.max()
+
+
+@pytest.mark.parametrize("mesh,smearing,temps", [((3, 5, 2), "gaussian", (300.0, 600.0)),
+                                                 ((7, 3, 7), "adaptive", (300.0, 600.0)),
+                                                 ((4, 8, 4), "gaussian", (100.0, 200.0, 300.0, 600.0)),
+                                                 ((9, 9, 9), "adaptive", (100.0, 200.0, 300.0, 600.0))])
+def test_split_tile_remainders(ctx, diamond, mesh, smearing, temps):
+    """Fewer points than a tile has rows, one tile full, remainders, and the shared
+    memory filled to its limit (4 temperatures, 43 R3), at the bar of the other meshes."""
+    A64, _, E, _ = _builder(ctx, diamond, mesh, smearing, temps, "fp64")
+    A16, _, _, _ = _builder(ctx, diamond, mesh, smearing, temps, "split_fp16")
+    big = (E.reshape(-1) >= C.phExcludeCutoff)[None, :] & (np.abs(A64) > 1e-8 * np.abs(A64).max())
+    assert big.any()
+    rel = np.abs(A16 - A64)[big] / np.abs(A64)[big]
+    assert rel.max() < 1e-5, rel.max()
