@@ -868,17 +868,32 @@ std::map<PlanKey, BuilderPlan> g_plans;
 // set-up of phases and eigenvectors costs).  Measured: split 5^3 2.02 -> 0.40
 // ms a call (7 -> 125 slots), FP64 8^3 4.3 -> 2.2 ms (8 -> 18 slots).
 // (slot_bytes: one slot's sums; at most 64 MB of them beyond the fixed count).
+long slot_cost(int tiles, int cnt, int s, int sms) {
+  return (((long)tiles * s + sms - 1) / sms) * ((cnt + s - 1) / s + 1);
+}
 int fill_slots(int tiles, int cnt, int fixed, int sms, size_t slot_bytes) {
   int best = std::min(fixed, cnt);
   long best_cost = -1;
   for (int s = 1; s <= cnt && (s <= fixed || s * slot_bytes <= (size_t(64) << 20)); ++s) {
-    const long waves = ((long)tiles * s + sms - 1) / sms, cost = waves * ((cnt + s - 1) / s + 1);
+    const long cost = slot_cost(tiles, cnt, s, sms);
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;
       best = s;
     }
   }
   return best;
+}
+
+// The same where the fixed count may fill the SMs well: it stays unless the
+// other costs 5% less by that measure (many waves even out by themselves, and
+// more, shorter blocks then balance tiles of unequal work better).  Measured:
+// FP64 matrix 11^3 21.8 -> 15.6 ms (8 -> 7 slots, 152 -> 133 blocks on 148 SMs),
+// BF16 matrix 15x13x11 11.7 -> 10.6 (28 -> 26).
+int better_slots(int tiles, int cnt, int fixed, int sms, size_t slot_bytes) {
+  cnt = std::max(1, cnt);
+  fixed = std::min(fixed, cnt);
+  const int s = fill_slots(tiles, cnt, fixed, sms, slot_bytes);
+  return 20 * slot_cost(tiles, cnt, s, sms) < 19 * slot_cost(tiles, cnt, fixed, sms) ? s : fixed;
 }
 
 bool find_plan(const PlanKey& k, BuilderPlan* out) {
@@ -1576,7 +1591,19 @@ int run_matrix_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
     const size_t per_q2 = 2 * sizeof(double) * (size_t)nT * ns * NB;
     chunk = (int)std::max<size_t>(1, std::min<size_t>(chunk, (size_t(4) << 30) / per_q2));
   }
-  const int slots = std::min(split ? (full ? 28 : 7) : 8, chunk);
+  // slots of a full chunk and of the remainder; the partial sums hold the larger count
+  const int tiles_pair = (nq + (split ? 127 : pair64::tile_q1(nr3) - 1)) / (split ? 128 : pair64::tile_q1(nr3));
+  const size_t slot_bytes = sizeof(double) * nq * NB * nT;
+  // (a grid within one wave stays as it is: the order of the few atomic sums of a
+  // matrix element then does not depend on which blocks run side by side)
+  const int fixed_slots = split ? (full ? 28 : 7) : 8;
+  auto chunk_slots = [&](int cnt) {
+    return tiles_pair * std::min(fixed_slots, cnt) <= ctx->num_sms
+               ? std::min(fixed_slots, cnt)
+               : better_slots(tiles_pair, cnt, fixed_slots, ctx->num_sms, slot_bytes);
+  };
+  const int rest = (q2e - q2b) % std::max(1, chunk);
+  const int slots = std::max(chunk_slots(chunk), rest ? chunk_slots(rest) : 1);
   const size_t nb3 = (size_t)NB * NB * NB;
   const size_t sz_dp = align_up(split ? sizeof(double2) * chunk * nr3 * nb3 : pair64::image_bytes(nr3) * chunk);
   const size_t sz_part = align_up(sizeof(double) * slots * nq * NB * nT);
@@ -1684,7 +1711,7 @@ int run_matrix_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
         fold_tiled_launch(NB, nr2, nr3, v, b, c0, cnt, Dp, st, fp16 ? dmax : nullptr);
         ++launches;
         const phx_split_matrix mo{full ? A_full : slabP, slabM, (long long)ns, slab_elems, full ? 1 : 0};
-        PHX_TRY(phx_split_pair_chunk(ctx, P.m, v, b, Dp, Bimg, rec, b->emax, c0, cnt, slots, partial, &launches,
+        PHX_TRY(phx_split_pair_chunk(ctx, P.m, v, b, Dp, Bimg, rec, b->emax, c0, cnt, chunk_slots(cnt), partial, &launches,
                                      nullptr, nullptr, fp16, dmax, edges, edge_count, phx_split_edge_cap(),
                                      edge_peak, edge_over, 0, &mo));
       } else {
@@ -1695,8 +1722,8 @@ int run_matrix_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
         pair64::Args Q = P;
         Q.q2_first = c0;
         Q.q2_count = cnt;
-        Q.q2_per_slot = (cnt + slots - 1) / slots;
-        PHX_CUDA(ctx, pair64::launch_pair(Q, slots, true, st));
+        Q.q2_per_slot = (cnt + chunk_slots(cnt) - 1) / chunk_slots(cnt);
+        PHX_CUDA(ctx, pair64::launch_pair(Q, chunk_slots(cnt), true, st));
         ++launches;
       }
       if (!full) {
