@@ -1049,6 +1049,8 @@ int run_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Aout_d,
   const int nq = b->nq, nT = p->num_temperatures, nr3 = v->nr3, nr2 = v->nr2;
   const int q2b = p->q2_begin, q2e = p->q2_end;
   const bool split = v->precision != PHX_PREC_FP64;
+  // (ahead of every size that is derived from it: past 1376 not one warp's phases fit)
+  PHX_ARG(ctx, split || nr3 <= pair64::kMaxR3, "phx_ph_linewidths: too many R3 vectors for the FP64 path");
   // candidate plans; the first is the default
   std::vector<BuilderPlan> cands;
   if (split)
@@ -1134,10 +1136,7 @@ int run_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Aout_d,
   P.img = reinterpret_cast<const double*>(Dp);
   P.partial = partial;
   P.status = ctx->d_status;
-  if (!split) {
-    PHX_ARG(ctx, nr3 <= pair64::kMaxR3, "phx_ph_linewidths: too many R3 vectors for the FP64 path");
-    PHX_CUDA(ctx, pair64::set_attributes(nr3, false, p->smearing));
-  }
+  if (!split) PHX_CUDA(ctx, pair64::set_attributes(nr3, false, p->smearing));
   const size_t smem_fold = fold_tiled_smem(NB, nr2);
   PHX_ARG(ctx, smem_fold <= 227 * 1024, "phx_ph_linewidths: too many R2 vectors");
   if (smem_fold > 48 * 1024)
@@ -1583,6 +1582,7 @@ int run_matrix_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
   const bool full = A_full != nullptr;
   const bool split = v->precision != PHX_PREC_FP64;
   const int fp16 = v->precision == PHX_PREC_SPLIT_FP16 ? 1 : 0;
+  PHX_ARG(ctx, split || nr3 <= pair64::kMaxR3, "scattering matrix: too many R3 vectors for the FP64 path");
   // plan: the FP64 kernel's default, or the split kernel's large plan (the
   // matrix-free mode takes its small one: the slabs are zeroed per chunk);
   // slab memory of mode 1: at most 4 GiB for the two slabs of all temperatures
@@ -1674,7 +1674,6 @@ int run_matrix_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
   P.ld = ns;
   P.mat_tstride = slab_elems;
   P.mat_full = full ? 1 : 0;
-  PHX_ARG(ctx, nr3 <= pair64::kMaxR3, "scattering matrix: too many R3 vectors for the FP64 path");
   if (!split) PHX_CUDA(ctx, pair64::set_attributes(nr3, true, p->smearing));
   const size_t smem_fold = fold_tiled_smem(NB, nr2);
   PHX_ARG(ctx, smem_fold <= 227 * 1024, "scattering matrix: too many R2 vectors");

@@ -17,7 +17,7 @@ pytestmark = pytest.mark.gpu
 
 def _fc3(cr, nr3):
     """A random real tensor on one R2 and nr3 R3 vectors (no sum rule: the kernels need none)."""
-    R, _ = synth.lattice_cube(cr, 3)
+    R, _ = synth.lattice_cube(cr, 3 if nr3 <= 343 else 6)
     rng = np.random.default_rng(nr3)
     o = np.argsort(np.linalg.norm(R, axis=1), kind="stable")
     D3 = rng.normal(size=(6, 6, 6, nr3, 1)) * 0.05
@@ -63,6 +63,25 @@ def test_linewidths_at_tile_edges(ctx, mesh, nr3, smearing, temps):
     rest = [sm.setup(0, 1, finalize=False), sm.setup(2, bands.nq, finalize=False)]
     whole = sm.setup(finalize=False)
     np.testing.assert_allclose(part + rest[0] + rest[1], whole, rtol=1e-12, atol=1e-14 * np.abs(whole).max())
+    v3.close()
+    bands.close()
+
+
+@pytest.mark.parametrize("nr3", [263, 1376, 1377, 1400])
+def test_too_many_r3_vectors_are_refused(ctx, nr3):
+    """Past 262 R3 vectors the path returns an error, also past 1376, where no warp's phases fit."""
+    from phoebe_b200.core import Interaction3Ph, PhScatteringMatrix
+    cr = synth.diamond_crystal()
+    bands = _bands(ctx, cr, (2, 2, 1))
+    v3 = Interaction3Ph(ctx, cr, _fc3(cr, nr3))
+    T = [C.kelvin_to_ry(300.0)]
+    sm = PhScatteringMatrix(v3, bands, T)
+    with pytest.raises(RuntimeError, match="too many R3 vectors"):
+        sm.setup()
+    with pytest.raises(RuntimeError, match="too many R3 vectors"):
+        sm.dot(np.zeros((1, 3, sm.num_states)))
+    with pytest.raises(RuntimeError, match="too many R3 vectors"):
+        PhScatteringMatrix(v3, bands, T, in_memory=True).setup()
     v3.close()
     bands.close()
 
