@@ -861,39 +861,51 @@ struct PlanKey {
 std::mutex g_plan_mutex;
 std::map<PlanKey, BuilderPlan> g_plans;
 
-// Slots of a chunk of `cnt` q2 for `tiles` q1 tiles: one block per (tile,
-// slot), one block per SM.  The fixed slot counts of the tuned plans leave most
-// SMs idle when there are few tiles (5^3: one tile), so this one takes the
-// count that minimises waves x (q2 of a slot + one, about what a block's
-// set-up of phases and eigenvectors costs).  Measured: split 5^3 2.02 -> 0.40
-// ms a call (7 -> 125 slots), FP64 8^3 4.3 -> 2.2 ms (8 -> 18 slots).
-// (slot_bytes: one slot's sums; at most 64 MB of them beyond the fixed count).
+// Time of a chunk of `cnt` q2 for `tiles` q1 tiles in s slots, in quarters of a q2 of one
+// tile: one block per (tile, slot), the tiles of a slot next to each other, taken in order by
+// the SMs as they come free, one block per SM.  A block costs its q2 and half a q2 of set-up
+// (phases, eigenvectors).  What is live differs from tile to tile by about half, which one
+// wave of long blocks waits for and many short blocks even out: half a block on top.
 long slot_cost(int tiles, int cnt, int s, int sms) {
-  return (((long)tiles * s + sms - 1) / sms) * ((cnt + s - 1) / s + 1);
+  const int per = (cnt + s - 1) / s, rest = cnt % per;
+  const long block = 2 * per + 1, blocks = (long)tiles * (cnt / per), late = blocks % sms;
+  long early_end = blocks / sms * block, late_end = early_end + block;   // SMs without and with one more
+  long end = late ? late_end : early_end;
+  if (rest)   // the blocks of the last slot
+    for (long left = tiles; left > 0;) {
+      const bool on_late = late && late_end < early_end;
+      long& t = on_late ? late_end : early_end;
+      t += 2 * rest + 1;
+      left -= on_late ? late : sms - late;
+      end = std::max(end, t);
+    }
+  return 2 * end + block;
 }
+
+// Slots of a chunk: the fixed count of the untuned plan, unless by that measure another one
+// takes less than 95% of its time, or less than 80% with at most 150 q2, where what the few q2 and
+// tiles have alive decides more than the measure.  (Few tiles leave most SMs idle: 5^3 is one tile
+// of the split kernel.)  One slot's sums are slot_bytes; at most 64 MB of them beyond the fixed
+// count.  Swept over 7 meshes from 5^3 to 24^3 and 4 to 800 q2 against every slot count (pair
+// kernel, split FP16 / FP64): the fixed counts of 7 and 8 lose 35% / 22% to the best one, waves x
+// (q2 of a slot + one) 6% / 12% and up to 38% to the fixed ones (20^3, 32 q2: 2 slots 676 us, 7
+// slots 506), this rule 2% / 4% and is nowhere slower than the fixed ones.  5^3, all q2: 1187 ->
+// 133 us.
 int fill_slots(int tiles, int cnt, int fixed, int sms, size_t slot_bytes) {
-  int best = std::min(fixed, cnt);
-  long best_cost = -1;
+  cnt = std::max(1, cnt);
+  fixed = std::min(fixed, cnt);
+  int best = fixed;
+  long best_cost = slot_cost(tiles, cnt, fixed, sms) * (cnt > 150 ? 95 : 80) / 100;
   for (int s = 1; s <= cnt && (s <= fixed || s * slot_bytes <= (size_t(64) << 20)); ++s) {
+    const int per = (cnt + s - 1) / s;
+    if ((cnt + per - 1) / per != s) continue;   // a slot would be empty
     const long cost = slot_cost(tiles, cnt, s, sms);
-    if (best_cost < 0 || cost < best_cost) {
+    if (cost < best_cost) {
       best_cost = cost;
       best = s;
     }
   }
   return best;
-}
-
-// The same where the fixed count may fill the SMs well: it stays unless the
-// other costs 5% less by that measure (many waves even out by themselves, and
-// more, shorter blocks then balance tiles of unequal work better).  Measured:
-// FP64 matrix 11^3 21.8 -> 15.6 ms (8 -> 7 slots, 152 -> 133 blocks on 148 SMs),
-// BF16 matrix 15x13x11 11.7 -> 10.6 (28 -> 26).
-int better_slots(int tiles, int cnt, int fixed, int sms, size_t slot_bytes) {
-  cnt = std::max(1, cnt);
-  fixed = std::min(fixed, cnt);
-  const int s = fill_slots(tiles, cnt, fixed, sms, slot_bytes);
-  return 20 * slot_cost(tiles, cnt, s, sms) < 19 * slot_cost(tiles, cnt, fixed, sms) ? s : fixed;
 }
 
 bool find_plan(const PlanKey& k, BuilderPlan* out) {
@@ -1600,7 +1612,7 @@ int run_matrix_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
   auto chunk_slots = [&](int cnt) {
     return tiles_pair * std::min(fixed_slots, cnt) <= ctx->num_sms
                ? std::min(fixed_slots, cnt)
-               : better_slots(tiles_pair, cnt, fixed_slots, ctx->num_sms, slot_bytes);
+               : fill_slots(tiles_pair, cnt, fixed_slots, ctx->num_sms, slot_bytes);
   };
   const int rest = (q2e - q2b) % std::max(1, chunk);
   const int slots = std::max(chunk_slots(chunk), rest ? chunk_slots(rest) : 1);

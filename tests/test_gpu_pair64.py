@@ -112,8 +112,10 @@ def test_matrix_modes_with_degenerate_points(ctx, diamond, smearing):
     bands.close()
 
 
-@pytest.mark.parametrize("mesh", [(2, 1, 1), (3, 3, 3), (7, 5, 4)])
-def test_coarse_meshes_fill_the_chip(ctx, diamond, mesh):
+# slots of 148 SMs: a q2 each where that is one wave or less, two (split) and three (FP64) q2 at
+# 7x5x4, whose tiles are 2 of 128 and 3 of 64 q1
+@pytest.mark.parametrize("mesh,slots64,slots16", [((2, 1, 1), 2, 2), ((3, 3, 3), 27, 27), ((7, 5, 4), 47, 70)])
+def test_coarse_meshes_fill_the_chip(ctx, diamond, mesh, slots64, slots16):
     """A q2 range too short to be tuned takes as many slots as fill the SMs; the split path's
     linewidths keep its 1e-5 bar against FP64, whose own slots sum in another order (1e-12)."""
     from phoebe_b200.core import Interaction3Ph, PhScatteringMatrix
@@ -121,16 +123,31 @@ def test_coarse_meshes_fill_the_chip(ctx, diamond, mesh):
     bands = _bands(ctx, cr, mesh)
     T = np.array([C.kelvin_to_ry(t) for t in (100.0, 300.0)])
     out = {}
-    for precision in ("fp64", "split_fp16"):
+    for precision, slots in (("fp64", slots64), ("split_fp16", slots16)):
         v3 = Interaction3Ph(ctx, cr, diamond["fc3"], precision=precision)
         sm = PhScatteringMatrix(v3, bands, T, "adaptive")
         out[precision] = sm.setup()
-        assert 1 <= sm.stats.plan_slots <= bands.nq
+        assert sm.stats.plan_slots == slots
         half = sm.setup(0, bands.nq // 2, finalize=False) + sm.setup(bands.nq // 2, bands.nq, finalize=False)
         whole = sm.setup(finalize=False)
         np.testing.assert_allclose(half, whole, rtol=1e-12 if precision == "fp64" else 1e-6,
                                    atol=1e-12 * np.abs(whole).max())
         v3.close()
-    if np.abs(out["fp64"]).max() > 0:
+    if bands.nq > 2:
         _close(out["split_fp16"], out["fp64"], 1e-5)
+    bands.close()
+
+
+@pytest.mark.parametrize("mesh,q2,slots", [((17, 17, 17), 32, 7), ((20, 20, 20), 24, 7), ((20, 20, 20), 32, 7),
+                                           ((24, 24, 24), 8, 7)])
+def test_short_slices_keep_blocks_for_several_waves(ctx, diamond, mesh, q2, slots):
+    """A slice of a few q2 of a fine mesh: one wave of long blocks waits for its slowest tile
+    (39 to 108 tiles of the split kernel), so the slots stay at the untuned plan's 7."""
+    from phoebe_b200.core import Interaction3Ph, PhScatteringMatrix
+    bands = _bands(ctx, diamond["crystal"], mesh)
+    v3 = Interaction3Ph(ctx, diamond["crystal"], diamond["fc3"], precision="split_fp16")
+    sm = PhScatteringMatrix(v3, bands, [C.kelvin_to_ry(300.0)])
+    sm.setup(0, q2, finalize=False)
+    assert sm.stats.plan_slots == slots
+    v3.close()
     bands.close()
