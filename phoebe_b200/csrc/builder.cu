@@ -1606,14 +1606,8 @@ int run_matrix_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
   // slots of a full chunk and of the remainder; the partial sums hold the larger count
   const int tiles_pair = (nq + (split ? 127 : pair64::tile_q1(nr3) - 1)) / (split ? 128 : pair64::tile_q1(nr3));
   const size_t slot_bytes = sizeof(double) * nq * NB * nT;
-  // (a grid within one wave stays as it is: the order of the few atomic sums of a
-  // matrix element then does not depend on which blocks run side by side)
   const int fixed_slots = split ? (full ? 28 : 7) : 8;
-  auto chunk_slots = [&](int cnt) {
-    return tiles_pair * std::min(fixed_slots, cnt) <= ctx->num_sms
-               ? std::min(fixed_slots, cnt)
-               : fill_slots(tiles_pair, cnt, fixed_slots, ctx->num_sms, slot_bytes);
-  };
+  auto chunk_slots = [&](int cnt) { return fill_slots(tiles_pair, cnt, fixed_slots, ctx->num_sms, slot_bytes); };
   const int rest = (q2e - q2b) % std::max(1, chunk);
   const int slots = std::max(chunk_slots(chunk), rest ? chunk_slots(rest) : 1);
   const size_t nb3 = (size_t)NB * NB * NB;

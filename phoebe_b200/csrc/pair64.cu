@@ -43,6 +43,10 @@
 //
 // Degenerate blocks of b1 and b3 are averaged in registers; those of b2 enter
 // through the rates: with S the block average, sum_b2 (S W) F = sum_b2 W (S F).
+// The members' shares of an element (q1 b1, q2 b2) are summed by the warp (in
+// local memory, only at a q2 with degenerate bands) before they go to the
+// matrix: an element receives one "+" and one "-" addition onto zero, which
+// commute, so it does not vary between runs either.
 #include <algorithm>
 #include <cstdint>
 
@@ -256,6 +260,32 @@ __global__ void __launch_bounds__(32 * kWarpsMax, 1) pair64_kernel(Args P, int w
 #pragma unroll
     for (int b = 0; b < kNb; ++b)
       if (!(E3[b] < phxc::phEnergyCutoff)) ok3 |= 0x1041u << b;
+    // (q1 b1o + i, q2 b) of the matrix
+    auto add_matrix = [&](int b, int i, int c, double vp, double vm) {
+      const size_t rw = (size_t)q1 * kNb + b1o + i;
+      double *dp, *dm, sgn;
+      if (P.mat_full) {
+        dp = P.matP + (size_t)(iq2 * kNb + b) * P.ld + rw;
+        dm = P.matP + (size_t)(iq2m * kNb + b) * P.ld + rw;
+        sgn = -2.0;
+      } else {
+        const size_t o = c * P.mat_tstride + (size_t)(j * kNb + b) * P.ld + rw;
+        dp = P.matP + o;
+        dm = P.matM + o;
+        sgn = 2.0;
+      }
+      // acc takes half of a rate, the matrix all of it
+      if (vp != 0.0) atomicAdd(dp, 2.0 * vp);
+      if (vm != 0.0) atomicAdd(dm, sgn * vm);
+    };
+    double msum[MAT ? kNb : 1][2][3][kMaxT];
+    if (MAT && s2 != kNoBlocks)
+#pragma unroll 1
+      for (int b = 0; b < kNb; ++b)
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int c = 0; c < kMaxT; ++c) msum[b][0][i][c] = msum[b][1][i][c] = 0.0;
 
 #pragma unroll 1
     for (int p = 0; p < 3; ++p) {
@@ -503,25 +533,29 @@ __global__ void __launch_bounds__(32 * kWarpsMax, 1) pair64_kernel(Args P, int w
 #pragma unroll
             for (int c = 0; c < kMaxT; ++c)
               if (c < nT) {
-                const size_t rw = (size_t)q1 * kNb + b1o + i;
-                double *dp, *dm, sgn;
-                if (P.mat_full) {
-                  dp = P.matP + (size_t)(iq2 * kNb + mb) * P.ld + rw;
-                  dm = P.matP + (size_t)(iq2m * kNb + mb) * P.ld + rw;
-                  sgn = -2.0;
+                if (s2 == kNoBlocks) {
+                  add_matrix(mb, i, c, sp[i][c], sm[i][c]);
                 } else {
-                  const size_t o = c * P.mat_tstride + (size_t)(j * kNb + mb) * P.ld + rw;
-                  dp = P.matP + o;
-                  dm = P.matM + o;
-                  sgn = 2.0;
+                  msum[mb][0][i][c] += sp[i][c];
+                  msum[mb][1][i][c] += sm[i][c];
                 }
-                // acc takes half of a rate, the matrix all of it
-                if (sp[i][c] != 0.0) atomicAdd(dp, 2.0 * sp[i][c]);
-                if (sm[i][c] != 0.0) atomicAdd(dm, sgn * sm[i][c]);
               }
       }
       __syncwarp();   // X may be written again
     }
+    if (MAT && s2 != kNoBlocks)
+#pragma unroll 1
+      for (int b = 0; b < kNb; ++b)
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int c = 0; c < kMaxT; ++c)
+            if (c < nT) {
+              // this thread's b2 and the other half's: one lane adds "+", the other "-"
+              const double vp = msum[b][0][i][c] + __shfl_xor_sync(0xffffffffu, msum[b][0][i][c], 2);
+              const double vm = msum[b][1][i][c] + __shfl_xor_sync(0xffffffffu, msum[b][1][i][c], 2);
+              add_matrix(b, i, c, b2l ? 0.0 : vp, b2l ? vm : 0.0);
+            }
   }
   // the two b2 halves of a row's sums, then this block's slot
 #pragma unroll

@@ -112,6 +112,23 @@ def test_matrix_modes_with_degenerate_points(ctx, diamond, smearing):
     bands.close()
 
 
+@pytest.mark.parametrize("mesh", [(4, 4, 4), (9, 9, 9), (11, 10, 12)])
+def test_stored_matrix_is_the_same_every_time(ctx, diamond, mesh):
+    """One "+" and one "-" addition onto zero for each element, whatever the order of the blocks (one
+    wave of them and several), also where the bands of q2 are degenerate."""
+    from phoebe_b200.core import Interaction3Ph, PhScatteringMatrix
+    bands = _bands(ctx, diamond["crystal"], mesh)
+    v3 = Interaction3Ph(ctx, diamond["crystal"], diamond["fc3"])
+    sm = PhScatteringMatrix(v3, bands, [C.kelvin_to_ry(300.0)], "gaussian", 0.5 / C.ryToTHz, in_memory=True)
+    diag, rows = sm.setup(), sm.getMatrixRows(0, sm.num_states)
+    for _ in range(8):
+        np.testing.assert_array_equal(sm.setup(), diag)
+        np.testing.assert_array_equal(sm.getMatrixRows(0, sm.num_states), rows)
+    sm.close()
+    v3.close()
+    bands.close()
+
+
 # slots of 148 SMs: a q2 each where that is one wave or less, two (split) and three (FP64) q2 at
 # 7x5x4, whose tiles are 2 of 128 and 3 of 64 q1
 @pytest.mark.parametrize("mesh,slots64,slots16", [((2, 1, 1), 2, 2), ((3, 3, 3), 27, 27), ((7, 5, 4), 47, 70)])
