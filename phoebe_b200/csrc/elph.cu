@@ -6,8 +6,8 @@
 //     g4 = sum_nu g3 ev3[nu][nu2], g = sum_w2 conj(U2[w2][b2]) g4, |g|^2.
 //   * ElScatteringMatrix::builder, linewidth mode (el_scattering.cpp:38-405) with
 //     symmetrizeCoupling (scattering.cpp:1209-1318) and degeneracyAveragingLinewidths
-//     (:1168-1207): one thread block per 4 final states k2 = k1 + q computes their
-//     couplings, symmetrises them and accumulates the rates of the k1 states.
+//     (:1168-1207): one thread block per 8 final states k2 = k1 + q, or per state,
+//     computes their couplings, symmetrises them and accumulates the rates of the k1 states.
 #include <algorithm>
 #include <cmath>
 #include <string>
@@ -42,6 +42,12 @@ constexpr int kMaxPh = 12;    // phonon branches
 constexpr int kPairThreads = 64;    // of a block that takes one final state at a time
 constexpr int kTileQ = 8;           // final states per FP64 tile (one row each of m8n8k4)
 constexpr int kTileThreads = 192;
+// Final states of a batch of k1 (active or not) up to which the split path gives each a block of its own
+// without listing them first: fewer tiles of 8 than that leave SMs idle, and the list is one more launch.
+// Split call of 6 branches, device us, a block a state / tiles: 64 states 98 / 108, 1024 99 / 109, 4096 107 / 112,
+// 8192 118 / 115; with every state active 104 / 121, 112 / 125, 141 / 156, 189 / 193.  Twice as many where
+// tiles have less than 2.5 times the states in flight: 3 branches, 8 bands (24 : 16), 8192 states 191 / 209.
+constexpr int kDirectStates = 4096;
 
 // D += A B on the FP64 tensor pipe: m8n8k4, lane l holds A(l/4, l%4), B(l%4, l/4)
 // and D(l/4, 2(l%4) + {0,1})
@@ -434,7 +440,7 @@ __device__ void pair_symmetrize(const double* E1, int nb1, int nph, const PairSm
 
 struct ElArgs {
   int nw, nph, nRp;
-  const double2* cached;   // batch of k1: cached + blockIdx.y * cper
+  const double2* cached;   // batch of k1: cached + j * cper for its row j
   size_t cper;
   const double* Rp;
   const double* degP;
@@ -447,8 +453,8 @@ struct ElArgs {
   const int* hi;
   const double* Eq;        // (nq,nph)
   const double2* evq;      // (nq,nph,nph)
-  int ik1s[kB1], i1s[kB1]; // per blockIdx.y: k1 mesh index and its row in the output
-  long long g3offs[kB1];   // per blockIdx.y: offset of its g3 columns in g3in
+  int ik1s[kB1], i1s[kB1]; // per row: k1 mesh index and its row in the output
+  long long g3offs[kB1];   // per row: offset of its g3 columns in g3in
   int nk1;
   int nT;
   double temps[pairc::kMaxT];
@@ -461,7 +467,8 @@ struct ElArgs {
   const float2* g3in;      // precomputed g3 of this k1, g3in[x * g3ld + q], or null
   int g3ld;
   // the final states with active bands of row j of the batch: (q, k2, nb2) at
-  // list[j * nq ..], count[j] of them; w1: the largest nb1 of the batch's k1
+  // list[j * nq ..], count[j] of them; no list: every state of every row is looked
+  // at.  w1: the largest nb1 of the call's k1
   int4* list;
   int* count;
   int nb, w1;
@@ -506,31 +513,33 @@ __device__ __forceinline__ double el_delta_tab(double ginv, double e, double2 w)
   return exp(-x * x) * w.y * (1.0 / (phxc::sqrtPi * phxc::erf2));
 }
 
-// Final states k2 = k1 + q of the batch's k1 (blockIdx.y) that have active
-// bands, in no fixed order.  With a window around the Fermi level most have none
+// The final state k2 = k1 + q of row jb of the batch, as (q, k2, nb2): nb2 active bands, maybe none.
+__device__ __forceinline__ int4 final_state(const ElArgs& A, int jb, int iq) {
+  const int ik1 = A.ik1s[jb];
+  const int x1 = ik1 % A.kmesh[0], y1 = (ik1 / A.kmesh[0]) % A.kmesh[1], z1 = ik1 / (A.kmesh[0] * A.kmesh[1]);
+  const int f0 = A.kmesh[0] / A.qmesh[0], f1 = A.kmesh[1] / A.qmesh[1], f2 = A.kmesh[2] / A.qmesh[2];
+  const int qx = iq % A.qmesh[0], qy = (iq / A.qmesh[0]) % A.qmesh[1], qz = iq / (A.qmesh[0] * A.qmesh[1]);
+  const int ik2 = (x1 + f0 * qx) % A.kmesh[0] +
+                  A.kmesh[0] * ((y1 + f1 * qy) % A.kmesh[1] + A.kmesh[1] * ((z1 + f2 * qz) % A.kmesh[2]));
+  return make_int4(iq, ik2, A.hi[ik2] - A.lo[ik2], 0);
+}
+
+// The final states of the batch's k1 (blockIdx.y) that have active bands, in no
+// fixed order within a k1.  With a window around the Fermi level most have none
 // (84% of them with +-0.3 eV on 8 bands of 2 eV hoppings), and a block of the
 // pair kernel for each of those cost as much as the pairs: 255 -> 128 us per 16 k1.
 __global__ void __launch_bounds__(256) el_list_kernel(ElArgs A) {
   const int iq = blockIdx.x * blockDim.x + threadIdx.x, jb = blockIdx.y;
-  const int ik1 = A.ik1s[jb];
-  int nb2 = 0, ik2 = 0;
-  if (iq < A.qmesh[0] * A.qmesh[1] * A.qmesh[2]) {
-    const int x1 = ik1 % A.kmesh[0], y1 = (ik1 / A.kmesh[0]) % A.kmesh[1], z1 = ik1 / (A.kmesh[0] * A.kmesh[1]);
-    const int f0 = A.kmesh[0] / A.qmesh[0], f1 = A.kmesh[1] / A.qmesh[1], f2 = A.kmesh[2] / A.qmesh[2];
-    const int qx = iq % A.qmesh[0], qy = (iq / A.qmesh[0]) % A.qmesh[1], qz = iq / (A.qmesh[0] * A.qmesh[1]);
-    ik2 = (x1 + f0 * qx) % A.kmesh[0] +
-          A.kmesh[0] * ((y1 + f1 * qy) % A.kmesh[1] + A.kmesh[1] * ((z1 + f2 * qz) % A.kmesh[2]));
-    nb2 = A.hi[ik2] - A.lo[ik2];
-  }
-  const unsigned have = __ballot_sync(0xffffffffu, nb2 > 0);
+  int4 fs = make_int4(0, 0, 0, 0);
+  if (iq < A.qmesh[0] * A.qmesh[1] * A.qmesh[2]) fs = final_state(A, jb, iq);
+  const unsigned have = __ballot_sync(0xffffffffu, fs.z > 0);
   if (!have) return;
   const int lane = threadIdx.x & 31;
   int first = 0;
   if (lane == 0) first = atomicAdd(A.count + jb, __popc(have));
   first = __shfl_sync(0xffffffffu, first, 0);
-  if (nb2 > 0)
-    A.list[(size_t)jb * (A.qmesh[0] * A.qmesh[1] * A.qmesh[2]) + first + __popc(have & ((1u << lane) - 1u))] =
-        make_int4(iq, ik2, nb2, 0);
+  if (fs.z > 0)
+    A.list[(size_t)jb * (A.qmesh[0] * A.qmesh[1] * A.qmesh[2]) + first + __popc(have & ((1u << lane) - 1u))] = fs;
 }
 
 // G3IN: g3 from the tensor-core GEMM (split path); SM: the smearing.  Each
@@ -543,27 +552,37 @@ __global__ void __launch_bounds__(256) el_list_kernel(ElArgs A) {
 // registers are held to 6 blocks per SM in the split path (4 blocks: 101 us), and
 // to 3 in FP64, whose phases fill shared memory.
 template <int QT, bool G3IN, int SM>
-__global__ void __launch_bounds__(QT == 1 ? kPairThreads : kTileThreads, QT == 1 ? 1 : G3IN ? 6 : 3)
+__global__ void __launch_bounds__(QT == 1 ? kPairThreads : kTileThreads, QT == 1 ? (G3IN ? 16 : 1) : G3IN ? 6 : 3)
     el_pair_kernel(ElArgs A) {
   extern __shared__ __align__(16) char sraw[];
   const int nw = A.nw, nph = A.nph, nRp = A.nRp;
   // no phase buffer when g3 comes from the tensor-core GEMM
   const PairSmem s = pair_carve<QT>(sraw, G3IN ? 0 : nRp, nph, nw, QT == 1 ? kMaxW : A.w1);
   const int tid = threadIdx.x, NT = blockDim.x, W1 = QT == 1 ? kMaxW : A.w1;
-  // lane j: tiles of the rows up to and with j of the batch
+  // lane j: items (QT states, listed) of the rows up to and with j of the batch
   static_assert(kB1 <= 31, "a lane for each k1 of a batch");
-  const int lane = tid & 31, own = lane < A.nb ? (A.count[lane] + QT - 1) / QT : 0;
+  const int nq = A.qmesh[0] * A.qmesh[1] * A.qmesh[2], lane = tid & 31;
+  const bool listed = QT > 1 || A.list;
+  const int own = listed && lane < A.nb ? (A.count[lane] + QT - 1) / QT : 0;
   int incl = own;
   for (int o = 1; o < 32; o <<= 1) {
     const int v = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += v;
   }
-  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  const int total = listed ? __shfl_sync(0xffffffffu, incl, 31) : nq * A.nb;   // or every state of every row
   for (int item = blockIdx.x; item < total; item += gridDim.x) {
-    const int jb = __popc(__ballot_sync(0xffffffffu, incl <= item));
-    const int first = (item - __shfl_sync(0xffffffffu, incl - own, jb)) * QT;
-    const int left = A.count[jb] - first;   // states of the row from here on
-    const int4* states = A.list + (size_t)jb * (A.qmesh[0] * A.qmesh[1] * A.qmesh[2]) + first;
+    int jb, left = 1;                   // row; its states from this item's first on
+    int4 fs = make_int4(0, 0, 0, 0);    // of thread q: state q of the item
+    if (listed) {
+      jb = __popc(__ballot_sync(0xffffffffu, incl <= item));
+      const int first = (item - __shfl_sync(0xffffffffu, incl - own, jb)) * QT;
+      left = A.count[jb] - first;
+      if (tid < QT && tid < left) fs = A.list[(size_t)jb * nq + first + tid];
+    } else {
+      jb = item / nq;
+      fs = final_state(A, jb, item - jb * nq);
+      if (fs.z <= 0) continue;
+    }
     const int ik1 = A.ik1s[jb], i1 = A.i1s[jb], lo1 = A.lo[ik1], nb1 = A.hi[ik1] - lo1;
     const double2* cached = A.cached + (size_t)jb * A.cper;
     const float2* g3in = G3IN ? A.g3in + A.g3offs[jb] : nullptr;
@@ -571,7 +590,6 @@ __global__ void __launch_bounds__(QT == 1 ? kPairThreads : kTileThreads, QT == 1
     __syncthreads();   // the previous final state's sums have been read
     for (int i = tid; i < kMaxW * pairc::kMaxT; i += NT) s.acc[i] = 0.0;
     if (tid < QT) {
-      const int4 fs = tid < left ? states[tid] : make_int4(0, 0, 0, 0);
       s.info[4 * tid] = tid < left;
       s.info[4 * tid + 1] = fs.z;
       s.info[4 * tid + 2] = fs.y;
@@ -1113,26 +1131,49 @@ extern "C" int phx_el_linewidths(phx_elph* e, phx_bands* el, phx_bands* ph, cons
     ++launches;
   }
   size_t soff[13];
-  size_t smem = pair_smem_layout<1>(split ? 0 : e->nRp, nph, nw, kMaxW, soff);
-  PHX_ARG(ctx, smem <= 227 * 1024, "phx_el_linewidths: too many phonon Bravais vectors");
+  const size_t state_smem = pair_smem_layout<1>(split ? 0 : e->nRp, nph, nw, kMaxW, soff);
+  PHX_ARG(ctx, state_smem <= 227 * 1024, "phx_el_linewidths: too many phonon Bravais vectors");
   A.w1 = std::max(1, *std::max_element(nb1all.begin(), nb1all.end()));
-  // tiles of 8 final states where the buffers of a tile fit (343 Rp, 6 branches, 8
-  // orbitals and all 8 bands active: 122 KB); past that, as with 12 branches and 8
-  // active bands, one state at a time
   const size_t tile_smem = pair_smem_layout<kTileQ>(split ? 0 : e->nRp, nph, nw, A.w1, soff);
-  const bool tiled = tile_smem <= 227 * 1024;
-  if (tiled) smem = tile_smem;
   constexpr int ad = PHX_SMEAR_ADAPTIVE, ga = PHX_SMEAR_GAUSSIAN;
   const bool adaptive = p->smearing == ad;
-  const auto pair_fn = split && tiled ? (adaptive ? el_pair_kernel<kTileQ, true, ad> : el_pair_kernel<kTileQ, true, ga>)
-                       : split ? (adaptive ? el_pair_kernel<1, true, ad> : el_pair_kernel<1, true, ga>)
-                       : tiled ? (adaptive ? el_pair_kernel<kTileQ, false, ad> : el_pair_kernel<kTileQ, false, ga>)
-                               : (adaptive ? el_pair_kernel<1, false, ad> : el_pair_kernel<1, false, ga>);
-  const int pair_threads = tiled ? kTileThreads : kPairThreads;
-  PHX_CUDA(ctx, cudaFuncSetAttribute(pair_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int resident = 1;   // pair blocks per SM
-  PHX_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, pair_fn, pair_threads, smem));
-  resident = std::max(1, resident);
+  struct PairPlan {
+    void (*fn)(ElArgs);
+    size_t smem;
+    int threads, resident;   // resident: blocks per SM
+  };
+  const PairPlan state_plan{split ? (adaptive ? el_pair_kernel<1, true, ad> : el_pair_kernel<1, true, ga>)
+                                  : (adaptive ? el_pair_kernel<1, false, ad> : el_pair_kernel<1, false, ga>),
+                            state_smem, kPairThreads, 0};
+  const PairPlan tile_plan{split ? (adaptive ? el_pair_kernel<kTileQ, true, ad> : el_pair_kernel<kTileQ, true, ga>)
+                                 : (adaptive ? el_pair_kernel<kTileQ, false, ad> : el_pair_kernel<kTileQ, false, ga>),
+                           tile_smem, kTileThreads, 0};
+  auto prepare = [&](PairPlan& k) {
+    cudaError_t ce = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
+    if (ce == cudaSuccess) ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k.resident, k.fn, k.threads, k.smem);
+    k.resident = std::max(1, k.resident);
+    return ce;
+  };
+  // Tiles of 8 final states where the buffers of a tile fit (12 branches and 8 active bands: they do not) and, in
+  // the split path, leave at least half as many states again per SM as blocks of one state: all stages of a
+  // tile wait for its barriers, so what counts is the states in flight.  20^3 q, 16 k1, 8 bands of 8 orbitals
+  // active, us: 6 branches (8 states against 13) tiles 5756, one state 2646; 5 active bands (16 : 13) 1650
+  // against 1531; 2 (32 : 13) 617 against 973.  In FP64 the Rp transform gains from the tile too: with one
+  // tile per SM (8 : 8) 5570 against 4579 with 27 Rp, 7785 against 10393 with 125.
+  PairPlan plan = state_plan;
+  const bool fits = tile_smem <= 227 * 1024;
+  // a batch of few final states: a block for each, no list
+  long long direct_states = split || !fits ? kDirectStates : 0;
+  auto direct = [&](int nb) { return (long long)ph->nq * nb <= direct_states; };
+  if (nact > 0 && direct((nact - 1) % kB1 + 1))   // the last batch, the smallest
+    PHX_CUDA(ctx, cudaFuncSetAttribute(plan.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
+  if (nact > 0 && !direct(std::min(nact, kB1))) {
+    PairPlan tile = tile_plan;
+    if (fits) PHX_CUDA(ctx, prepare(tile));
+    if (split || tile.resident < 2) PHX_CUDA(ctx, prepare(plan));
+    if (2 * kTileQ * tile.resident < 5 * plan.resident) direct_states *= 2;
+    if (fits && (split ? 2 * kTileQ * tile.resident >= 3 * plan.resident : tile.resident > 1 || e->nRp >= 64)) plan = tile;
+  }
   const int nq = ph->nq;
   const size_t per = N;
   long long pairs = 0;
@@ -1156,7 +1197,7 @@ extern "C" int phx_el_linewidths(phx_elph* e, phx_bands* el, phx_bands* ph, cons
                                     &g3ld, xoff.data()));
       launches += 2;
     }
-    // one launch for the batch: blockIdx.y = k1 of the batch
+    // the pair kernel of the batch's k1
     A.cached = dcached;
     A.cper = per;
     A.nb = nb;
@@ -1169,11 +1210,17 @@ extern "C" int phx_el_linewidths(phx_elph* e, phx_bands* el, phx_bands* ph, cons
       A.g3in = dg3;
       A.g3ld = g3ld;
     }
-    el_list_kernel<<<dim3((nq + 255) / 256, nb), 256, 0, st>>>(A);
-    const int grid = (int)std::min<long long>((long long)nq * nb, (long long)resident * ctx->num_sms);
-    pair_fn<<<grid, pair_threads, smem, st>>>(A);
-    ++launches;
-    ++launches;
+    if (direct(nb)) {
+      A.list = nullptr;
+      state_plan.fn<<<nq * nb, state_plan.threads, state_plan.smem, st>>>(A);
+      ++launches;
+    } else {
+      A.list = dlist;
+      el_list_kernel<<<dim3((nq + 255) / 256, nb), 256, 0, st>>>(A);
+      const int grid = (int)std::min<long long>((long long)nq * nb, (long long)plan.resident * ctx->num_sms);
+      plan.fn<<<grid, plan.threads, plan.smem, st>>>(A);
+      launches += 2;
+    }
     pairs += (long long)nq * nb;
     PHX_CUDA(ctx, cudaGetLastError());
   }

@@ -17,20 +17,8 @@ def _crystal(nat):
     return lattice.Crystal(p.direct_cell, p.positions[:nat], np.arange(nat), np.array(masses) * C.massAmuToRy)
 
 
-# nat (3 nat branches), nw, ncell of Re and Rp, k mesh, q mesh, bands in the window, smearing, k1.
-# 4 atoms with all 8 bands active are past the tile's shared memory; with 5 they are within.
-# 21 and 17 k1 leave a second batch of at most 8.
-@pytest.mark.parametrize("nat,nw,ce,cp,kmesh,qmesh,window,smearing,nk1", [
-    (1, 1, 1, 1, (3, 3, 3), (3, 3, 3), "all", "gaussian", 3),
-    (1, 5, 1, 2, (4, 2, 6), (2, 2, 3), "some", "adaptive", 21),
-    (2, 3, 2, 1, (5, 5, 3), (5, 5, 3), "all", "adaptive", 17),
-    (2, 8, 1, 0, (6, 4, 2), (3, 2, 2), "some", "gaussian", 16),
-    (4, 8, 1, 1, (4, 4, 2), (2, 2, 2), "some", "adaptive", 9),
-    (4, 8, 1, 1, (4, 4, 2), (2, 2, 2), "all", "adaptive", 9),
-    (4, 8, 0, 1, (4, 4, 2), (2, 2, 2), "all", "gaussian", 2),
-])
-@pytest.mark.parametrize("precision", ["fp64", "split_bf16"])
-def test_el_linewidths_tiles(ctx, nat, nw, ce, cp, kmesh, qmesh, window, smearing, nk1, precision):
+def _compare(ctx, nat, nw, ce, cp, kmesh, qmesh, window, smearing, nk1, precision):
+    """The linewidths of nk1 initial states against the oracle; returns the call's stats."""
     from phoebe_b200.core import ElectronH0Wannier, ElScatteringMatrix, InteractionElPhWan, PhononH0
     cr = _crystal(nat)
     Rh, degh, H = synth.wannier_hamiltonian(cr, nw, 1)
@@ -52,7 +40,8 @@ def test_el_linewidths_tiles(ctx, nat, nw, ce, cp, kmesh, qmesh, window, smearin
     sigma = 0.05
     gpu = InteractionElPhWan(ctx, Re, degE, Rp, degP, g)
     gpu.setPrecision(precision)
-    A = ElScatteringMatrix(gpu, el, ph, temps, mu, win, smearing, sigma).setup(k1)
+    sm = ElScatteringMatrix(gpu, el, ph, temps, mu, win, smearing, sigma)
+    A = sm.setup(k1)
     ref = oracle.InteractionElPhWan(Re, degE, Rp, degP, g)
     kc = lattice.Mesh(cr, kmesh).cartesian_coords()
     B = oracle.el_linewidths(ref, kmesh, qmesh, Ek, Uk, vk, lo, hi, Eq, evq, kc, cr.reciprocal_cell, k1, temps, mu,
@@ -66,3 +55,39 @@ def test_el_linewidths_tiles(ctx, nat, nw, ce, cp, kmesh, qmesh, window, smearin
     assert np.abs(A - B).max() < tol * np.abs(B).max()
     for h in (gpu, ph, h0, el, wan):
         h.close()
+    return sm.stats
+
+
+# nat (3 nat branches), nw, ncell of Re and Rp, k mesh, q mesh, bands in the window, smearing, k1.
+# 4 atoms with all 8 bands active are past the tile's shared memory; with 5 they are within.
+# 21 and 17 k1 leave a second batch of at most 8.
+@pytest.mark.parametrize("nat,nw,ce,cp,kmesh,qmesh,window,smearing,nk1", [
+    (1, 1, 1, 1, (3, 3, 3), (3, 3, 3), "all", "gaussian", 3),
+    (1, 5, 1, 2, (4, 2, 6), (2, 2, 3), "some", "adaptive", 21),
+    (2, 3, 2, 1, (5, 5, 3), (5, 5, 3), "all", "adaptive", 17),
+    (2, 8, 1, 0, (6, 4, 2), (3, 2, 2), "some", "gaussian", 16),
+    (4, 8, 1, 1, (4, 4, 2), (2, 2, 2), "some", "adaptive", 9),
+    (4, 8, 1, 1, (4, 4, 2), (2, 2, 2), "all", "adaptive", 9),
+    (4, 8, 0, 1, (4, 4, 2), (2, 2, 2), "all", "gaussian", 2),
+])
+@pytest.mark.parametrize("precision", ["fp64", "split_bf16"])
+def test_el_linewidths_tiles(ctx, nat, nw, ce, cp, kmesh, qmesh, window, smearing, nk1, precision):
+    _compare(ctx, nat, nw, ce, cp, kmesh, qmesh, window, smearing, nk1, precision)
+
+
+# Split: up to 4096 final states of a batch a block for each, none listed; past that tiles of 8, or past 8192
+# blocks of one state where the buffers of a tile leave few of them on an SM (6 branches, 8 bands) or do not
+# fit (12).  FP64: tiles, but blocks of one state with a tile per SM and few Rp, or where tiles do not fit.
+# The launches tell: one more per batch with a list.
+@pytest.mark.parametrize("nat,nw,ce,cp,kmesh,qmesh,window,smearing,nk1,precision,launches", [
+    (1, 5, 1, 1, (8, 8, 8), (8, 8, 8), "some", "adaptive", 8, "split_bf16", 11),
+    (1, 5, 1, 1, (8, 8, 8), (8, 8, 8), "some", "adaptive", 9, "split_bf16", 12),
+    (2, 8, 0, 1, (9, 8, 8), (9, 8, 8), "all", "gaussian", 14, "split_bf16", 11),
+    (2, 8, 1, 1, (9, 8, 8), (9, 8, 8), "all", "gaussian", 17, "split_bf16", 19),
+    (4, 8, 0, 0, (9, 8, 8), (9, 8, 8), "all", "adaptive", 15, "split_bf16", 12),
+    (2, 8, 0, 1, (9, 8, 8), (9, 8, 8), "all", "adaptive", 8, "fp64", 8),
+    (4, 8, 0, 1, (4, 4, 2), (2, 2, 2), "all", "gaussian", 3, "fp64", 7),
+])
+def test_el_linewidths_routes(ctx, nat, nw, ce, cp, kmesh, qmesh, window, smearing, nk1, precision, launches):
+    stats = _compare(ctx, nat, nw, ce, cp, kmesh, qmesh, window, smearing, nk1, precision)
+    assert stats.kernel_launches == launches
