@@ -2029,7 +2029,17 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
   const int nchunks = (q2e - q2b + chunk - 1) / chunk;
   const size_t sz_dp = align_up(sizeof(double2) * nr3 * nb3 * chunk);
   const size_t sz_img = split ? align_up(wide::split_img_bytes(nb, Kp) * chunk) : 0;
-  const size_t sz_lw = align_up(sizeof(double) * (size_t)nq * nb * nT);
+  // slots of the isotope kernel (slot 0 takes the pair kernel's sums too): one block per 32 q1 and slot, four per SM
+  // as in the shared-memory builder, at most 64 MB of sums.  One slot left most SMs idle: 15 branches 4^3
+  // FP64 1.95 ms a call, 0.90 without isotopes.
+  const size_t lw_slot = (size_t)nq * nb * nT;
+  const int iso_tiles = (nq + kTile - 1) / kTile;
+  const int iso_slots =
+      !p->isotope_coupling ? 1
+                           : (int)std::max<size_t>(1, std::min<size_t>({(size_t)(q2e - q2b),
+                                                                        (size_t)(4 * ctx->num_sms + iso_tiles - 1) / iso_tiles,
+                                                                        (size_t(64) << 20) / (sizeof(double) * lw_slot)}));
+  const size_t sz_lw = align_up(sizeof(double) * lw_slot * iso_slots);
   const size_t sz_bose = align_up(sizeof(double) * (size_t)nT * nq * nb);
   const size_t sz_T = align_up(sizeof(double) * 8);
   const size_t sz_win = align_up(sizeof(double) * 2 * nq);
@@ -2171,7 +2181,7 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
   for (int c0 = q2b; c0 < q2e; c0 += chunk) pairs += (long long)nq * std::min(chunk, q2e - c0);
   auto work = [&](phx_builder_graph& g) -> int {
     int launches = 0;
-    PHX_CUDA(ctx, cudaMemsetAsync(lw, 0, sizeof(double) * (size_t)nq * nb * nT, st));
+    PHX_CUDA(ctx, cudaMemsetAsync(lw, 0, sizeof(double) * lw_slot * iso_slots, st));
     PHX_CUDA(ctx, cudaMemsetAsync(counters, 0, sizeof(unsigned) * (nchunks + 1), st));
     bose_kernel<<<std::min(1024, (nq * nb * nT + 255) / 256), 256, 0, st>>>(nq, nb, nT, b->d_E, temps, bose);
     ++launches;
@@ -2206,12 +2216,12 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
     }
     PHX_CUDA(ctx, phx_record_event(g.vertex_end, st));
     if (giso) {
-      IsoArgs I{A.m, v->nat, giso, q2b, q2e - q2b, q2e - q2b, lw};
-      isotope_kernel<<<dim3((nq + kTile - 1) / kTile, 1), kTile * nb, iso_smem(nb), st>>>(I);
+      IsoArgs I{A.m, v->nat, giso, q2b, q2e - q2b, (q2e - q2b + iso_slots - 1) / iso_slots, lw};
+      isotope_kernel<<<dim3(iso_tiles, iso_slots), kTile * nb, iso_smem(nb), st>>>(I);
       ++launches;
       PHX_CUDA(ctx, cudaGetLastError());
     }
-    finalize_kernel<<<(nq + kFinWarps - 1) / kFinWarps, 32 * kFinWarps, 0, st>>>(nq, nb, nT, 1, lw, b->d_E, p->finalize, b->d_vg, temps,
+    finalize_kernel<<<(nq + kFinWarps - 1) / kFinWarps, 32 * kFinWarps, 0, st>>>(nq, nb, nT, iso_slots, lw, b->d_E, p->finalize, b->d_vg, temps,
                                                       p->boundary_length, Aout_d);
     ++launches;
     PHX_CUDA(ctx, cudaGetLastError());

@@ -104,3 +104,35 @@ def test_fp64_matches_oracle(ctx, nat, mesh, nr3, window, smearing):
     assert big.any()
     assert (np.abs(A - ref)[big] / np.abs(ref)[big]).max() < 1e-10
     bands.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "split_fp16"])
+@pytest.mark.parametrize("nat,mesh,window", [(1, (3, 2, 2), False), (3, (4, 4, 2), True), (3, (5, 7, 1), False),
+                                             (5, (3, 3, 2), True)])
+def test_isotopes_in_slots_match_oracle(ctx, monkeypatch, nat, mesh, window, precision):
+    """Isotope rates of the many-branch builder, a slot per q2 on these meshes: one tile of 32 q1,
+    exactly one, and a remainder; slices of q2 add up.  FP64 at 1e-10, split at its 1e-5."""
+    from phoebe_b200.core import Interaction3Ph, PhScatteringMatrix, isotope_coupling
+    monkeypatch.setenv("PHX_WIDE", "1")
+    cr = _cell(nat)
+    E, U, V, bands = _bands(ctx, cr, mesh, np.random.default_rng(nat))
+    fc3 = _fc3(cr, 5)
+    fc3.D3 *= 1e-3   # rates of the size of the isotopes'
+    T = np.array([C.kelvin_to_ry(t) for t in (100.0, 300.0)])
+    win = synth.q2_window(E, mesh) if window else None
+    g = isotope_coupling(cr, np.linspace(1e-2, 3e-2, nat))
+    v3 = Interaction3Ph(ctx, cr, fc3, precision=precision)
+    sm = PhScatteringMatrix(v3, bands, T, "adaptive", 0.0, window=win, isotope_coupling=g)
+    A = sm.setup(finalize=False)
+    parts = sm.setup(0, 2, finalize=False) + sm.setup(2, bands.nq, finalize=False)
+    np.testing.assert_allclose(parts, A, rtol=1e-12 if precision == "fp64" else 1e-5, atol=1e-8 * np.abs(A).max())
+    v3.close()
+    q = lattice.Mesh(cr, mesh).cartesian_coords()
+    ref, without = (oracle.Interaction3Ph(cr, fc3).linewidths(mesh, E, U, V, q, cr.reciprocal_cell, T, "adaptive", 0.0,
+                                                              window=win, finalize=False, isotope_coupling=i)
+                    for i in (g, None))
+    assert (ref > 1.01 * without).any()
+    tol = 1e-10 if precision == "fp64" else 1e-5
+    big = np.abs(ref) > 1e-8 * np.abs(ref).max()
+    assert (np.abs(A - ref)[big] / np.abs(ref)[big]).max() < tol
+    bands.close()
