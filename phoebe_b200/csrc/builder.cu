@@ -2288,6 +2288,25 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
   return rc;
 }
 
+// Is the shared-memory builder faster than the FP64 tensor-pipe kernel for this
+// many q1 and q2 (both fit)?  The tensor-pipe kernel takes a q2 and 16 q1 as one
+// item, with nb padded to 16, and a block walks all its R3 and b2 in turn; the other
+// one has blocks of 4 q1 and, of few q2, one each.  So the first needs an
+// item for every SM, four where padding takes most of it, and with many branches
+// only to beat one wave of the other's blocks.  ms a call, shared memory / tensor pipe:
+//   3 branches, 57 R3: 8^3 1 q2 0.09 / 0.15, 6^3 16 q2 0.20 / 0.22, 5^3 all 0.56 / 0.53, 6^3 all 1.62 / 1.33
+//   9:  8^3 1 q2 0.17 / 0.32, 3^3 all 0.31 / 0.36, 4^3 all 0.78 / 0.59
+//   15: 8^3 1 q2 0.37 / 0.62, 4^3 8 q2 0.60 / 0.70, 3^3 all 0.91 / 0.77, 4^3 all 2.68 / 1.36
+bool shared_memory_builder_is_faster(const phx_v3* v, int nq, int q2) {
+  if (generic_smem_bytes(v->nb, v->nr3, 1) > 227 * 1024 ||
+      sizeof(double2) * ((size_t)v->nr2 + 2 * (size_t)v->nb * v->nb) > 227 * 1024)
+    return false;   // it refuses these
+  const long long sms = v->ctx->num_sms, items = (long long)((nq + 15) / 16) * q2;
+  if (v->nb < 9) return items < 4 * sms;
+  if (v->nb < 12) return items < sms;
+  return (long long)((nq + 3) / 4) * q2 <= sms;
+}
+
 }  // namespace
 
 extern "C" int phx_ph_linewidths_d(phx_v3* v, phx_bands* b, const phx_lw_params* p,
@@ -2314,9 +2333,10 @@ extern "C" int phx_ph_linewidths_d(phx_v3* v, phx_bands* b, const phx_lw_params*
   if (v->nb == 6 && !p->window_energy) return run_builder<6>(v, b, p, Aout_d, stats);
   // the split precisions, cells beyond 16 branches and FP64 where the tensor-pipe
   // kernel fits run on the many-branch builder; FP64 with more R3 vectors (over
-  // 332 at 15 branches) or R2 vectors than that on the shared-memory one
+  // 332 at 15 branches) or R2 vectors than that, or with little work, on the shared-memory one
   if (v->precision != PHX_PREC_FP64 || v->nb > kMaxNbGeneric ||
-      (wide::q1_fp64_mma(v->nb, v->nr3) && wide::fold_smem(v->nb, v->nr2) <= 227 * 1024))
+      (wide::q1_fp64_mma(v->nb, v->nr3) && wide::fold_smem(v->nb, v->nr2) <= 227 * 1024 &&
+       !shared_memory_builder_is_faster(v, b->nq, p->q2_end - p->q2_begin)))
     return run_builder_wide(v, b, p, Aout_d, stats);
   return run_builder_generic(v, b, p, Aout_d, stats);
 }

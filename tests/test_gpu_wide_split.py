@@ -84,11 +84,7 @@ def test_split_matches_fp64(ctx, nat, mesh, nr3, window, smearing):
     bands.close()
 
 
-@pytest.mark.parametrize("smearing", ["adaptive", "gaussian"])
-@pytest.mark.parametrize("nat,mesh,nr3,window", [(1, (3, 2, 2), 1, False), (2, (5, 4, 1), 4, True), (3, (3, 3, 2), 27, False),
-                                                 (5, (3, 2, 2), 67, True), (5, (3, 2, 1), 130, False),
-                                                 (5, (3, 1, 1), 343, True)])
-def test_fp64_matches_oracle(ctx, nat, mesh, nr3, window, smearing):
+def _fp64_against_oracle(ctx, nat, mesh, nr3, window, smearing):
     from phoebe_b200.core import Interaction3Ph, PhScatteringMatrix
     cr = _cell(nat)
     E, U, V, bands = _bands(ctx, cr, mesh, np.random.default_rng(nat))
@@ -103,6 +99,48 @@ def test_fp64_matches_oracle(ctx, nat, mesh, nr3, window, smearing):
     big = np.abs(ref) > 1e-8 * np.abs(ref).max()
     assert big.any()
     assert (np.abs(A - ref)[big] / np.abs(ref)[big]).max() < 1e-10
+    bands.close()
+
+
+@pytest.mark.parametrize("smearing", ["adaptive", "gaussian"])
+@pytest.mark.parametrize("nat,mesh,nr3,window", [(1, (3, 2, 2), 1, False), (2, (5, 4, 1), 4, True), (3, (3, 3, 2), 27, False),
+                                                 (5, (3, 2, 2), 67, True), (5, (3, 2, 1), 130, False),
+                                                 (5, (3, 1, 1), 343, True)])
+def test_fp64_matches_oracle(ctx, nat, mesh, nr3, window, smearing):
+    _fp64_against_oracle(ctx, nat, mesh, nr3, window, smearing)
+
+
+@pytest.mark.parametrize("smearing", ["adaptive", "gaussian"])
+@pytest.mark.parametrize("nat,mesh,nr3,window", [(1, (3, 2, 2), 1, False), (2, (5, 4, 1), 4, True), (3, (3, 3, 2), 27, False),
+                                                 (5, (3, 2, 2), 67, True), (5, (3, 2, 1), 130, False),
+                                                 (5, (3, 1, 1), 343, True)])
+def test_fp64_tensor_pipe_matches_oracle(ctx, monkeypatch, nat, mesh, nr3, window, smearing):
+    """The same on the tensor-pipe kernel, which problems as small as these reach only when forced."""
+    monkeypatch.setenv("PHX_WIDE", "1")
+    _fp64_against_oracle(ctx, nat, mesh, nr3, window, smearing)
+
+
+# items of 16 q1 and a q2, blocks of 4 q1 and a q2, on 148 SMs
+@pytest.mark.parametrize("nat,mesh,q2,tensor_pipe", [
+    (1, (8, 8, 2), 73, False), (1, (8, 8, 2), 74, True), (2, (8, 8, 2), 73, False), (2, (8, 8, 2), 74, True),
+    (3, (5, 5, 3), 29, False), (3, (5, 5, 3), 30, True), (4, (4, 4, 2), 18, False), (4, (4, 4, 2), 19, True),
+    (5, (3, 3, 1), 9, False), (5, (4, 4, 2), 18, False), (5, (4, 4, 2), 19, True)])
+def test_fp64_route_by_size(ctx, monkeypatch, nat, mesh, q2, tensor_pipe):
+    """Little work stays on the shared-memory builder (no pair events); both sides of the line agree with
+    the forced tensor-pipe kernel."""
+    from phoebe_b200.core import Interaction3Ph, PhScatteringMatrix
+    cr = _cell(nat)
+    E, _, _, bands = _bands(ctx, cr, mesh, np.random.default_rng(nat))
+    v3 = Interaction3Ph(ctx, cr, _fc3(cr, 9))
+    sm = PhScatteringMatrix(v3, bands, [C.kelvin_to_ry(300.0)], "adaptive", 0.0,
+                            window=synth.q2_window(E, mesh) if nat == 2 else None)
+    A = sm.setup(0, q2, finalize=False)
+    assert (sm.stats.pair_launches > 0) == tensor_pipe
+    monkeypatch.setenv("PHX_WIDE", "1")
+    B = sm.setup(0, q2, finalize=False)
+    assert np.abs(B).max() > 0
+    np.testing.assert_allclose(A, B, rtol=1e-10, atol=1e-14 * np.abs(B).max())
+    v3.close()
     bands.close()
 
 
