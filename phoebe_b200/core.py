@@ -247,19 +247,22 @@ class Interaction3Ph:
         nb = self.nb
 
         def pad(evs):
-            # full bands at every q1 (one stacked array of them above all) need no loop over q1
-            if isinstance(evs, (np.ndarray, list, tuple)) and len(evs) == nq1 and nq1 and np.shape(evs[0]) == (nb, nb):
-                try:
-                    whole = np.asarray(evs, dtype=np.complex128)
-                except ValueError:
-                    whole = None
-                if whole is not None and whole.shape == (nq1, nb, nb):
-                    return whole, np.full(nq1, nb)
+            # full bands at every q1: one stacked array of them as it is, a list of them in one copy
+            if isinstance(evs, np.ndarray) and evs.shape == (nq1, nb, nb):
+                return evs, np.full(nq1, nb)
+            full = (nb, nb)
+            evs = list(evs)
+            for e in evs:
+                if type(e) is not np.ndarray or e.shape != full:
+                    break
+            else:
+                if nq1 and len(evs) == nq1:
+                    return np.array(evs, dtype=np.complex128), np.full(nq1, nb)
+            evs = [np.asarray(e) for e in evs]
             out = np.zeros((nq1, nb, nb), dtype=np.complex128)
             for i, e in enumerate(evs):
-                e = np.asarray(e)
                 out[i, :, :e.shape[1]] = e
-            return out, np.array([np.asarray(e).shape[1] for e in evs])
+            return out, [e.shape[1] for e in evs]
 
         (e1, n1), (e3p, n3p), (e3m, n3m) = pad(ev1s), pad(ev3Pluss), pad(ev3Minss)
         ev2 = np.asarray(ev2)
@@ -277,7 +280,7 @@ class Interaction3Ph:
         check(_abi.load().phx_v3_couplings_sq(self.h, nq1, dptr(q1), dptr(E1), iptr(nb1s), dptr(E2),
                                               nb2, dptr(E3p), iptr(nb3p), dptr(E3m), iptr(nb3m),
                                               dptr(outP), dptr(outM)), self.ctx.h)
-        if nq1 and all(len(x) == nq1 and (x == x[0]).all() for x in (nb1s, nb3p, nb3m)):
+        if nq1 >= 8 and all(len(x) == nq1 and (x == x[0]).all() for x in (nb1s, nb3p, nb3m)):
             return (list(outP[:sizeP].reshape(nq1, nb1s[0], nb2, nb3p[0])),
                     list(outM[:sizeM].reshape(nq1, nb1s[0], nb2, nb3m[0])))
         cp, cm = [], []

@@ -102,6 +102,41 @@ def test_ragged_band_counts(ctx, diamond):
         np.testing.assert_allclose(cm[i], M0[i][:nb1[i], :nb2, :nb3m[i]], rtol=1e-11, atol=1e-25)
 
 
+@pytest.mark.parametrize("nq1", [1, 7, 8, 33])
+def test_eigenvector_containers(ctx, diamond, nq1):
+    """Stacked arrays, lists, tuples, nested lists, other types, orders and strides of full bands, and
+    lists in which one q1 has fewer: the same couplings, entry by entry."""
+    from phoebe_b200.core import Interaction3Ph
+    cr = diamond["crystal"]
+    v3 = Interaction3Ph(ctx, cr, diamond["fc3"])
+    rng = np.random.default_rng(nq1)
+    q1, q2 = rng.normal(size=(nq1, 3)), rng.normal(size=3)
+    U = [rng.normal(size=(nq1, 6, 6)) + 1j * rng.normal(size=(nq1, 6, 6)) for _ in range(3)]
+    U2 = rng.normal(size=(6, 6)) + 1j * rng.normal(size=(6, 6))
+    v3.cacheD3(q2)
+    cp, cm = v3.getCouplingsSquared(q1, q2, U[0], U2, U[1], U[2])
+    assert len(cp) == len(cm) == nq1 and cp[0].shape == (6, 6, 6)
+    for make in (list, tuple, lambda u: u.tolist(), np.asfortranarray, lambda u: [np.asfortranarray(e) for e in u],
+                 lambda u: np.repeat(u, 2, axis=0)[::2], lambda u: [e.tolist() for e in u]):
+        a, b = v3.getCouplingsSquared(q1, q2, make(U[0]), U2, make(U[1]), make(U[2]))
+        np.testing.assert_array_equal(np.stack(a), np.stack(cp))
+        np.testing.assert_array_equal(np.stack(b), np.stack(cm))
+    real = [u.real.copy() for u in U]
+    a, b = v3.getCouplingsSquared(q1, q2, real[0], U2, list(real[1]), real[2].astype(np.float32))
+    c, d = v3.getCouplingsSquared(q1, q2, *[(r + 0j) for r in real[:1]], U2, real[1] + 0j,
+                                  real[2].astype(np.float32).astype(np.complex128))
+    np.testing.assert_array_equal(np.stack(a), np.stack(c))
+    np.testing.assert_array_equal(np.stack(b), np.stack(d))
+    few = list(U[0])
+    few[-1] = few[-1][:, :4]
+    a, b = v3.getCouplingsSquared(q1, q2, few, U2, U[1], U[2])
+    assert a[-1].shape == (4, 6, 6)
+    for i in range(nq1):
+        np.testing.assert_array_equal(a[i], cp[i][:a[i].shape[0]])
+        np.testing.assert_array_equal(b[i], cm[i][:b[i].shape[0]])
+    v3.close()
+
+
 def test_couplings_before_cache_is_an_error(ctx, diamond):
     from phoebe_b200 import _abi
     from phoebe_b200.core import Interaction3Ph
