@@ -192,6 +192,7 @@ __global__ void __launch_bounds__(kThreads, 1) el_gemm_kernel(GemmArgs P) {
                        kBBytes, &full[s]);
         }
       }
+      tc::ring_drain(full, it, kStages, P.status, 1);
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
@@ -412,6 +413,8 @@ __global__ void __launch_bounds__(kThreads, 1) el_g1_gemm_kernel(G1Args P) {
                        &full[s]);
         }
       }
+      tc::ring_drain(bfull, 1, 1, P.status, 1);
+      tc::ring_drain(full, it, kG1Stages, P.status, 1);
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------

@@ -103,6 +103,14 @@ __device__ __forceinline__ unsigned count_done(unsigned* p) {
   return old;
 }
 
+// A wait of this warp gave up: its own copies and the fills issued so far have landed when it
+// returns.  The last warp to give up has seen the last fill.
+__device__ __noinline__ void give_up(uint64_t* full, int* status) {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  volatile unsigned* fills = reinterpret_cast<unsigned*>(full + kStages) + kStages;
+  for (int s = 0; s < kStages; ++s) tc::ring_drain(full + s, fills[s], 1, status, 2);
+}
+
 // Forward-scan degenerate blocks of six energies, 4 bits per band: its block's first band.
 constexpr unsigned kNoBlocks = 0x543210u;
 __device__ __forceinline__ unsigned block_starts(const double* e) {
@@ -153,7 +161,7 @@ __global__ void __launch_bounds__(32 * kWarpsMax, 1) pair64_kernel(Args P, int w
   const MeshArgs& M = P.m;
   const int nks = ksteps(P.nr3), kc = stage_steps(nks), nkc = (nks + kc - 1) / kc;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);
-  unsigned* done = reinterpret_cast<unsigned*>(full + kStages);   // warps that have read a stage
+  unsigned* done = reinterpret_cast<unsigned*>(full + kStages);   // warps that have read a stage, then copies issued to it
   unsigned char* ring = smem + kBarBytes;
   const int stage_bytes = kc * kStepBytes;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -169,11 +177,12 @@ __global__ void __launch_bounds__(32 * kWarpsMax, 1) pair64_kernel(Args P, int w
                  reinterpret_cast<const unsigned char*>(P.img) +
                      (((size_t)jbeg * 9 + g) * nks + (size_t)k * kc) * kStepBytes,
                  bytes, full + s);
+    ++done[kStages + s];
   };
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       tc::mbar_init(full + s, 1);
-      done[s] = 0;
+      done[s] = done[kStages + s] = 0;
     }
     tc::fence_mbar_init();
     for (unsigned i = 0; i < min((unsigned)kStages, nstage); ++i) issue(i);
@@ -297,7 +306,10 @@ __global__ void __launch_bounds__(32 * kWarpsMax, 1) pair64_kernel(Args P, int w
         for (int a = 0; a < kNb; ++a) cr[a][0] = cr[a][1] = ci[a][0] = ci[a][1] = 0.0;
         for (int k = 0; k < nkc; ++k, ++it) {
           const unsigned s = it % kStages;
-          if (!__all_sync(0xffffffffu, tc::mbar_wait(full + s, (it / kStages) & 1, P.status, 2))) return;
+          if (!__all_sync(0xffffffffu, tc::mbar_wait(full + s, (it / kStages) & 1, P.status, 2))) {
+            give_up(full, P.status);
+            return;
+          }
           const double2* B = reinterpret_cast<const double2*>(ring + s * stage_bytes) + lane;
           const double2* A = ph + k * kc * 32 + lane;
           const int steps = min(kc, nks - k * kc);

@@ -725,6 +725,7 @@ __global__ void __launch_bounds__(kThreads, 1) pair_tc_kernel(TcArgs P) {
                        kStageBytes, &full[s]);
         }
       }
+      tc::ring_drain(full, it, kStages, P.status, 1);
     }
   } else if (warp == kEpiWarps + 1) {
     // ---------------- MMA issuer ----------------

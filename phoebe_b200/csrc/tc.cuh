@@ -105,6 +105,22 @@ __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gmem_src, u
       : "memory");
 }
 
+// The last copies of a ring have landed: fill k of `issued` (from 0) went to stage k % stages, whose
+// barrier completes phase k / stages with it.  Whoever issues copies calls this before the block ends,
+// also after a wait that gave up: none is left to write to shared memory that is no longer the block's.
+static __device__ __noinline__ void ring_drain(uint64_t* full, unsigned issued, unsigned stages, int* status, int code) {
+  for (unsigned k = issued > stages ? issued - stages : 0; k < issued; ++k) {
+    const unsigned long long t0 = globaltimer();
+    while (!mbar_try_wait(full + k % stages, (k / stages) & 1)) {
+      __nanosleep(64);
+      if (globaltimer() - t0 > kWaitNs) {
+        atomicOr(status, code | 0x40000000);
+        return;
+      }
+    }
+  }
+}
+
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }

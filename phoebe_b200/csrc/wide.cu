@@ -980,6 +980,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) wide_split_kernel(WideArgs P
           break;
         }
       }
+      tc::ring_drain(full, it, kAStages, P.status, 1 << 9);
     }
   } else if (warp == kSplitEpiWarps + 1) {
     // ---------------- MMA issuer ----------------

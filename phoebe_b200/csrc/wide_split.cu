@@ -207,6 +207,7 @@ __global__ void __launch_bounds__((NQ + 2) * 32, 1) wide_warp_kernel(WideArgs P,
     // ---------------- producer: work queue and A tiles ----------------
     if (lane == 0) {
       int st = 0;
+      unsigned issued = 0;
       uint32_t par = 1;   // parity of the next wait for an empty stage
       for (int n = 0;; ++n) {
         const int slot = n % kItems;
@@ -235,6 +236,7 @@ __global__ void __launch_bounds__((NQ + 2) * 32, 1) wide_warp_kernel(WideArgs P,
             const uint32_t bytes = min(group, nkc - g * group) * kStage;
             tc::mbar_arrive_expect_tx(&full[st], bytes);
             tc::bulk_g2s(As + st * stage_bytes, src, bytes, &full[st]);
+            ++issued;
             src += bytes;
             if (++st == stages) {
               st = 0;
@@ -246,6 +248,7 @@ __global__ void __launch_bounds__((NQ + 2) * 32, 1) wide_warp_kernel(WideArgs P,
           break;
         }
       }
+      tc::ring_drain(full, issued, stages, P.status, 1 << 9);
     }
   } else if (warp == NQ + 1) {
     // ---------------- MMA issuer ----------------
