@@ -228,7 +228,8 @@ struct PairArgs {
 
 // ---------------------------------------------------------------------------
 // Any nb up to kMaxNbGeneric, with an optional per-q1 window on q2, where the R3
-// vectors are too many for wide64.cu's phases in shared memory: one block per (q1, q2 slot), the R3 transform, the e1 and e3
+// vectors are too many for wide64.cu's phases in shared memory or the work too
+// little for its items: one block per (q1 tile, q2 slot), the R3 transform, the e1 and e3
 // contractions, |V|^2, the three symmetrisation passes and the rates of each
 // q2 run through shared memory (two nb^3 complex buffers).  Same algebra,
 // cutoffs and time-reversal pairing as pair64_kernel: the "+" vertex of
@@ -1061,7 +1062,7 @@ int run_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Aout_d,
   const int nq = b->nq, nT = p->num_temperatures, nr3 = v->nr3, nr2 = v->nr2;
   const int q2b = p->q2_begin, q2e = p->q2_end;
   const bool split = v->precision != PHX_PREC_FP64;
-  // (ahead of every size that is derived from it: past 1376 not one warp's phases fit)
+  // (ahead of every size that is derived from it: past 1380 not one warp's phases fit)
   PHX_ARG(ctx, split || nr3 <= pair64::kMaxR3, "phx_ph_linewidths: too many R3 vectors for the FP64 path");
   // candidate plans; the first is the default
   std::vector<BuilderPlan> cands;
@@ -1149,9 +1150,10 @@ int run_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Aout_d,
   P.partial = partial;
   P.status = ctx->d_status;
   if (!split) PHX_CUDA(ctx, pair64::set_attributes(nr3, false, p->smearing));
+  // (the split path's fold; FP64 keeps its limit)
   const size_t smem_fold = fold_tiled_smem(NB, nr2);
   PHX_ARG(ctx, smem_fold <= 227 * 1024, "phx_ph_linewidths: too many R2 vectors");
-  if (smem_fold > 48 * 1024)
+  if (split && smem_fold > 48 * 1024)
     PHX_CUDA(ctx, cudaFuncSetAttribute(fold_q2_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem_fold));
   if (split) PHX_TRY(phx_split_set_attributes(ctx, nr3, nT));
@@ -1681,9 +1683,9 @@ int run_matrix_builder(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
   P.mat_tstride = slab_elems;
   P.mat_full = full ? 1 : 0;
   if (!split) PHX_CUDA(ctx, pair64::set_attributes(nr3, true, p->smearing));
-  const size_t smem_fold = fold_tiled_smem(NB, nr2);
+  const size_t smem_fold = fold_tiled_smem(NB, nr2);   // (the split path's fold; FP64 keeps its limit)
   PHX_ARG(ctx, smem_fold <= 227 * 1024, "scattering matrix: too many R2 vectors");
-  if (smem_fold > 48 * 1024)
+  if (split && smem_fold > 48 * 1024)
     PHX_CUDA(ctx, cudaFuncSetAttribute(fold_q2_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem_fold));
   const int tiles = (nq + kTile - 1) / kTile;
@@ -2582,8 +2584,9 @@ int run_builder_static(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* 
     return PHX_ERR_ARG;
   }
   PHX_ARG(ctx, nr3 <= pair64::kMaxR3, "phx_ph_linewidths_static: too many R3 vectors");
-  const size_t smem_fold = sizeof(double2) * ((size_t)nr2 + 2 * NB * NB);
-  PHX_ARG(ctx, smem_fold <= 227 * 1024, "phx_ph_linewidths_static: too many R2 vectors");
+  // (the limit of an earlier fold's shared memory, kept; fold64_kernel streams R2)
+  PHX_ARG(ctx, sizeof(double2) * ((size_t)nr2 + 2 * NB * NB) <= 227 * 1024,
+          "phx_ph_linewidths_static: too many R2 vectors");
   // the operand image pads R3 to a multiple of four; kStaticPadBytes holds the padding of one q2
   const int chunk = (int)std::min<size_t>({(kStaticScratchBytes + kStaticPadBytes - fixed) / pair64::image_bytes(nr3),
                                            (size_t)512, (size_t)(q2e - q2b)});

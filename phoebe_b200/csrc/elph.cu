@@ -36,6 +36,8 @@ int phx_el_split_g1(phx_ctx* ctx, const uint8_t* gimg, int nRe, long long N, con
 
 namespace {
 
+using pairc::dmma;
+
 constexpr int kB1 = 16;       // k1 points per pass over the coupling tensor
 constexpr int kMaxW = 8;      // Wannier orbitals
 constexpr int kMaxPh = 12;    // phonon branches
@@ -48,14 +50,6 @@ constexpr int kTileThreads = 192;
 // 8192 118 / 115; with every state active 104 / 121, 112 / 125, 141 / 156, 189 / 193.  Twice as many where
 // tiles have less than 2.5 times the states in flight: 3 branches, 8 bands (24 : 16), 8192 states 191 / 209.
 constexpr int kDirectStates = 4096;
-
-// D += A B on the FP64 tensor pipe: m8n8k4, lane l holds A(l/4, l%4), B(l%4, l/4)
-// and D(l/4, 2(l%4) + {0,1})
-__device__ __forceinline__ void dmma(double* d, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
 
 // g1[b][e] = sum_Re ph[b][Re] g[Re][e] for the nb k1 of the batch (e over
 // nRp*nph*nw*nw): a product of the 8 MT phases of each Re with g, read once per

@@ -69,7 +69,7 @@ constexpr int kXStride = 73;           // complex per q1 of X
 constexpr int kSigBytes = 1536;        // widths [8 q1][2 b2][6 b3][+-]
 constexpr int kXBytes = 8 * kXStride * 16;
 static_assert(18 * 32 * 8 + kSigBytes <= kXBytes, "W and the widths take the place of X");
-constexpr int kWarpFixed = 2 * 8 * kEvStride * 16 + kXBytes + 64;
+constexpr int kWarpFixed = 2 * 8 * kEvStride * 16 + kXBytes;
 constexpr int kBarBytes = 128;
 constexpr int kSmemMax = 227 * 1024;
 
@@ -85,12 +85,6 @@ int warps_for(int nks) {
 }
 size_t smem_bytes(int nks, int warps) {
   return kBarBytes + (size_t)kStages * stage_steps(nks) * kStepBytes + (size_t)warps * warp_bytes(nks);
-}
-
-__device__ __forceinline__ void dmma(double* c, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
 }
 
 __device__ __forceinline__ void cp16(void* dst, const void* src) {
@@ -135,20 +129,7 @@ __device__ __forceinline__ int block_size(unsigned s, int b) {
   return n;
 }
 
-__device__ __forceinline__ bool state_ok(double e) { return e >= phxc::phExcludeCutoff && e >= phxc::phEnergyCutoff; }
-
-// s = sum_i (qT_i . dv)^2 of the adaptive width sqrt(s / 6), floored like
-// floor_sigma; 0 only for a zero velocity difference.
-__device__ __forceinline__ double width_sq(const double* qT, double v0, double v1, double v2) {
-  double s = 0.0;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const double d = qT[3 * i] * v0 + qT[3 * i + 1] * v1 + qT[3 * i + 2] * v2;
-    s += d * d;
-  }
-  return s;
-}
-// A bound on |e| above which delta(e) is zero, for the queue: the exact test
+// A bound on |e| above which delta(e) is zero, for the marking: the exact test
 // is the evaluation's.  FP32 square root, widened beyond its error.
 __device__ __forceinline__ double width_limit(double s) {
   constexpr float kFloor = (float)(2.0 * phxc::adaptiveCutoff * 1.00001);
@@ -197,7 +178,6 @@ __global__ void __launch_bounds__(32 * kWarpsMax, 1) pair64_kernel(Args P, int w
   double2* X = reinterpret_cast<double2*>(xw);                       // [8][row (b2l, b1)][c]
   double* w18 = reinterpret_cast<double*>(xw);                       // [18][lane] W, after X
   double2* sig = reinterpret_cast<double2*>(xw + kXBytes - kSigBytes);   // [8][2][6] squared widths of + and -
-  int* q3s = reinterpret_cast<int*>(xw + kXBytes);                   // [8]
 
   const int row = lane >> 2, l = lane & 3;     // q1 of the warp; column / quarter of the rows
   const int nq = M.nq, nT = M.nT, n0 = M.n0, n1 = M.n1, n2 = M.n2;
@@ -247,7 +227,6 @@ __global__ void __launch_bounds__(32 * kWarpsMax, 1) pair64_kernel(Args P, int w
     const int iq2 = P.q2_first + j;
     const int iq2m = mesh_neg(iq2, n0, n1, n2);
     const int iq3 = mesh_add(q1, iq2, n0, n1, n2);
-    if (l == 0) q3s[row] = iq3;
     for (int t = lane; t < 8 * kNbb; t += 32) {
       const int q = t / kNbb, e = t % kNbb;
       const int q3 = __shfl_sync(0xffffffffu, iq3, q * 4);

@@ -34,15 +34,20 @@ __device__ __forceinline__ int mesh_neg(int i, int n0, int n1, int n2) {
   return ((n2 - iz) % n2) * n0 * n1 + ((n1 - iy) % n1) * n0 + (n0 - ix) % n0;
 }
 
-// AdaptiveGaussianDeltaFunction sigma (delta_function.cpp:71-83) before the floor.
-__device__ __forceinline__ double adaptive_sigma(const double* qT, double v0, double v1, double v2) {
+// s = sum_i (qT_i . dv)^2 of the adaptive width sqrt(s / 6); 0 for equal velocities
+__device__ __forceinline__ double width_sq(const double* qT, double v0, double v1, double v2) {
   double s = 0.0;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const double d = qT[3 * i] * v0 + qT[3 * i + 1] * v1 + qT[3 * i + 2] * v2;
     s += d * d;
   }
-  return sqrt(s / 6.0);
+  return s;
+}
+
+// AdaptiveGaussianDeltaFunction sigma (delta_function.cpp:71-83) before the floor.
+__device__ __forceinline__ double adaptive_sigma(const double* qT, double v0, double v1, double v2) {
+  return sqrt(width_sq(qT, v0, v1, v2) / 6.0);
 }
 
 __device__ __forceinline__ double floor_sigma(double s) {
@@ -64,27 +69,15 @@ __device__ __forceinline__ double delta_fn(int smearing, double sigma, double e,
   return exp(-x * x) / phxc::sqrtPi / sigma / phxc::erf2;
 }
 
-// Forward-scan degeneracy blocks (scattering.cpp:1218-1230): gs[b] = first
-// band of b's block, gn[b] = its size.
-template <int NB>
-__device__ __forceinline__ void deg_blocks(const double* e, int* gs, int* gn) {
-  int start = 0;
-#pragma unroll
-  for (int b = 0; b < NB; ++b) {
-    if (b > start) {
-      // b continues the block iff |e[start] - e[b]| < thr and all between did
-      if (!(fabs(e[start] - e[b]) < phxc::degThreshold)) start = b;
-    }
-    gs[b] = start;
-  }
-#pragma unroll
-  for (int b = 0; b < NB; ++b) {
-    int n = 0;
-#pragma unroll
-    for (int k = 0; k < NB; ++k) n += (gs[k] == gs[b]);
-    gn[b] = n;
-  }
-}
+// does a state of energy e take part at all
+__device__ __forceinline__ bool state_ok(double e) { return e >= phxc::phExcludeCutoff && e >= phxc::phEnergyCutoff; }
 
+// D += A B on the FP64 tensor pipe: m8n8k4, lane l holds A(l/4, l%4), B(l%4, l/4)
+// and D(l/4, 2(l%4) + {0,1})
+__device__ __forceinline__ void dmma(double* d, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
 
 }  // namespace pairc

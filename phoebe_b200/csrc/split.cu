@@ -36,6 +36,7 @@
 #include <cuda_fp16.h>
 #include <vector>
 
+#include "half_split.cuh"
 #include "pair_common.cuh"
 #include "tc.cuh"
 
@@ -110,30 +111,6 @@ struct EdgeEvent {
   int iq2;
   uint2 entry;       // the queue entry (|V|^2 / n1, meta)
 };
-
-// Power-of-2 scale of the B operand for FP16 hi/lo: max |Dp| * scale in [0.5, 1]
-__device__ __forceinline__ float fp16_scale(unsigned maxbits) {
-  const float m = __uint_as_float(maxbits);
-  if (!(m > 0.f)) return 1.f;
-  int e;
-  frexpf(m, &e);
-  return ldexpf(1.f, -e);
-}
-
-// hi/lo split of v into two 16-bit values of the operand format
-__device__ __forceinline__ void split16(double v, bool fp16, uint16_t* hi, uint16_t* lo) {
-  if (fp16) {
-    const __half h = __double2half(v);
-    const __half l = __double2half(v - (double)__half2float(h));
-    *hi = __half_as_ushort(h);
-    *lo = __half_as_ushort(l);
-  } else {
-    const __nv_bfloat16 h = __double2bfloat16(v);
-    const __nv_bfloat16 l = __double2bfloat16(v - (double)__bfloat162float(h));
-    *hi = __bfloat16_as_ushort(h);
-    *lo = __bfloat16_as_ushort(l);
-  }
-}
 
 // ---------------------------------------------------------------------------
 // degenerate blocks of 6 sorted energies, packed as 3-bit block starts
@@ -231,7 +208,7 @@ __global__ void pack_records_kernel(MeshArgs M, uint4* __restrict__ rec) {
 __global__ void convert_b_kernel(const double2* __restrict__ Dp, int nr3, int Kp, int q2_count,
                                  uint8_t* __restrict__ Bimg, int fp16, const unsigned* __restrict__ dmax) {
   const int nkc = Kp / kKC;
-  const double sc = fp16 ? (double)fp16_scale(*dmax) : 1.0;
+  const double sc = fp16 ? (double)halves::fp16_scale(*dmax) : 1.0;
   const int j = blockIdx.x;
   const int h = blockIdx.y / nkc, kc = blockIdx.y % nkc;
   if (j >= q2_count) return;
@@ -251,7 +228,7 @@ __global__ void convert_b_kernel(const double2* __restrict__ Dp, int nr3, int Kp
       v = (ri == 0 ? (part == 0 ? B.x : -B.y) : (part == 0 ? B.y : B.x)) * sc;
     }
     uint16_t hi, lo;
-    split16(v, fp16 != 0, &hi, &lo);
+    halves::split16(v, fp16 != 0, &hi, &lo);
     const uint32_t off = tc::core_offset(n, kk, kKC, 2);
     *reinterpret_cast<uint16_t*>(img + off) = hi;
     *reinterpret_cast<uint16_t*>(img + kPartBytes + off) = lo;
@@ -679,7 +656,7 @@ __global__ void __launch_bounds__(kThreads, 1) pair_tc_kernel(TcArgs P) {
       v = k < P.nr3 ? cs : sn;
     }
     uint16_t hi, lo;
-    split16(v, P.fp16 != 0, &hi, &lo);
+    halves::split16(v, P.fp16 != 0, &hi, &lo);
     const uint32_t off = tc::core_offset(mm, k, Kp, 2);
     *reinterpret_cast<uint16_t*>(S.A + off) = hi;
     *reinterpret_cast<uint16_t*>(S.A + S.aPart + off) = lo;
@@ -779,7 +756,7 @@ __global__ void __launch_bounds__(kThreads, 1) pair_tc_kernel(TcArgs P) {
     // FP16 operands: |V|^2 carries the square of the B scale, undone here (power of 4)
     float pre = P.edge_only ? 0.f : (float)(phxc::pi * 0.25 * 0.5) * (float)M.norm;
     if (P.fp16) {
-      const float sc = fp16_scale(*P.dmax);
+      const float sc = halves::fp16_scale(*P.dmax);
       pre *= 1.f / (sc * sc);
     }
     const unsigned gp1 = P.rec[(size_t)q1c * kRecChunks + kChGp].x;
@@ -803,7 +780,7 @@ __global__ void __launch_bounds__(kThreads, 1) pair_tc_kernel(TcArgs P) {
     int qn = 0;  // queued live triplets (warp-uniform)
     const unsigned lanemask_lt = (1u << lane) - 1u;
     const uint32_t lane_base = (uint32_t)(qd * 32) << 16;
-    // fold the quarter's accumulators of b1 = k, k+3 (this lane's row) into FP64
+    // fold the quarter's accumulators of b1 = k, k + 4 (this lane's row) into FP64
     auto flush = [&]() {
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
@@ -1149,7 +1126,7 @@ __device__ __forceinline__ void edge_correction(const TcArgs& P, int q1, int iq2
   const MeshArgs& M = P.m;
   float pre = (float)(phxc::pi * 0.25 * 0.5) * (float)M.norm;
   if (P.fp16) {
-    const float sc = fp16_scale(*P.dmax);
+    const float sc = halves::fp16_scale(*P.dmax);
     pre *= 1.f / (sc * sc);
   }
   constexpr float kNorm = (float)(1.0 / (phxc::sqrtPi * phxc::erf2));

@@ -19,20 +19,6 @@ namespace warprates {
 
 using namespace pairc;
 
-__device__ __forceinline__ bool state_ok(double e) { return e >= phxc::phExcludeCutoff && e >= phxc::phEnergyCutoff; }
-
-// s = sum_i (qT_i . dv)^2 of the adaptive width sqrt(s / 6); 0 for equal velocities
-__device__ __forceinline__ double width_sq(const double* qT, const double* a, const double* b) {
-  const double v0 = a[0] - b[0], v1 = a[1] - b[1], v2 = a[2] - b[2];
-  double s = 0.0;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const double d = qT[3 * i] * v0 + qT[3 * i + 1] * v1 + qT[3 * i + 2] * v2;
-    s += d * d;
-  }
-  return s;
-}
-
 // W averaged over `count` degenerate blocks (first band f, size z) of the index with stride `step`, a lane
 // per value of the other index (stride `line`)
 template <class R>
@@ -154,7 +140,8 @@ struct Vertex {
     __syncwarp();   // the previous table has been read
     for (int e = lane; e < 2 * nb; e += 32) {
       if (ADAPTIVE) {
-        const double s2 = width_sq(M.qT, M.vg + ((size_t)(e & 1 ? iq2m : iq2) * nb + m2) * 3, V3 + 3 * (e >> 1));
+        const double *a = M.vg + ((size_t)(e & 1 ? iq2m : iq2) * nb + m2) * 3, *b = V3 + 3 * (e >> 1);
+        const double s2 = width_sq(M.qT, a[0] - b[0], a[1] - b[1], a[2] - b[2]);
         sq[e] = s2;
         lim[e] = s2 == 0.0 ? tol
                            : fmaxf(__fsqrt_rn((float)s2) * (float)(2.0 * 0.4082482904638631 * 1.00001),

@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "cplx.cuh"
+#include "half_split.cuh"
 #include "pair_common.cuh"
 #include "phx_consts.h"
 #include "phx_internal.h"
@@ -843,41 +844,6 @@ __device__ inline SplitSmem carve_split(uint8_t* base, int nb, int Kp, int qp) {
   return s;
 }
 
-// Power-of-2 scale of the FP16 A operand: max |Dp| * scale in [0.5, 1]
-__device__ __forceinline__ float wide_fp16_scale(const unsigned* dmax) {
-  const float m = __uint_as_float(*dmax);
-  if (!(m > 0.f)) return 1.f;
-  int e;
-  frexpf(m, &e);
-  return ldexpf(1.f, -e);
-}
-__device__ __forceinline__ void wide_split16(double v, bool fp16, uint16_t* hi, uint16_t* lo) {
-  if (fp16) {
-    const __half h = __double2half(v);
-    const __half l = __double2half(v - (double)__half2float(h));
-    *hi = __half_as_ushort(h);
-    *lo = __half_as_ushort(l);
-  } else {
-    const __nv_bfloat16 h = __double2bfloat16(v);
-    const __nv_bfloat16 l = __double2bfloat16(v - (double)__bfloat162float(h));
-    *hi = __bfloat16_as_ushort(h);
-    *lo = __bfloat16_as_ushort(l);
-  }
-}
-
-// is any q1 of tile t paired with q2 or -q2 (the producer's item filter)
-__device__ bool tile_live(const WideArgs& P, int tile, int iq2, int iq2m) {
-  if (!P.win_energy && !P.skip) return true;
-  for (int i = 0; i < P.nq1; ++i) {
-    const int k = tile * P.nq1 + i;
-    if (k >= P.m.nq) break;
-    const int q1 = P.q1_order[k];
-    if (P.skip && P.skip[(size_t)(iq2 - P.skip_base) * P.m.nq + q1]) continue;
-    if (!P.win_energy || P.win_energy[iq2] <= P.win_cut[q1] || P.win_energy[iq2m] <= P.win_cut[q1]) return true;
-  }
-  return false;
-}
-
 // Epilogue-side bounded wait by thread 0, broadcast to the 8 warps: true if
 // the barrier completed and nobody aborted.
 __device__ bool epi_wait(uint64_t* bar, uint32_t parity, const SplitSmem& S, const WideArgs& P, int code, int tid) {
@@ -956,7 +922,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) wide_split_kernel(WideArgs P
           if (item >= total) break;
           const int j = item / P.ntiles, tl = item % P.ntiles;
           const int iq2 = P.q2_first + j;
-          if (tile_live(P, tl, iq2, mesh_neg(iq2, M.n0, M.n1, M.n2))) break;
+          if (wide::tile_live(P, P.nq1, tl, iq2, mesh_neg(iq2, M.n0, M.n1, M.n2))) break;
         }
         S.items[slot] = item < total ? (int)item : -1;
         tc::mbar_arrive(&ifull[slot]);
@@ -1038,7 +1004,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) wide_split_kernel(WideArgs P
     const int qd = warp & 3, grp = warp >> 2;   // TMEM lane quarter; group of M tiles drained
     const uint32_t bBytes = (uint32_t)kN * Kp * 2;
     const int qp = P.qp;
-    const double sc = P.fp16 ? (double)wide_fp16_scale(P.dmax) : 1.0;
+    const double sc = P.fp16 ? (double)halves::fp16_scale(*P.dmax) : 1.0;
     const double wscale = 1.0 / (sc * sc);
     const int segs = wide_rate_segments(kWideQ1, nb, nth);
     int s = 0;
@@ -1068,11 +1034,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) wide_split_kernel(WideArgs P
           im = k < nr3 ? sn : cs;    // column 2q + 1: Ti = sum Dr sin + Di cos
         }
         uint16_t h, l;
-        wide_split16(re, P.fp16 != 0, &h, &l);
+        halves::split16(re, P.fp16 != 0, &h, &l);
         uint32_t off = tc::core_offset(2 * q, k, Kp, 2);
         *reinterpret_cast<uint16_t*>(Bh + off) = h;
         *reinterpret_cast<uint16_t*>(Bh + bBytes + off) = l;
-        wide_split16(im, P.fp16 != 0, &h, &l);
+        halves::split16(im, P.fp16 != 0, &h, &l);
         off = tc::core_offset(2 * q + 1, k, Kp, 2);
         *reinterpret_cast<uint16_t*>(Bh + off) = h;
         *reinterpret_cast<uint16_t*>(Bh + bBytes + off) = l;
@@ -1127,7 +1093,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) wide_split_kernel(WideArgs P
 __global__ void convert_wide_kernel(int nb, int nr3, int Kp, int q2_count, const double2* __restrict__ Dp,
                                     uint8_t* __restrict__ img, int fp16, const unsigned* __restrict__ dmax) {
   const int nbb = nb * nb, nkc = Kp / kAKC, mt_n = split_nt(nb);
-  const float sc = fp16 ? wide_fp16_scale(dmax) : 1.f;
+  const float sc = fp16 ? halves::fp16_scale(*dmax) : 1.f;
   const size_t tiles = (size_t)q2_count * nb * mt_n * nkc;
   for (size_t u = (size_t)blockIdx.x * blockDim.x + threadIdx.x; u < tiles * 256; u += (size_t)gridDim.x * blockDim.x) {
     const size_t tile = u / 256;
@@ -1145,7 +1111,7 @@ __global__ void convert_wide_kernel(int nb, int nr3, int Kp, int q2_count, const
         const double2 d = Dp[(((size_t)j * nr3 + r3) * nb + a) * nbb + (size_t)b2 * nb + c];
         v = (k < nr3 ? d.x : d.y) * (double)sc;
       }
-      wide_split16(v, fp16 != 0, &hi[i], &lo[i]);
+      halves::split16(v, fp16 != 0, &hi[i], &lo[i]);
     }
     uint8_t* base = img + tile * kAStage;
     const uint32_t off = tc::core_offset(r, kh * 8, kAKC, 2);

@@ -35,6 +35,19 @@ struct Args {
   int rt, qp;                 // split kernel tile shape: register tile (2 or 4), q1 planes per contraction pass
 };
 
+// is any of the nq1 q1 of the tile paired with q2 or -q2 (the filter of the work queue)
+__device__ inline bool tile_live(const Args& P, int nq1, int tile, int iq2, int iq2m) {
+  if (!P.win_energy && !P.skip) return true;
+  for (int i = 0; i < nq1; ++i) {
+    const int k = tile * nq1 + i;
+    if (k >= P.m.nq) break;
+    const int q1 = P.q1_order[k];
+    if (P.skip && P.skip[(size_t)(iq2 - P.skip_base) * P.m.nq + q1]) continue;
+    if (!P.win_energy || P.win_energy[iq2] <= P.win_cut[q1] || P.win_energy[iq2m] <= P.win_cut[q1]) return true;
+  }
+  return false;
+}
+
 // FP64 kernel: q1 per item for this nb and nr3 (0: too large), and its shared memory
 int fp64_q1(int nb, int nr3);
 size_t fp64_smem(int nq1, int nb, int nr3);

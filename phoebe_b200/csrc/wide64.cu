@@ -61,25 +61,6 @@ Layout make_layout(int nb, int nr3) {
   return L;
 }
 
-__device__ __forceinline__ void dmma(double* c, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
-
-// is any q1 of the tile paired with q2 or -q2
-__device__ bool tile_live(const wide::Args& P, int tile, int iq2, int iq2m) {
-  if (!P.win_energy && !P.skip) return true;
-  for (int i = 0; i < kQ; ++i) {
-    const int k = tile * kQ + i;
-    if (k >= P.m.nq) break;
-    const int q1 = P.q1_order[k];
-    if (P.skip && P.skip[(size_t)(iq2 - P.skip_base) * P.m.nq + q1]) continue;
-    if (!P.win_energy || P.win_energy[iq2] <= P.win_cut[q1] || P.win_energy[iq2m] <= P.win_cut[q1]) return true;
-  }
-  return false;
-}
-
 template <bool ADAPTIVE>
 __global__ void __launch_bounds__(kThreads, 1) wide64_kernel(wide::Args P, Layout L) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -103,7 +84,7 @@ __global__ void __launch_bounds__(kThreads, 1) wide64_kernel(wide::Args P, Layou
         item = atomicAdd(P.counter, 1u);
         if (item >= total) break;
         const int iq2 = P.q2_first + (int)(item / P.ntiles);
-        if (tile_live(P, item % P.ntiles, iq2, mesh_neg(iq2, M.n0, M.n1, M.n2))) break;
+        if (wide::tile_live(P, kQ, item % P.ntiles, iq2, mesh_neg(iq2, M.n0, M.n1, M.n2))) break;
       }
       ctl[0] = item < total ? (int)item : -1;
     }

@@ -31,7 +31,7 @@
 // 36) and the marked ones evaluated in FP64 with the reference's own cut-off.
 //
 // Measured (24^3 windowed slice of 128 q2, nb = 15, nr3 = 67 / 12^3 slice of 32
-// q2, nb = 36, nr3 = 33): 248 -> 74 ms / 114 -> 62 ms a call.  By parts, each
+// q2, nb = 36, nr3 = 33): 248 -> 75 ms / 114 -> 63 ms a call.  By parts, each
 // left out of a copy: A stages and MMAs alone 36 / 17 ms (45 / 27 ms with one K
 // step per stage: the handshake of producer and MMA thread costs some 450
 // cycles), contractions to 60 / 53 ms, rates the rest.  Packed FMAs were slower
@@ -45,6 +45,7 @@
 #include <cuda_fp16.h>
 
 #include "cplx.cuh"
+#include "half_split.cuh"
 #include "pair_common.cuh"
 #include "phx_consts.h"
 #include "tc.cuh"
@@ -110,38 +111,6 @@ Layout make_layout(int nb, int Kp, int nq, bool es) {
   }
   L.total = 0;
   return L;
-}
-
-__device__ __forceinline__ float fp16_scale(const unsigned* dmax) {
-  const float m = __uint_as_float(*dmax);
-  if (!(m > 0.f)) return 1.f;
-  int e;
-  frexpf(m, &e);
-  return ldexpf(1.f, -e);
-}
-__device__ __forceinline__ void split16(double v, bool fp16, uint16_t* hi, uint16_t* lo) {
-  if (fp16) {
-    const __half h = __double2half(v);
-    *hi = __half_as_ushort(h);
-    *lo = __half_as_ushort(__double2half(v - (double)__half2float(h)));
-  } else {
-    const __nv_bfloat16 h = __double2bfloat16(v);
-    *hi = __bfloat16_as_ushort(h);
-    *lo = __bfloat16_as_ushort(__double2bfloat16(v - (double)__bfloat162float(h)));
-  }
-}
-
-// is any q1 of the tile paired with q2 or -q2
-__device__ bool tile_live(const WideArgs& P, int tile, int iq2, int iq2m) {
-  if (!P.win_energy && !P.skip) return true;
-  for (int i = 0; i < P.nq1; ++i) {
-    const int k = tile * P.nq1 + i;
-    if (k >= P.m.nq) break;
-    const int q1 = P.q1_order[k];
-    if (P.skip && P.skip[(size_t)(iq2 - P.skip_base) * P.m.nq + q1]) continue;
-    if (!P.win_energy || P.win_energy[iq2] <= P.win_cut[q1] || P.win_energy[iq2m] <= P.win_cut[q1]) return true;
-  }
-  return false;
 }
 
 template <int NQ, int TR, int TC, bool ES, bool ADAPTIVE>
@@ -220,7 +189,7 @@ __global__ void __launch_bounds__((NQ + 2) * 32, 1) wide_warp_kernel(WideArgs P,
           item = *abort_flag ? total : atomicAdd(P.counter, 1u);
           if (item >= total) break;
           const int iq2 = P.q2_first + (int)(item / P.ntiles);
-          if (tile_live(P, item % P.ntiles, iq2, mesh_neg(iq2, M.n0, M.n1, M.n2))) break;
+          if (wide::tile_live(P, P.nq1, item % P.ntiles, iq2, mesh_neg(iq2, M.n0, M.n1, M.n2))) break;
         }
         items[slot] = item < total ? (int)item : -1;
         tc::mbar_arrive(&ifull[slot]);
@@ -312,7 +281,7 @@ __global__ void __launch_bounds__((NQ + 2) * 32, 1) wide_warp_kernel(WideArgs P,
     const int qd = warp & 3, grp = warp >> 2;
     const int lr = lane >> 2, lc = lane & 3;
     const int nq = M.nq;
-    const double sc = P.fp16 ? (double)fp16_scale(P.dmax) : 1.0;
+    const double sc = P.fp16 ? (double)halves::fp16_scale(*P.dmax) : 1.0;
     warprates::Vertex<float, TR, TC, ADAPTIVE> v(M, smem + L.warp + (size_t)warp * L.warp_bytes, lane, 1.0 / (sc * sc));
     float2* e1s = reinterpret_cast<float2*>(smem + L.ev) + (size_t)warp * 2 * nbb;
     float2* e3s = e1s + nbb;
@@ -353,11 +322,11 @@ __global__ void __launch_bounds__((NQ + 2) * 32, 1) wide_warp_kernel(WideArgs P,
           im = k < nr3 ? sn : cs;    // column 2q + 1: Ti = sum Dr sin + Di cos
         }
         uint16_t h, l;
-        split16(re, P.fp16 != 0, &h, &l);
+        halves::split16(re, P.fp16 != 0, &h, &l);
         uint32_t off = tc::core_offset(2 * warp, k, Kp, 2);
         *reinterpret_cast<uint16_t*>(Bh + off) = h;
         *reinterpret_cast<uint16_t*>(Bh + bBytes + off) = l;
-        split16(im, P.fp16 != 0, &h, &l);
+        halves::split16(im, P.fp16 != 0, &h, &l);
         off = tc::core_offset(2 * warp + 1, k, Kp, 2);
         *reinterpret_cast<uint16_t*>(Bh + off) = h;
         *reinterpret_cast<uint16_t*>(Bh + bBytes + off) = l;

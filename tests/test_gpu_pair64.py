@@ -67,9 +67,9 @@ def test_linewidths_at_tile_edges(ctx, mesh, nr3, smearing, temps):
     bands.close()
 
 
-@pytest.mark.parametrize("nr3", [263, 1376, 1377, 1400])
+@pytest.mark.parametrize("nr3", [263, 1380, 1381, 1400])
 def test_too_many_r3_vectors_are_refused(ctx, nr3):
-    """Past 262 R3 vectors the path returns an error, also past 1376, where no warp's phases fit."""
+    """Past 262 R3 vectors the path returns an error, also past 1380, where no warp's phases fit."""
     from phoebe_b200.core import Interaction3Ph, PhScatteringMatrix
     cr = synth.diamond_crystal()
     bands = _bands(ctx, cr, (2, 2, 1))
