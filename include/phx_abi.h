@@ -196,10 +196,11 @@ typedef struct phx_lw_stats {
  * accumulation, degeneracy averaging (src/bte/ph_scattering.cpp:60-935;
  * src/bte/scattering.cpp:1168-1318).  A_out (nT, nq*nb) host, the reference's
  * internalDiagonal (linewidth * n(n+1)).  stats may be NULL.  nb = 6 without
- * a q2 window runs on the fused kernels (FP64 or split precision); FP64 up to
- * nb = 16 or with a window on the shared-memory kernel; the split precisions
- * otherwise, and FP64 beyond 16 branches, on the many-branch builder (nb <= 48,
- * tcgen05 R3 transform, persistent work queue, tile shape tuned per problem). */
+ * a q2 window runs on the fused kernels (FP64 or split precision); everything
+ * else on the many-branch builder (nb <= 48, persistent work queue; R3 transform
+ * by tcgen05 in the split precisions, on the FP64 tensor pipe up to nb = 16), but
+ * FP64 up to nb = 16 with little work, or with more R3 vectors than that takes,
+ * on the shared-memory kernel. */
 int phx_ph_linewidths(phx_v3* v3, phx_bands* bands, const phx_lw_params* params,
                       double* A_out, phx_lw_stats* stats);
 /* Same with a device output buffer (nT*nq*nb doubles). */

@@ -1,6 +1,6 @@
 """Tiles of the electron-phonon pair kernel: final states in eights per initial
-state, Rp and Re in fours, columns in eights and 32s, and the sizes past which
-one final state is taken at a time, against the oracle."""
+state, Rp and Re in fours, columns in eights and 32s, and the sizes where one
+final state is taken at a time, from a list or without one, against the oracle."""
 import numpy as np
 import pytest
 

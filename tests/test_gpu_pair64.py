@@ -2,7 +2,9 @@
 the oracle on identical band structures, at the edges of its tiles: meshes
 smaller than a warp's 8 q1 and than a block's tile, q1 counts that are no
 multiple of either, R3 counts around the K step of 4 and beyond one ring stage,
-and the largest R3 count the path takes (fewer warps per block).  1e-10 is the
+and the largest R3 count the path takes (fewer warps per block); larger ones are
+refused.  The stored matrix is the same in every build, and the slots of coarse
+meshes and of short slices are those that pay.  1e-10 is the
 bar of the other FP64 linewidth tests (sums of ~1e5 terms, each with a few
 rounding errors of 1e-16, and the cancellation of the R3 sum)."""
 import numpy as np

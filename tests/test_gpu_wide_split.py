@@ -3,8 +3,10 @@ classes of tile and of its lanes' tiles, against the FP64 builder on the same ba
 split paths' bar of 1e-5 on linewidths above 1e-8 of the largest.  Cells of 1 to 12 atoms (the
 twelve-atom cell's first atoms), q1 counts that are no multiple of an item, R3 counts of one K step
 and of several A stages, q2 windows, both smearings, and an R3 count that leaves no room for the
-kernel (the older one takes over).  The FP64 builder itself, whose kernel for up to 16 branches runs
-on the FP64 tensor pipe, against the oracle at the 1e-10 of the other FP64 linewidth tests."""
+kernel (the older one takes over).  The FP64 builders of up to 16 branches against the oracle at the
+1e-10 of the other FP64 linewidth tests: as routed, where problems as small as these run on the
+shared-memory builder, and forced onto the FP64 tensor pipe; the route between the two; isotope
+scattering in slots of q2."""
 import numpy as np
 import pytest
 
