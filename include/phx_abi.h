@@ -198,7 +198,7 @@ typedef struct phx_lw_stats {
  * internalDiagonal (linewidth * n(n+1)).  stats may be NULL.  nb = 6 without
  * a q2 window runs on the fused kernels (FP64 or split precision); everything
  * else on the many-branch builder (nb <= 48, persistent work queue; R3 transform
- * by tcgen05 in the split precisions, on the FP64 tensor pipe up to nb = 16), but
+ * by tcgen05 in the split precisions, on the FP64 tensor pipe from 6 to 16 branches), but
  * FP64 up to nb = 16 with little work, or with more R3 vectors than that takes,
  * on the shared-memory kernel. */
 int phx_ph_linewidths(phx_v3* v3, phx_bands* bands, const phx_lw_params* params,

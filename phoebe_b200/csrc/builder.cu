@@ -1989,6 +1989,18 @@ int wide_prepare_blocks(phx_v3* v) {
   return PHX_OK;
 }
 
+// q1 per item of the FP64 tensor-pipe kernel (wide64.cu) where it runs, else 0: it pads to 16
+// branches, so at 6 only the R3 transform of 50 and more R3 vectors pays for that, and below 6
+// not even that; wide.cu's FP64 kernel takes those.  ms a call with windows, tensor pipe / wide.cu:
+// 3 branches, 12^3 128 q2, 19 R3 2.67 / 2.05, 125 R3 5.64 / 4.88; 6 branches, 12^3 32 q2, 19 R3 1.52
+// / 1.37, 57 R3 2.13 / 2.04 (8^3 all q2 8.4 / 9.4), 125 R3 3.15 / 3.30; 9 branches, 12^3 32 q2, 19 R3
+// 2.23 / 2.50.
+int mma64_q1(int nb, int nr3) {
+  const int q1 = wide::q1_fp64_mma(nb, nr3);
+  const bool pays = nb > 6 || (nb == 6 && nr3 >= 50);
+  return pays || !wide::fp64_q1(nb, nr3) ? q1 : 0;
+}
+
 // Builder for cells with many branches (wide.cu), both precisions, with an
 // optional per-q1 q2 window: per chunk of q2 the sparse R2 fold, for the
 // split path the FP16/BF16 hi/lo image of the folded vertex, then one
@@ -2009,7 +2021,7 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
   // the kernel with one warp per q1 (wide_split.cu) wherever it fits: nb <= 36
   // and an R3 count that leaves room for its T; it has no shape to tune
   int warp_q1 = 0, warp_rows = 0;
-  const int mma_q1 = split ? 0 : wide::q1_fp64_mma(nb, nr3);
+  const int mma_q1 = split ? 0 : mma64_q1(nb, nr3);
   if (split) {
     PHX_ARG(ctx, wide::split_smem(nb, Kp, 2) > 0,
             "phx_ph_linewidths: too many branches or R3 vectors for the split path");
@@ -2026,8 +2038,9 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
   const size_t per_q2 = sizeof(double2) * nr3 * nb3 + (split ? wide::split_img_bytes(nb, Kp) : 0);
   // q2 per chunk: at most 2 GiB of folded vertex (and its image), at most 512 q2 (512 MiB up to 16 branches in
   // FP64, the bound of the shared-memory builder)
+  const bool few_branches = !split && nb <= kMaxNbGeneric;
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>({(size_t)512, (size_t)(q2e - q2b),
-                                                                (mma_q1 ? size_t(512) << 20 : size_t(2) << 30) / per_q2}));
+                                                                (few_branches ? size_t(512) << 20 : size_t(2) << 30) / per_q2}));
   const int nchunks = (q2e - q2b + chunk - 1) / chunk;
   const size_t sz_dp = align_up(sizeof(double2) * nr3 * nb3 * chunk);
   const size_t sz_img = split ? align_up(wide::split_img_bytes(nb, Kp) * chunk) : 0;
@@ -2290,13 +2303,14 @@ int run_builder_wide(phx_v3* v, phx_bands* b, const phx_lw_params* p, double* Ao
   return rc;
 }
 
-// Is the shared-memory builder faster than the FP64 tensor-pipe kernel for this
-// many q1 and q2 (both fit)?  The tensor-pipe kernel takes a q2 and 16 q1 as one
-// item, with nb padded to 16, and a block walks all its R3 and b2 in turn; the other
+// Is the shared-memory builder faster than the FP64 many-branch builder for this
+// many q1 and q2 (both fit)?  The latter takes a q2 and 16 q1 (8 with few branches) as one
+// item, and a block walks all its R3 and b2 in turn; the other
 // one has blocks of 4 q1 and, of few q2, one each.  So the first needs an
-// item for every SM, four where padding takes most of it, and with many branches
-// only to beat one wave of the other's blocks.  ms a call, shared memory / tensor pipe:
-//   3 branches, 57 R3: 8^3 1 q2 0.09 / 0.15, 6^3 16 q2 0.20 / 0.22, 5^3 all 0.56 / 0.53, 6^3 all 1.62 / 1.33
+// item of 16 q1 for every SM, two with few branches, and with many branches
+// only to beat one wave of the other's blocks.  ms a call, shared memory / many-branch, 57 R3:
+//   3 branches: 8^3 1 q2 0.09 / 0.14, 6^3 16 q2 0.20 / 0.20, 8^3 16 q2 0.36 / 0.30, 12^3 128 q2 6.3 / 4.4
+//   6, windows: 8^3 1 q2 0.12 / 0.24, 8^3 16 q2 0.55 / 0.48, 12^3 32 q2 2.6 / 2.0
 //   9:  8^3 1 q2 0.17 / 0.32, 3^3 all 0.31 / 0.36, 4^3 all 0.78 / 0.59
 //   15: 8^3 1 q2 0.37 / 0.62, 4^3 8 q2 0.60 / 0.70, 3^3 all 0.91 / 0.77, 4^3 all 2.68 / 1.36
 bool shared_memory_builder_is_faster(const phx_v3* v, int nq, int q2) {
@@ -2304,7 +2318,7 @@ bool shared_memory_builder_is_faster(const phx_v3* v, int nq, int q2) {
       sizeof(double2) * ((size_t)v->nr2 + 2 * (size_t)v->nb * v->nb) > 227 * 1024)
     return false;   // it refuses these
   const long long sms = v->ctx->num_sms, items = (long long)((nq + 15) / 16) * q2;
-  if (v->nb < 9) return items < 4 * sms;
+  if (v->nb < 9) return items < 2 * sms;
   if (v->nb < 12) return items < sms;
   return (long long)((nq + 3) / 4) * q2 <= sms;
 }
@@ -2334,7 +2348,7 @@ extern "C" int phx_ph_linewidths_d(phx_v3* v, phx_bands* b, const phx_lw_params*
   if (env_on("PHX_WIDE")) return run_builder_wide(v, b, p, Aout_d, stats);
   if (v->nb == 6 && !p->window_energy) return run_builder<6>(v, b, p, Aout_d, stats);
   // the split precisions, cells beyond 16 branches and FP64 where the tensor-pipe
-  // kernel fits run on the many-branch builder; FP64 with more R3 vectors (over
+  // kernel would fit run on the many-branch builder; FP64 with more R3 vectors (over
   // 332 at 15 branches) or R2 vectors than that, or with little work, on the shared-memory one
   if (v->precision != PHX_PREC_FP64 || v->nb > kMaxNbGeneric ||
       (wide::q1_fp64_mma(v->nb, v->nr3) && wide::fold_smem(v->nb, v->nr2) <= 227 * 1024 &&

@@ -1,5 +1,5 @@
-// FP64 pair kernel for cells of up to 16 branches (with per-q1 q2 windows and
-// screening masks): the items and folded vertex of wide.cu, all three
+// FP64 pair kernel for cells of up to 16 branches, but for few of them with few R3
+// vectors (with per-q1 q2 windows and screening masks): the items and folded vertex of wide.cu, all three
 // contractions on the FP64 tensor pipe (mma.sync m8n8k4.f64), one warp per q1
 // from T to the rates.
 //

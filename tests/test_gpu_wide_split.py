@@ -5,8 +5,8 @@ twelve-atom cell's first atoms), q1 counts that are no multiple of an item, R3 c
 and of several A stages, q2 windows, both smearings, and an R3 count that leaves no room for the
 kernel (the older one takes over).  The FP64 builders of up to 16 branches against the oracle at the
 1e-10 of the other FP64 linewidth tests: as routed, where problems as small as these run on the
-shared-memory builder, and forced onto the FP64 tensor pipe; the route between the two; isotope
-scattering in slots of q2."""
+shared-memory builder, and forced onto the many-branch one (FP64 tensor pipe, wide.cu's kernel up to 6
+branches); the route between the two; isotope scattering in slots of q2."""
 import numpy as np
 import pytest
 
@@ -113,23 +113,25 @@ def test_fp64_matches_oracle(ctx, nat, mesh, nr3, window, smearing):
 
 
 @pytest.mark.parametrize("smearing", ["adaptive", "gaussian"])
-@pytest.mark.parametrize("nat,mesh,nr3,window", [(1, (3, 2, 2), 1, False), (2, (5, 4, 1), 4, True), (3, (3, 3, 2), 27, False),
-                                                 (5, (3, 2, 2), 67, True), (5, (3, 2, 1), 130, False),
-                                                 (5, (3, 1, 1), 343, True)])
-def test_fp64_tensor_pipe_matches_oracle(ctx, monkeypatch, nat, mesh, nr3, window, smearing):
-    """The same on the tensor-pipe kernel, which problems as small as these reach only when forced."""
+@pytest.mark.parametrize("nat,mesh,nr3,window", [(1, (3, 2, 2), 1, False), (1, (5, 4, 1), 343, True), (2, (5, 4, 1), 4, True),
+                                                 (2, (5, 4, 1), 49, True), (2, (5, 4, 1), 50, True), (2, (3, 2, 2), 250, True),
+                                                 (3, (3, 3, 2), 27, False), (4, (5, 4, 1), 1, True), (5, (3, 2, 2), 67, True),
+                                                 (5, (3, 2, 1), 130, False)])
+def test_fp64_many_branch_matches_oracle(ctx, monkeypatch, nat, mesh, nr3, window, smearing):
+    """The same on the many-branch builder, which problems as small as these reach only when forced: the
+    tensor-pipe kernel, and wide.cu's up to 6 branches (6 branches: fewer than 50 R3)."""
     monkeypatch.setenv("PHX_WIDE", "1")
     _fp64_against_oracle(ctx, nat, mesh, nr3, window, smearing)
 
 
 # items of 16 q1 and a q2, blocks of 4 q1 and a q2, on 148 SMs
-@pytest.mark.parametrize("nat,mesh,q2,tensor_pipe", [
-    (1, (8, 8, 2), 73, False), (1, (8, 8, 2), 74, True), (2, (8, 8, 2), 73, False), (2, (8, 8, 2), 74, True),
+@pytest.mark.parametrize("nat,mesh,q2,many_branch", [
+    (1, (8, 8, 2), 36, False), (1, (8, 8, 2), 37, True), (2, (8, 8, 2), 36, False), (2, (8, 8, 2), 37, True),
     (3, (5, 5, 3), 29, False), (3, (5, 5, 3), 30, True), (4, (4, 4, 2), 18, False), (4, (4, 4, 2), 19, True),
     (5, (3, 3, 1), 9, False), (5, (4, 4, 2), 18, False), (5, (4, 4, 2), 19, True)])
-def test_fp64_route_by_size(ctx, monkeypatch, nat, mesh, q2, tensor_pipe):
+def test_fp64_route_by_size(ctx, monkeypatch, nat, mesh, q2, many_branch):
     """Little work stays on the shared-memory builder (no pair events); both sides of the line agree with
-    the forced tensor-pipe kernel."""
+    the forced many-branch builder."""
     from phoebe_b200.core import Interaction3Ph, PhScatteringMatrix
     cr = _cell(nat)
     E, _, _, bands = _bands(ctx, cr, mesh, np.random.default_rng(nat))
@@ -137,7 +139,7 @@ def test_fp64_route_by_size(ctx, monkeypatch, nat, mesh, q2, tensor_pipe):
     sm = PhScatteringMatrix(v3, bands, [C.kelvin_to_ry(300.0)], "adaptive", 0.0,
                             window=synth.q2_window(E, mesh) if nat == 2 else None)
     A = sm.setup(0, q2, finalize=False)
-    assert (sm.stats.pair_launches > 0) == tensor_pipe
+    assert (sm.stats.pair_launches > 0) == many_branch
     monkeypatch.setenv("PHX_WIDE", "1")
     B = sm.setup(0, q2, finalize=False)
     assert np.abs(B).max() > 0
